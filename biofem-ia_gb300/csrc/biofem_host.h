@@ -16,10 +16,9 @@
 namespace biofem {
 
 constexpr int kMaxQp = 6;
-constexpr int kRefPerQp = 20;     /* FP64 reference constants per (element, qp) */
-constexpr int kRefPerElem = 4;    /* gamma, gamma', c1, pref0 */
-constexpr int kGeomShape = 18;    /* primal element geometry stored for the FP64 tangent (elem_geom_store) */
-constexpr int kGeomPrimal = kGeomShape + 17;   /* + the primal resultants (elem_res_store) */
+constexpr int kRefPerQp = 45;     /* reference constants per (element, thickness point), see element.cuh */
+constexpr int kRefPerElem = 1;    /* pref0 */
+constexpr int kTanCoefs = 116;    /* per-element coefficients of the FP64 tangent (tangent_coefs) */
 constexpr int kCapTable = 11;     /* flat apex-cap triangle: a1 = x2 - x1, a2 = x3 - x1, no curvature */
 constexpr int kNumTables = 12;    /* 0 = regular 12-node patch, v = 3..10 irregular, kCapTable */
 constexpr int kDeStride = 240;    /* per-element tangent block: D = df/dy (15 x 15, row-major), */
@@ -73,8 +72,7 @@ struct DevMesh {
   const int *einfo;          /* ne: nen | (table << 8) */
   const int *ecorner;        /* ne: patch slots of nv1, nv2, nv3 (5 bits each) */
   const double *eref;        /* (kRefPerQp*nq + kRefPerElem) * ne, SoA */
-  const float *erefF;        /* the same in FP32 (FP32-bulk handles only) */
-  const void *erefFF;        /* the same as float-float pairs (FP32-bulk handles only; ff.cuh FF) */
+  const float *erefF;        /* FP32-bulk handles: the same as float-float, the plane of heads then the plane of tails */
   const void *ntabFF;        /* basis tables and their row sums as float-float pairs (FP32-bulk handles) */
   const double *ntab;        /* kNumTables * 5 * 16 basis-derivative tables */
   const float *ntabF;        /* the same in FP32, followed by the kNumTables*5 row sums */
@@ -103,16 +101,15 @@ struct DevMesh {
   int *dptr, *didx;          /* per node, the real triangles with that corner, in triangle order */
   double *xn, *xnm1, *xd, *xdd;   /* 3*nt dynamic state (previous positions, velocity, acceleration) */
   double *dyn_diag;          /* nt: d Fdyn / d x on the diagonal of each free row */
-  double *gmq;               /* FP64 handles: 6 nq x ne thickness-point metrics, k_elem_residual -> k_elem_tangent */
-  double *gpr;               /* FP64 handles: kGeomPrimal x ne primal geometry and resultants, k_elem_residual -> k_elem_tangent */
-  double *gtape;             /* FP64 handles: nq x (6 + 23 C33 iterations) x ne primal stress values, likewise */
+  double *cq;                /* FP64 handles: 15 nq x ne stress gradients d S / d metric (k_elem_residual's own scratch) */
+  double *tcoef;             /* FP64 handles: kTanCoefs x ne tangent coefficients, k_elem_residual -> k_elem_tangent */
   unsigned long long *fmax;  /* max |Fext| as ordered bits */
 };
 
 /* kernel launchers (kernels.cu); return cudaError_t as int */
 int launch_ref_prep(const DevMesh &m, const KParams &p, const double *fib, const double *gscale, double *eref_out, void *stream);
 int launch_positions(const DevMesh &m, const KParams &p, const double *x, void *stream);
-int launch_elem_residual(const DevMesh &m, const KParams &p, void *stream, bool store_metric = false);
+int launch_elem_residual(const DevMesh &m, const KParams &p, void *stream, bool tangent = false);
 int launch_elem_tangent(const DevMesh &m, const KParams &p, void *stream);
 int launch_node_gather(const DevMesh &m, const KParams &p, const double *x, double *R, void *stream,
                        double *parts = nullptr);
@@ -126,8 +123,7 @@ int row_assemble_max_blocks(bool f32);             /* blocks per row each row as
 int launch_scale(const DevMesh &m, const KParams &p, double *R, void *stream);
 int launch_elem_tangent_f32(const DevMesh &m, const KParams &p, void *stream);
 int launch_elem_residual_ff(const DevMesh &m, const KParams &p, void *stream);
-int launch_to_ff(const double *a, void *b, long long n, void *stream);
-int launch_to_float(const double *a, float *b, long long n, void *stream);
+int launch_to_ff(const double *a, float *b, long long n, void *stream);   /* heads, then tails */
 int launch_dyn_diag(const DevMesh &m, const KParams &p, void *stream);
 int launch_dyn_update(const DevMesh &m, const KParams &p, const double *x, void *stream);
 int upload_tables(double *d_ntab);

@@ -575,21 +575,19 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
   if (params->precision == BIOFEM_FP64) {
     double *dK = nullptr;
     if ((rc = dalloc(m, &dm.De, (size_t)kDeStride * ne)) || (rc = dalloc(m, &dK, 9 * (size_t)m->nnzb)) ||
-        (rc = dalloc(m, &dm.gmq, 6 * (size_t)kp.nq * ne)) || (rc = dalloc(m, &dm.gpr, (size_t)kGeomPrimal * ne)) ||
-        (rc = dalloc(m, &dm.gtape, (size_t)(6 + 23 * kp.iters) * kp.nq * ne))) {
+        (rc = dalloc(m, &dm.cq, 15 * (size_t)kp.nq * ne)) || (rc = dalloc(m, &dm.tcoef, (size_t)kTanCoefs * ne))) {
       free_mesh(m);
       return rc;
     }
     m->d_K = dK;
   } else {
     float *dK = nullptr;
-    FF *d_erefFF = nullptr, *d_ntabFF = nullptr;
+    FF *d_ntabFF = nullptr;
     if ((rc = dalloc(m, &dm.DeF, (size_t)kDeStride * ne)) || (rc = dalloc(m, &dK, 9 * (size_t)m->nnzb)) ||
-        (rc = dalloc(m, &d_erefF, nref)) || (rc = dalloc(m, &d_erefFF, nref)) || (rc = dupload(m, &d_ntabFF, tabsFF))) {
+        (rc = dalloc(m, &d_erefF, 2 * nref)) || (rc = dupload(m, &d_ntabFF, tabsFF))) {
       free_mesh(m);
       return rc;
     }
-    dm.erefFF = d_erefFF;
     dm.ntabFF = d_ntabFF;
     m->d_K = dK;
   }
@@ -604,8 +602,7 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
     free_mesh(m);
     return fail(76, std::string("reference preparation launch: ") + cudaGetErrorString((cudaError_t)rc));
   }
-  if (d_erefF && ((rc = launch_to_float(d_eref, d_erefF, (long long)nref, m->st)) ||
-                  (rc = launch_to_ff(d_eref, const_cast<void *>(dm.erefFF), (long long)nref, m->st)))) {
+  if (d_erefF && (rc = launch_to_ff(d_eref, d_erefF, (long long)nref, m->st))) {
     free_mesh(m);
     return fail(76, std::string("reference conversion launch: ") + cudaGetErrorString((cudaError_t)rc));
   }
@@ -1100,8 +1097,7 @@ int SetGpuElementGamma(BiofemGpuMesh *m, const double *gamma_e)
   int rc = launch_positions(m->dm, kp, m->dm.X, m->st);
   if (!rc) rc = launch_ref_prep(m->dm, kp, m->d_fib, m->d_gam, const_cast<double *>(m->dm.eref), m->st);
   const size_t nref = (size_t)(kRefPerQp * kp.nq + kRefPerElem) * ne;
-  if (!rc && m->dm.erefF) rc = launch_to_float(m->dm.eref, const_cast<float *>(m->dm.erefF), (long long)nref, m->st);
-  if (!rc && m->dm.erefFF) rc = launch_to_ff(m->dm.eref, const_cast<void *>(m->dm.erefFF), (long long)nref, m->st);
+  if (!rc && m->dm.erefF) rc = launch_to_ff(m->dm.eref, const_cast<float *>(m->dm.erefF), (long long)nref, m->st);
   if (rc) return fail(76, std::string("activation update launch: ") + cudaGetErrorString((cudaError_t)rc));
   CUDA_TRY(cudaStreamSynchronize(m->st));
   return 0;

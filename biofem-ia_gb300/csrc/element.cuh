@@ -1,8 +1,7 @@
 /*
  * Element physics of the active-strain Kirchhoff-Love shell, written once for
- * double and for a one-direction dual number (value + derivative), so the same
- * code gives the internal force and, lane by lane, the columns of its
- * derivative.
+ * double, float and float-float: the internal force, the gradient of the
+ * stress along the metric, and from it the force's derivative.
  *
  * The element is reduced to 15 "generalised coordinates"
  *   y = (a1, a2, Aaa, Abb, Aab) = N x_patch,
@@ -32,9 +31,10 @@
  *   Qxy = (A^T x)^T Ci (A^T y),  v = Fa_inv.Cov G^-1 e3,  w = H v,
  *   alpha = K (Je^2 - Je) - mu,  beta = K Je (2 Je - 1) / 2,
  * which is the contraction the reference evaluates with its 3^6 and 3^8 loops
- * (active_strain.c:1381-1434, 1494-1532, 1592-1651).  The per-(element, qp)
- * reference constants (G^-1 entries, s, t, rho, A^T v, A^T w, A^T e3) are
- * computed once per mesh.
+ * (active_strain.c:1381-1434, 1494-1532, 1592-1651).  All of it is linear in
+ * Ci but for alpha, beta and the products of the Q's, so the per-(element, qp)
+ * reference constants are the linear forms' coefficients, computed once per
+ * mesh.
  */
 #ifndef BIOFEM_ELEMENT_CUH
 #define BIOFEM_ELEMENT_CUH
@@ -45,143 +45,98 @@
 namespace biofem {
 
 /* ---------------- scalar types ---------------- */
-/* One-direction dual number over the real type R (double or float). */
-template <class R> struct D1 { R v, d; };
-typedef D1<double> D1d;
-typedef D1<float> D1f;
-
-template <class R> __host__ __device__ __forceinline__ R val(R a) { return a; }
-template <class R> __host__ __device__ __forceinline__ R val(const D1<R> &a) { return a.v; }
-
-template <class R> __host__ __device__ __forceinline__ D1<R> operator+(D1<R> a, D1<R> b) { return {a.v + b.v, a.d + b.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator-(D1<R> a, D1<R> b) { return {a.v - b.v, a.d - b.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator-(D1<R> a) { return {-a.v, -a.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator*(D1<R> a, D1<R> b) { return {a.v * b.v, a.d * b.v + a.v * b.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator+(D1<R> a, R b) { return {a.v + b, a.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator+(R a, D1<R> b) { return {a + b.v, b.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator-(D1<R> a, R b) { return {a.v - b, a.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator-(R a, D1<R> b) { return {a - b.v, -b.d}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator*(D1<R> a, R b) { return {a.v * b, a.d * b}; }
-template <class R> __host__ __device__ __forceinline__ D1<R> operator*(R a, D1<R> b) { return {a * b.v, a * b.d}; }
-/* Quotients take one reciprocal for value and derivative (the dual types are
-   used only by the tangent kernels, whose primal values feed derivatives
-   alone; the residual is evaluated separately in the plain type). */
-template <class R> __host__ __device__ __forceinline__ D1<R> operator/(D1<R> a, D1<R> b)
-{
-  const R r = R(1) / b.v, q = a.v * r;
-  return {q, (a.d - q * b.d) * r};
-}
-template <class R> __host__ __device__ __forceinline__ D1<R> operator/(R a, D1<R> b)
-{
-  const R r = R(1) / b.v, q = a * r;
-  return {q, -(q * b.d) * r};
-}
-template <class R> __host__ __device__ __forceinline__ D1<R> operator/(D1<R> a, R b) { const R r = R(1) / b; return {a.v * r, a.d * r}; }
-__host__ __device__ __forceinline__ D1d dsqrt(D1d a) { double r = sqrt(a.v); return {r, a.d * (0.5 / r)}; }
-__host__ __device__ __forceinline__ D1f dsqrt(D1f a) { float r = sqrtf(a.v); return {r, a.d * (0.5f / r)}; }
-/* K-direction dual number (the constitutive derivatives of the tangent
-   kernels carry 2 or 3 metric directions per lane). */
-template <class R, int K> struct DK { R v; R d[K]; };
-template <class R, int K> __host__ __device__ __forceinline__ R val(const DK<R, K> &a) { return a.v; }
-#define BIOFEM_DK_LOOP _Pragma("unroll") for (int i = 0; i < K; i++)
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator+(const DK<R, K> &a, const DK<R, K> &b)
-{ DK<R, K> c; c.v = a.v + b.v; BIOFEM_DK_LOOP c.d[i] = a.d[i] + b.d[i]; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator-(const DK<R, K> &a, const DK<R, K> &b)
-{ DK<R, K> c; c.v = a.v - b.v; BIOFEM_DK_LOOP c.d[i] = a.d[i] - b.d[i]; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator-(const DK<R, K> &a)
-{ DK<R, K> c; c.v = -a.v; BIOFEM_DK_LOOP c.d[i] = -a.d[i]; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator*(const DK<R, K> &a, const DK<R, K> &b)
-{ DK<R, K> c; c.v = a.v * b.v; BIOFEM_DK_LOOP c.d[i] = a.d[i] * b.v + a.v * b.d[i]; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator+(const DK<R, K> &a, R b)
-{ DK<R, K> c = a; c.v = a.v + b; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator+(R a, const DK<R, K> &b)
-{ DK<R, K> c = b; c.v = a + b.v; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator-(const DK<R, K> &a, R b)
-{ DK<R, K> c = a; c.v = a.v - b; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator-(R a, const DK<R, K> &b)
-{ DK<R, K> c; c.v = a - b.v; BIOFEM_DK_LOOP c.d[i] = -b.d[i]; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator*(const DK<R, K> &a, R b)
-{ DK<R, K> c; c.v = a.v * b; BIOFEM_DK_LOOP c.d[i] = a.d[i] * b; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator*(R a, const DK<R, K> &b)
-{ DK<R, K> c; c.v = a * b.v; BIOFEM_DK_LOOP c.d[i] = a * b.d[i]; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator/(const DK<R, K> &a, const DK<R, K> &b)
-{ DK<R, K> c; const R r = R(1) / b.v; c.v = a.v * r; BIOFEM_DK_LOOP c.d[i] = (a.d[i] - c.v * b.d[i]) * r; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator/(R a, const DK<R, K> &b)
-{ DK<R, K> c; const R r = R(1) / b.v; c.v = a * r; BIOFEM_DK_LOOP c.d[i] = -(c.v * b.d[i]) * r; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> operator/(const DK<R, K> &a, R b)
-{ DK<R, K> c; const R r = R(1) / b; c.v = a.v * r; BIOFEM_DK_LOOP c.d[i] = a.d[i] * r; return c; }
-template <class R, int K> __host__ __device__ __forceinline__ DK<R, K> dsqrt(const DK<R, K> &a)
-{ DK<R, K> c; c.v = sqrt(a.v); const R h = R(0.5) / c.v; BIOFEM_DK_LOOP c.d[i] = a.d[i] * h; return c; }
-#undef BIOFEM_DK_LOOP
 __host__ __device__ __forceinline__ double dsqrt(double a) { return sqrt(a); }
 __host__ __device__ __forceinline__ float dsqrt(float a) { return sqrtf(a); }
 __host__ __device__ __forceinline__ double dabs(double a) { return fabs(a); }
 __host__ __device__ __forceinline__ float dabs(float a) { return fabsf(a); }
 
-/* real type underlying a scalar */
-template <class T> struct RealOf { typedef T type; };
-template <class R> struct RealOf<D1<R>> { typedef R type; };
-
 template <class T> struct V3 { T x, y, z; };
 template <class T> __host__ __device__ __forceinline__ V3<T> operator+(const V3<T> &a, const V3<T> &b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
 template <class T> __host__ __device__ __forceinline__ V3<T> operator-(const V3<T> &a, const V3<T> &b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
 template <class T, class S> __host__ __device__ __forceinline__ V3<T> scl(const S &s, const V3<T> &a) { return {s * a.x, s * a.y, s * a.z}; }
-template <class T> __host__ __device__ __forceinline__ T dot(const V3<T> &a, const V3<T> &b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+
+/* A sum of products: one chain of fused multiply-adds, or its float-float form. */
+template <class R> struct Acc {
+  R v;
+  __host__ __device__ __forceinline__ Acc(R c) : v(c) {}
+  __host__ __device__ __forceinline__ Acc(R a, R b) : v(a * b) {}
+  __host__ __device__ __forceinline__ void add(R a, R b) { v = v + a * b; }
+  __host__ __device__ __forceinline__ R get() const { return v; }
+};
+template <> struct Acc<FF> : FFAcc { using FFAcc::FFAcc; };
+template <class R> __host__ __device__ __forceinline__ R pow2(R x, float c) { return x * R(c); }
+
+/* a b + c d (+ e f) */
+template <class R> __host__ __device__ __forceinline__ R sop(R a, R b, R c, R d) { Acc<R> s(a, b); s.add(c, d); return s.get(); }
+template <class R> __host__ __device__ __forceinline__ R sop(R a, R b, R c, R d, R e, R f)
+{
+  Acc<R> s(a, b);
+  s.add(c, d); s.add(e, f);
+  return s.get();
+}
+/* c + a b */
+template <class R> __host__ __device__ __forceinline__ R mad(R a, R b, R c) { Acc<R> s(c); s.add(a, b); return s.get(); }
+
+template <class T> __host__ __device__ __forceinline__ T dot(const V3<T> &a, const V3<T> &b) { return sop(a.x, b.x, a.y, b.y, a.z, b.z); }
 template <class T> __host__ __device__ __forceinline__ V3<T> cross(const V3<T> &a, const V3<T> &b)
 {
-  return {a.y * b.z - b.y * a.z, b.x * a.z - a.x * b.z, a.x * b.y - b.x * a.y};
+  return {sop(a.y, b.z, -b.y, a.z), sop(b.x, a.z, -a.x, b.z), sop(a.x, b.y, -b.x, a.y)};
 }
-
-/* One-hot directions of the FP64 tangent's chain rule.  Lane 3 r + c of an
-   element group differentiates along the Cartesian component c of the r-th
-   of (a1, a2, Aaa, Abb, Aab); a product with that unit vector is a selection
-   of primal values (integer pipe), not FP64 arithmetic. */
-__device__ __forceinline__ double ineg(double x)
+/* c + s a */
+template <class T> __host__ __device__ __forceinline__ V3<T> mad(const T &s, const V3<T> &a, const V3<T> &c)
 {
-  return __longlong_as_double(__double_as_longlong(x) ^ (long long)(1ull << 63));
+  return {mad(s, a.x, c.x), mad(s, a.y, c.y), mad(s, a.z, c.z)};
 }
-__device__ __forceinline__ float ineg(float x) { return __int_as_float(__float_as_int(x) ^ (int)(1u << 31)); }
-
-template <class R> __device__ __forceinline__ R comp(const V3<R> &v, int c) { return c == 0 ? v.x : (c == 1 ? v.y : v.z); }
-
-/* e_c x v */
-template <class R> __device__ __forceinline__ V3<R> ecross(int c, const V3<R> &v)
+/* r a + s b + t c */
+template <class T>
+__host__ __device__ __forceinline__ V3<T> lin3(const T &r, const V3<T> &a, const T &s, const V3<T> &b, const T &t, const V3<T> &c)
 {
-  return {c == 1 ? v.z : (c == 2 ? ineg(v.y) : R(0)), c == 0 ? ineg(v.z) : (c == 2 ? v.x : R(0)),
-          c == 0 ? v.y : (c == 1 ? ineg(v.x) : R(0))};
+  return {sop(r, a.x, s, b.x, t, c.x), sop(r, a.y, s, b.y, t, c.y), sop(r, a.z, s, b.z, t, c.z)};
+}
+/* a x b + c x d */
+template <class T>
+__host__ __device__ __forceinline__ V3<T> cross2(const V3<T> &a, const V3<T> &b, const V3<T> &c, const V3<T> &d)
+{
+  Acc<T> x(a.y, b.z), y(b.x, a.z), z(a.x, b.y);
+  x.add(-b.y, a.z); x.add(c.y, d.z); x.add(-d.y, c.z);
+  y.add(-a.x, b.z); y.add(d.x, c.z); y.add(-c.x, d.z);
+  z.add(-b.x, a.y); z.add(c.x, d.y); z.add(-d.x, c.y);
+  return {x.get(), y.get(), z.get()};
 }
 
-/* v, -v or 0 */
-template <class R> __device__ __forceinline__ V3<R> sel_sign(const V3<R> &v, bool on, bool neg)
-{
-  return {on ? (neg ? ineg(v.x) : v.x) : R(0), on ? (neg ? ineg(v.y) : v.y) : R(0),
-          on ? (neg ? ineg(v.z) : v.z) : R(0)};
-}
+/* Reference constants of one (element, thickness point), kRefPerQp values.
+   Everything the stress contracts the in-plane inverse metric with is linear
+   in c = (c00, c11, c01, c22), so the constants are the forms' coefficients,
+   four each, computed once per mesh (ref_point_consts in kernels.cu):
+     S^33 etc. = S.. + alpha/2 B..(c),  Q_xy(c) of v, w, e3.
+   A form costs 3 + 1 multiply-adds against the 5 to 9 of evaluating it from
+   s, t, A^T v, ..., at 25 more loads a point, and FP64 is the bound: residual
+   0.39 -> 0.31 ms on the 98,304-triangle sheet, 0.63 ms with gradients. */
+enum {
+  kRfS33 = 0, kRfS00, kRfS11, kRfS01,                       /* mu (G^-1 + c1 s s^T) */
+  kRfB33 = 4, kRfB00 = 8, kRfB11 = 12, kRfB01 = 16,         /* Ci + A Ci H */
+  kRfQvv = 20, kRfQww = 24, kRfQee = 28, kRfQvw = 32, kRfQve = 36, kRfQwe = 40,
+  kRfRho = 44
+};
+static_assert(kRefPerQp == kRfRho + 1, "reference constants");
 
-/* v + s e_c: one add */
-template <class R> __device__ __forceinline__ V3<R> add_at(const V3<R> &v, int c, R s)
-{
-  const R t = comp(v, c) + s;
-  return {c == 0 ? t : v.x, c == 1 ? t : v.y, c == 2 ? t : v.z};
-}
-
-/* a x b + acc and a.b + acc as FMA chains */
-template <class R> __device__ __forceinline__ V3<R> cross_acc(const V3<R> &a, const V3<R> &b, const V3<R> &acc)
-{
-  return {fma(a.y, b.z, fma(-b.y, a.z, acc.x)), fma(b.x, a.z, fma(-a.x, b.z, acc.y)),
-          fma(a.x, b.y, fma(-b.x, a.y, acc.z))};
-}
-template <class R> __device__ __forceinline__ R dot_acc(const V3<R> &a, const V3<R> &b, R acc)
-{
-  return fma(a.z, b.z, fma(a.y, b.y, fma(a.x, b.x, acc)));
-}
-
-/* Reference constants of one (element, qp), see the header comment. */
-template <class R> struct QpRef {
-  R gc00, gc11, gc01, gc22;   /* G^-1 entries used by S */
-  R s[3], t[3];
-  R rho;
-  R av[3], aw[3], ae[3];      /* A^T v, A^T w, A^T e3 */
+/* One element's column of the reference constants (SoA, stride = ne).  The
+   float-float form keeps the heads and the tails as two float planes, the
+   heads being the FP32 tangent's constants. */
+template <class R> struct RefCol {
+  const R *p;
+  size_t stride;
+  __host__ __device__ __forceinline__ R operator()(int k) const { return p[(size_t)k * stride]; }
+  __host__ __device__ __forceinline__ RefCol at(int k) const { return {p + (size_t)k * stride, stride}; }
+};
+template <> struct RefCol<FF> {
+  const float *p;
+  size_t stride, tail;          /* distance of the tails' plane */
+  __host__ __device__ __forceinline__ FF operator()(int k) const
+  {
+    return FF(p[(size_t)k * stride], p[tail + (size_t)k * stride]);
+  }
+  __host__ __device__ __forceinline__ RefCol at(int k) const { return {p + (size_t)k * stride, stride, tail}; }
 };
 
 /* Material / quadrature constants in the working precision R. */
@@ -222,26 +177,20 @@ template <> __host__ __device__ __forceinline__ EPar<float> epar<float>(const KP
   return e;
 }
 
-/* Quadratic form (A^T x)^T Ci (A^T y) with Ci = [[c00 c01 0][c01 c11 0][0 0 c22]]. */
-template <class T, class R>
-__host__ __device__ __forceinline__ T qform(const T &c00, const T &c11, const T &c01, const T &c22,
-                                            const R *x, const R *y)
+/* d/dg of a symmetric inverse c = g^-1, restricted to the in-plane block:
+   L[m][k] = d c_m / d g_k for c_m = c00, c11, c01 and the metric components
+   g_k = 00, 11, 01, 02, 12 (dc = -c dg c; c02 = c12 = 0 for a 2x2 inverse). */
+template <class R>
+__host__ __device__ __forceinline__ void inverse_rows(R c00, R c11, R c01, R c02, R c12, R L[3][5])
 {
-  return x[0] * (c00 * y[0] + c01 * y[1]) + x[1] * (c01 * y[0] + c11 * y[1]) + (x[2] * y[2]) * c22;
+  const R two = R(2);
+  L[0][0] = -(c00 * c00); L[0][1] = -(c01 * c01); L[0][2] = -(two * c00 * c01);
+  L[0][3] = -(two * c00 * c02); L[0][4] = -(two * c01 * c02);
+  L[1][0] = L[0][1]; L[1][1] = -(c11 * c11); L[1][2] = -(two * c01 * c11);
+  L[1][3] = -(two * c01 * c12); L[1][4] = -(two * c11 * c12);
+  L[2][0] = -(c00 * c01); L[2][1] = -(c01 * c11); L[2][2] = -(c00 * c11 + c01 * c01);
+  L[2][3] = -(c00 * c12 + c01 * c02); L[2][4] = -(c01 * c12 + c11 * c02);
 }
-
-/* Primal values of the C33 sub-iterations of one thickness point that the
-   FP64 tangent's derivative-only form reads (qp_stress_tl): the residual
-   kernel of the same call records them (SoA over elements).  Slots: the
-   initial cofactors and inverses, then per sub-iteration it (base
-   kTapeInit + kTapeIt * it) the values named in qp_stress. */
-constexpr int kTapeInit = 6;    /* cof00 cof11 cof01 cofx 1/det 1/(g00 g11 - g01^2) */
-constexpr int kTapeIt = 23;
-enum {
-  kTpC00, kTpC11, kTpC01, kTpC22, kTpPre, kTpQd, kTpHJ, kTpJe, kTpAlpha, kTpBeta, kTpB33,
-  kTpQvv, kTpQww, kTpQee, kTpQvw, kTpQve, kTpQwe, kTpICC, kTpDC, kTpLo, kTpB0, kTpB1, kTpB2
-};
-__host__ __device__ __forceinline__ int tape_per_qp(int iters) { return kTapeInit + kTapeIt * iters; }
 
 /* Stress of one thickness point after the C33 sub-iterations:
    returns S^11, S^22, S^12 in sv[0..2]; status bit 1 on a vanishing CC3333.
@@ -249,100 +198,182 @@ __host__ __device__ __forceinline__ int tape_per_qp(int iters) { return kTapeIni
    taken before the last one, so final_update = false skips that update
    (CC3333 and its check included) when only the stress is wanted and another
    kernel of the same call performs the check.  c33_out receives C33 after
-   the last update; tape (stride ts) receives the primal values of
-   qp_stress_tl (the arithmetic is the same with or without it). */
-template <class T, class R>
-__host__ __device__ __forceinline__ void qp_stress(const T gm[6] /* 00 11 01 02 12 22 */, const QpRef<R> &r,
-                                                   R gam, R gamp, R c1, R mu, R K,
-                                                   int iters, T sv[3], int &status, T *c33_out = nullptr,
-                                                   bool final_update = true, R *tape = nullptr, size_t ts = 0)
+   the last update.
+
+   grad: C[i][k] = d sv_i / d g_k for the metric components g_k = 00, 11, 01,
+   02, 12 (the sixth, g33 = n.n, is 1 for every state).  The stress depends on
+   the metric only through c(0), the in-plane block of the first
+   sub-iteration's inverse, c(1), the in-plane 2x2 inverse of all later ones,
+   and the scalar C33, whose update of each sub-iteration depends on four
+   numbers (c00, c11, c01, c22 = 1/C33).  So one gradient of that scalar per
+   sub-iteration replaces a forward derivative along each of the five
+   components: X, Y carry dC33 as a combination of dc(0) and dc(1) (XJ, YJ of
+   the determinants in Je), and the metric enters once at the end through
+   dc = -c dg c and d ln det = c:dg.  The damping factor of a bisected update
+   is constant, as in the update itself.  About 0.3 of the arithmetic of five
+   forward directions. */
+template <class R>
+__host__ __device__ __forceinline__ void qp_stress(const R gm[5] /* 00 11 01 02 12 */, const RefCol<R> &r, R mu, R K,
+                                                   int iters, R sv[3], int &status, R *c33_out = nullptr,
+                                                   bool final_update = true, bool grad = false, R C[3][5] = nullptr)
 {
-  const R one = R(1), two = R(2), half = R(0.5), quarter = R(0.25);
-  const T &g00 = gm[0], &g11 = gm[1], &g01 = gm[2], &g02 = gm[3], &g12 = gm[4], &g22 = gm[5];
-  /* ElemCGDefTens: C_inv in-plane = in-plane block of gm^-1, C33 = 1 */
-  T cof00 = g11 * g22 - g12 * g12;
-  T cof11 = g00 * g22 - g02 * g02;
-  T cof01 = g02 * g12 - g01 * g22;
-  const T cofx = g01 * g12 - g11 * g02;
-  T det = g00 * cof00 + g01 * cof01 + g02 * cofx;
-  T idet = one / det;
-  T c00 = cof00 * idet, c11 = cof11 * idet, c01 = cof01 * idet;
-  T c22 = T{one};
-  T C33 = T{one};
-  if (tape) {
-    tape[0] = val(cof00); tape[ts] = val(cof11); tape[2 * ts] = val(cof01); tape[3 * ts] = val(cofx);
-    tape[4 * ts] = val(idet);
+  const R one = R(1), two = R(2), half = R(0.5), quarter = R(0.25), four = R(4);
+  const R g00 = gm[0], g11 = gm[1], g01 = gm[2], g02 = gm[3], g12 = gm[4];
+  /* ElemCGDefTens: C_inv in-plane = in-plane block of gm^-1 (g33 = n.n = 1), C33 = 1 */
+  const R cof00 = mad(-g12, g12, g11);
+  const R cof11 = mad(-g02, g02, g00);
+  const R cof01 = mad(g02, g12, -g01);
+  const R cofx = sop(g01, g12, -g11, g02);
+  const R det = sop(g00, cof00, g01, cof01, g02, cofx);
+  const R idet = one / det;
+  R c00 = cof00 * idet, c11 = cof11 * idet, c01 = cof01 * idet;
+  R c22 = one;
+  R C33 = one;
+  R X[3], Y[3], XJ = R(0), YJ = R(0);        /* grad: dC33 = X.dc(0) + XJ d ln det(0) + Y.dc(1) + YJ d ln det(1) */
+  const R k00 = c00, k11 = c11, k01 = c01;   /* c(0) */
+  const R den = sop(g00, g11, -g01, g01);
+  /* 1 / (c00 c11 - c01^2), the determinant the in-plane inverse was divided
+     by: det for c(0), the 2x2 determinant for c(1).  Je takes it from here,
+     1 / det Ci = ipre C33, rather than from the rounded inverse: one division
+     less a sub-iteration and about half the rounding error. */
+  R ipre = det;
+  /* the in-plane parts of the seven forms of c every sub-iteration needs; c
+     changes in the plane once, after the first */
+  constexpr int kForm[7] = {kRfB33, kRfQvv, kRfQww, kRfQee, kRfQvw, kRfQve, kRfQwe};
+  R ip[7];
+  auto in_plane = [&]() {
+#pragma unroll
+    for (int f = 0; f < 7; f++) ip[f] = sop(r(kForm[f]), c00, r(kForm[f] + 1), c11, r(kForm[f] + 2), c01);
+  };
+  in_plane();
+  if (grad) {
+#pragma unroll
+    for (int m = 0; m < 3; m++) X[m] = Y[m] = R(0);
   }
   for (int it = 0; it < iters; it++) {
-    R *tp = tape ? tape + (size_t)(kTapeInit + kTapeIt * it) * ts : nullptr;
-    const T u0 = c00 * r.t[0] + c01 * r.t[1];
-    const T u1 = c01 * r.t[0] + c11 * r.t[1];
-    const T u2 = c22 * r.t[2];
-    const T tau = r.t[0] * u0 + r.t[1] * u1 + r.t[2] * u2;
-    const T pre = c00 * c11 - c01 * c01;
-    const T detci = pre * c22;
-    const T qrd = r.rho / detci;
-    const T Je = dsqrt(qrd);
-    const T alpha = K * (Je * Je - Je) - mu;
-    const T beta = (half * K) * Je * (two * Je - one);
-    const T half_a = half * alpha;
-    const R gg = gam * gamp;
-    /* S^33 */
-    const T B33 = two * c22 + (gamp - gam) * r.s[2] * u2 - gg * r.s[2] * r.s[2] * tau;
-    const T S33 = mu * (r.gc22 + c1 * r.s[2] * r.s[2]) + half_a * B33;
-    if (tp) {
-      tp[kTpC00 * ts] = val(c00); tp[kTpC11 * ts] = val(c11); tp[kTpC01 * ts] = val(c01); tp[kTpC22 * ts] = val(c22);
-      tp[kTpPre * ts] = val(pre); tp[kTpQd * ts] = val(qrd) / val(detci); tp[kTpHJ * ts] = half / val(Je);
-      tp[kTpJe * ts] = val(Je); tp[kTpAlpha * ts] = val(alpha); tp[kTpBeta * ts] = val(beta); tp[kTpB33 * ts] = val(B33);
+    const bool last = it == iters - 1;
+    const R J2 = r(kRfRho) * ipre * C33;
+    const R Je = dsqrt(J2);
+    const R alpha = mad(K, J2 - Je, -mu);
+    const R half_a = pow2(alpha, 0.5f);
+    if (last) {
+      R Bi[3];
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const int o = kRfB00 + 4 * i;
+        Acc<R> b(r(o), c00);
+        b.add(r(o + 1), c11); b.add(r(o + 2), c01); b.add(r(o + 3), c22);
+        Bi[i] = b.get();
+        sv[i] = mad(half_a, Bi[i], r(kRfS00 + i));
+      }
+      if (grad) {
+        /* dJe = Je/2 (d ln ipre + dC33/C33), d ln ipre = c:dg */
+        const R sJ = (half * K) * (two * Je - one) * (half * Je);
+        if (it > 0) {
+          /* v = dC33/dg: the rows of dc and d ln det at c(0) (cofactor (1, 2)
+             of the 3x3 inverse is g01 g02 - g00 g12), then at c(1) */
+          R L[3][5], v[5];
+          const R k02 = cofx * idet, k12 = (g01 * g02 - g00 * g12) * idet;
+          const R ln0[5] = {k00, k11, two * k01, two * k02, two * k12};
+          inverse_rows<R>(k00, k11, k01, k02, k12, L);
+#pragma unroll
+          for (int k = 0; k < 5; k++) v[k] = X[0] * L[0][k] + X[1] * L[1][k] + X[2] * L[2][k] + XJ * ln0[k];
+          inverse_rows<R>(c00, c11, c01, R(0), R(0), L);
+          const R ln1[3] = {c00, c11, two * c01};
+#pragma unroll
+          for (int k = 0; k < 3; k++) v[k] = v[k] + (Y[0] * L[0][k] + Y[1] * L[1][k] + Y[2] * L[2][k] + YJ * ln1[k]);
+          const R hc = half_a * (c22 * c22);
+#pragma unroll
+          for (int i = 0; i < 3; i++) {
+            const int o = kRfB00 + 4 * i;
+            const R a = sJ * Bi[i], d00 = half_a * r(o), d11 = half_a * r(o + 1), d01 = half_a * r(o + 2);
+            const R z = a * c22 - hc * r(o + 3);                 /* along C33 (dc22 = -c22^2 dC33) */
+#pragma unroll
+            for (int k = 0; k < 3; k++) C[i][k] = d00 * L[0][k] + d11 * L[1][k] + d01 * L[2][k] + a * ln1[k] + z * v[k];
+            C[i][3] = z * v[3]; C[i][4] = z * v[4];
+          }
+        } else {
+          R L[3][5];
+          const R k02 = cofx * idet, k12 = (g01 * g02 - g00 * g12) * idet;
+          const R ln0[5] = {k00, k11, two * k01, two * k02, two * k12};
+          inverse_rows<R>(k00, k11, k01, k02, k12, L);
+#pragma unroll
+          for (int i = 0; i < 3; i++) {
+            const int o = kRfB00 + 4 * i;
+            const R a = sJ * Bi[i], d00 = half_a * r(o), d11 = half_a * r(o + 1), d01 = half_a * r(o + 2);
+#pragma unroll
+            for (int k = 0; k < 5; k++) C[i][k] = d00 * L[0][k] + d11 * L[1][k] + d01 * L[2][k] + a * ln0[k];
+          }
+        }
+      }
+      if (!final_update) break;
     }
-    if (it == iters - 1) {
-      const T B0 = two * c00 + (gamp - gam) * r.s[0] * u0 - gg * r.s[0] * r.s[0] * tau;
-      const T B1 = two * c11 + (gamp - gam) * r.s[1] * u1 - gg * r.s[1] * r.s[1] * tau;
-      const T B2 = two * c01 + gamp * r.s[1] * u0 - gam * r.s[0] * u1 - gg * r.s[0] * r.s[1] * tau;
-      sv[0] = mu * (r.gc00 + c1 * r.s[0] * r.s[0]) + half_a * B0;
-      sv[1] = mu * (r.gc11 + c1 * r.s[1] * r.s[1]) + half_a * B1;
-      sv[2] = mu * (r.gc01 + c1 * r.s[0] * r.s[1]) + half_a * B2;
-      if (tp) { tp[kTpB0 * ts] = val(B0); tp[kTpB1 * ts] = val(B1); tp[kTpB2 * ts] = val(B2); }
-    }
-    if (!final_update && it == iters - 1) break;
-    /* CC3333 */
-    const T qvv = qform(c00, c11, c01, c22, r.av, r.av);
-    const T qww = qform(c00, c11, c01, c22, r.aw, r.aw);
-    const T qee = qform(c00, c11, c01, c22, r.ae, r.ae);
-    const T qvw = qform(c00, c11, c01, c22, r.av, r.aw);
-    const T qve = qform(c00, c11, c01, c22, r.av, r.ae);
-    const T qwe = qform(c00, c11, c01, c22, r.aw, r.ae);
-    const T twob = two * beta;
-    const T CC = quarter * (two * (beta - alpha) * qvv * qvv + two * twob * qvv * qwe - R(4) * alpha * qvw * qve
-                            + (twob - alpha) * qwe * qwe - alpha * qww * qee);
+    /* S^33 and CC3333 */
+    const R beta = pow2(K * Je, 0.5f) * (pow2(Je, 2.f) - one);
+    const R B33 = mad(r(kRfB33 + 3), c22, ip[0]);
+    const R S33 = mad(half_a, B33, r(kRfS33));
+    const R qvv = mad(r(kRfQvv + 3), c22, ip[1]), qww = mad(r(kRfQww + 3), c22, ip[2]);
+    const R qee = mad(r(kRfQee + 3), c22, ip[3]), qvw = mad(r(kRfQvw + 3), c22, ip[4]);
+    const R qve = mad(r(kRfQve + 3), c22, ip[5]), qwe = mad(r(kRfQwe + 3), c22, ip[6]);
+    /* 4 CC3333 = Qvv (2 (beta - alpha) Qvv + 4 beta Qwe) + Qwe (2 beta - alpha) Qwe - alpha (4 Qvw Qve + Qww Qee) */
+    const R twob = pow2(beta, 2.f);
+    const R CC = pow2(sop(qvv, sop(twob - pow2(alpha, 2.f), qvv, pow2(twob, 2.f), qwe), qwe * (twob - alpha), qwe,
+                          -alpha, sop(pow2(qvw, 4.f), qve, qww, qee)), 0.25f);
     /* ModElemC33 (active_strain.c:1654-1707) */
-    if (!(dabs(val(CC)) > R(1e-14))) { status |= 1; return; }
-    T dC = -S33 / CC;
-    if (tp) {
-      tp[kTpQvv * ts] = val(qvv); tp[kTpQww * ts] = val(qww); tp[kTpQee * ts] = val(qee);
-      tp[kTpQvw * ts] = val(qvw); tp[kTpQve * ts] = val(qve); tp[kTpQwe * ts] = val(qwe);
-      tp[kTpICC * ts] = one / val(CC); tp[kTpDC * ts] = val(dC); tp[kTpLo * ts] = one;
-    }
-    T Ct = C33 + dC;
-    if (val(g00) * (val(g11) * val(Ct)) - val(g01) * (val(g01) * val(Ct)) <= R(0)) {
+    if (!(dabs(CC) > R(1e-14))) { status |= 1; return; }
+    const R iCC = one / CC;
+    R dC = -(S33 * iCC);
+    const R dC0 = dC;
+    R damp = one;
+    R Ct = C33 + dC;
+    if (den * Ct <= R(0)) {
       R lo = R(0), hi = one;
       for (int bk = 0; bk < 16; bk++) {
         const R mid = half * (lo + hi);
-        const R ct = val(C33) + mid * val(dC);
-        if (val(g00) * (val(g11) * ct) - val(g01) * (val(g01) * ct) > R(0)) lo = mid; else hi = mid;
+        const R ct = C33 + mid * dC;
+        if (den * ct > R(0)) lo = mid; else hi = mid;
       }
       dC = dC * lo;
       Ct = C33 + dC;
-      if (tp) tp[kTpLo * ts] = lo;
+      damp = lo;
+    }
+    if (grad && !last) {
+      /* d dC = damp (-(dS33 + dC0 dCC) / CC) through Je (coefficient wJ on
+         d ln ipre + dC33/C33), B33 (wB) and the quadratic forms (p..) */
+      const R e = -(damp * iCC);
+      const R kj = K * (two * Je - one);
+      const R sum = qvv + qwe;
+      const R CCa = -(quarter * (two * qvv * qvv + four * qvw * qve + qwe * qwe + qww * qee));
+      const R CCb = half * sum * sum;
+      const R wJ = e * (half * kj * B33 + dC0 * (CCa * kj + CCb * ((half * K) * (four * Je - one)))) * (half * Je);
+      const R wQ = e * dC0, wa = wQ * alpha, wb = wQ * beta;
+      const R w[7] = {e * half_a, (wb - wa) * qvv + wb * qwe, -(quarter * wa * qee), -(quarter * wa * qww),
+                      -(wa * qve), -(wa * qvw), wb * qvv + (wb - half * wa) * qwe};
+      R d[4];
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        d[m] = w[0] * r(kForm[0] + m);
+#pragma unroll
+        for (int f = 1; f < 7; f++) d[m] = d[m] + w[f] * r(kForm[f] + m);
+      }
+      if (it == 0) {
+        X[0] = d[0]; X[1] = d[1]; X[2] = d[2]; XJ = wJ;
+      } else {
+        const R f = one + wJ * c22 - d[3] * (c22 * c22);
+#pragma unroll
+        for (int m = 0; m < 3; m++) { X[m] = f * X[m]; Y[m] = f * Y[m] + d[m]; }
+        XJ = f * XJ; YJ = f * YJ + wJ;
+      }
     }
     C33 = Ct;
-    if (it + 1 < iters) {
+    if (!last) {
       /* C_inv = INV([[gm00 gm01 0][gm01 gm11 0][0 0 C33]]): the in-plane block
          is the same in every later sub-iteration */
       if (it == 0) {
-        const T id2 = one / (g00 * g11 - g01 * g01);
+        const R id2 = one / den;
         c00 = g11 * id2; c11 = g00 * id2; c01 = -g01 * id2;
-        if (tape) tape[5 * ts] = val(id2);
+        ipre = den;
+        in_plane();
       }
       c22 = one / C33;
     }
@@ -350,121 +381,15 @@ __host__ __device__ __forceinline__ void qp_stress(const T gm[6] /* 00 11 01 02 
   if (c33_out) *c33_out = C33;
 }
 
-/* Derivative of qp_stress along KD directions dgm of the metric, from the
-   primal values qp_stress recorded in tp (stride ts): only derivatives are
-   computed, operation by operation.  The C33 update after the last stress is
-   not differentiated (the tangent needs the stress only). */
-template <class R, int KD>
-__device__ __forceinline__ void qp_stress_tl(const R gm[6], const R dgm[6][KD], const QpRef<R> &r, R gam, R gamp,
-                                             R c1, R mu, R K, int iters, const R *tp0, size_t ts, R sv[3],
-                                             R dsv[3][KD])
-{
-  const R two = R(2), half = R(0.5), quarter = R(0.25), four = R(4);
-  const R g00 = gm[0], g11 = gm[1], g01 = gm[2], g02 = gm[3], g12 = gm[4], g22 = gm[5];
-  const R cof00 = tp0[0], cof01 = tp0[2 * ts], cofx = tp0[3 * ts], idet = tp0[4 * ts];
-  const R cof11 = tp0[ts];
-  R dc00[KD], dc11[KD], dc01[KD], dc22[KD], dC33[KD];
-#pragma unroll
-  for (int i = 0; i < KD; i++) {
-    const R d00 = dgm[0][i], d11 = dgm[1][i], d01 = dgm[2][i], d02 = dgm[3][i], d12 = dgm[4][i], d22 = dgm[5][i];
-    const R dcof00 = d11 * g22 + g11 * d22 - two * g12 * d12;
-    const R dcof11 = d00 * g22 + g00 * d22 - two * g02 * d02;
-    const R dcof01 = d02 * g12 + g02 * d12 - d01 * g22 - g01 * d22;
-    const R dcofx = d01 * g12 + g01 * d12 - d11 * g02 - g11 * d02;
-    const R ddet = d00 * cof00 + g00 * dcof00 + d01 * cof01 + g01 * dcof01 + d02 * cofx + g02 * dcofx;
-    const R didet = -(idet * idet) * ddet;
-    dc00[i] = dcof00 * idet + cof00 * didet;
-    dc11[i] = dcof11 * idet + cof11 * didet;
-    dc01[i] = dcof01 * idet + cof01 * didet;
-    dc22[i] = R(0);
-    dC33[i] = R(0);
-  }
-  const R gg = gam * gamp;
-  for (int it = 0; it < iters; it++) {
-    const R *tp = tp0 + (size_t)(kTapeInit + kTapeIt * it) * ts;
-    const R c00 = tp[kTpC00 * ts], c11 = tp[kTpC11 * ts], c01 = tp[kTpC01 * ts], c22 = tp[kTpC22 * ts];
-    const R pre = tp[kTpPre * ts], qd = tp[kTpQd * ts], hJ = tp[kTpHJ * ts], Je = tp[kTpJe * ts];
-    const R alpha = tp[kTpAlpha * ts], beta = tp[kTpBeta * ts], B33 = tp[kTpB33 * ts];
-    const R half_a = half * alpha;
-    const bool last = it == iters - 1;
-    R B0 = R(0), B1 = R(0), B2 = R(0);
-    if (last) {
-      B0 = tp[kTpB0 * ts]; B1 = tp[kTpB1 * ts]; B2 = tp[kTpB2 * ts];
-      sv[0] = mu * (r.gc00 + c1 * r.s[0] * r.s[0]) + half_a * B0;
-      sv[1] = mu * (r.gc11 + c1 * r.s[1] * r.s[1]) + half_a * B1;
-      sv[2] = mu * (r.gc01 + c1 * r.s[0] * r.s[1]) + half_a * B2;
-    }
-    R qvv = R(0), qww = R(0), qee = R(0), qvw = R(0), qve = R(0), qwe = R(0), iCC = R(0), dC = R(0), lo = R(1);
-    if (!last) {
-      qvv = tp[kTpQvv * ts]; qww = tp[kTpQww * ts]; qee = tp[kTpQee * ts];
-      qvw = tp[kTpQvw * ts]; qve = tp[kTpQve * ts]; qwe = tp[kTpQwe * ts];
-      iCC = tp[kTpICC * ts]; dC = tp[kTpDC * ts]; lo = tp[kTpLo * ts];
-    }
-#pragma unroll
-    for (int i = 0; i < KD; i++) {
-      const R du0 = dc00[i] * r.t[0] + dc01[i] * r.t[1];
-      const R du1 = dc01[i] * r.t[0] + dc11[i] * r.t[1];
-      const R du2 = dc22[i] * r.t[2];
-      const R dtau = r.t[0] * du0 + r.t[1] * du1 + r.t[2] * du2;
-      const R dpre = dc00[i] * c11 + c00 * dc11[i] - two * c01 * dc01[i];
-      const R ddetci = dpre * c22 + pre * dc22[i];
-      const R dJe = hJ * (-(qd * ddetci));
-      const R dalpha = K * (two * Je - R(1)) * dJe;
-      const R dbeta = (half * K) * (four * Je - R(1)) * dJe;
-      const R dhalf_a = half * dalpha;
-      const R dB33 = two * dc22[i] + (gamp - gam) * r.s[2] * du2 - gg * r.s[2] * r.s[2] * dtau;
-      const R dS33 = dhalf_a * B33 + half_a * dB33;
-      if (last) {
-        const R dB0 = two * dc00[i] + (gamp - gam) * r.s[0] * du0 - gg * r.s[0] * r.s[0] * dtau;
-        const R dB1 = two * dc11[i] + (gamp - gam) * r.s[1] * du1 - gg * r.s[1] * r.s[1] * dtau;
-        const R dB2 = two * dc01[i] + gamp * r.s[1] * du0 - gam * r.s[0] * du1 - gg * r.s[0] * r.s[1] * dtau;
-        dsv[0][i] = dhalf_a * B0 + half_a * dB0;
-        dsv[1][i] = dhalf_a * B1 + half_a * dB1;
-        dsv[2][i] = dhalf_a * B2 + half_a * dB2;
-        continue;
-      }
-      const R dqvv = qform(dc00[i], dc11[i], dc01[i], dc22[i], r.av, r.av);
-      const R dqww = qform(dc00[i], dc11[i], dc01[i], dc22[i], r.aw, r.aw);
-      const R dqee = qform(dc00[i], dc11[i], dc01[i], dc22[i], r.ae, r.ae);
-      const R dqvw = qform(dc00[i], dc11[i], dc01[i], dc22[i], r.av, r.aw);
-      const R dqve = qform(dc00[i], dc11[i], dc01[i], dc22[i], r.av, r.ae);
-      const R dqwe = qform(dc00[i], dc11[i], dc01[i], dc22[i], r.aw, r.ae);
-      const R dCC = quarter * (two * (dbeta - dalpha) * qvv * qvv + four * (beta - alpha) * qvv * dqvv
-                               + four * dbeta * qvv * qwe + four * beta * (dqvv * qwe + qvv * dqwe)
-                               - four * dalpha * qvw * qve - four * alpha * (dqvw * qve + qvw * dqve)
-                               + (two * dbeta - dalpha) * qwe * qwe + two * (two * beta - alpha) * qwe * dqwe
-                               - dalpha * qww * qee - alpha * (dqww * qee + qww * dqee));
-      const R ddC = lo * (-(dS33 + dC * dCC) * iCC);
-      dC33[i] = dC33[i] + ddC;
-    }
-    if (last) break;
-    /* the in-plane inverse from iteration 1 on, and c22 = 1/C33 */
-    const R *tpn = tp0 + (size_t)(kTapeInit + kTapeIt * (it + 1)) * ts;
-    const R c22n = tpn[kTpC22 * ts];
-    const R id2 = tp0[5 * ts];
-#pragma unroll
-    for (int i = 0; i < KD; i++) {
-      if (it == 0) {
-        const R dden = dgm[0][i] * g11 + g00 * dgm[1][i] - two * g01 * dgm[2][i];
-        const R did2 = -(id2 * id2) * dden;
-        dc00[i] = dgm[1][i] * id2 + g11 * did2;
-        dc11[i] = dgm[0][i] * id2 + g00 * did2;
-        dc01[i] = -(dgm[2][i] * id2 + g01 * did2);
-      }
-      dc22[i] = -(c22n * c22n) * dC33[i];
-    }
-  }
-}
-
 /* Mid-surface geometry of the element from y = (a1, a2, Aaa, Abb, Aab). */
 template <class T> struct ElemGeom {
   V3<T> a1, a2, Aaa, Abb, Aab, n, gc1, gc2, a31, a32;
 };
 
-template <class T, class R>
-__host__ __device__ __forceinline__ ElemGeom<T> elem_geom(const T y[15], const EPar<R> &p)
+template <class T>
+__host__ __device__ __forceinline__ ElemGeom<T> elem_geom(const T y[15], const EPar<T> &p)
 {
-  const R one = R(1);
+  const T one = T(1);
   ElemGeom<T> g;
   g.a1 = {y[0], y[1], y[2]}; g.a2 = {y[3], y[4], y[5]};
   g.Aaa = {y[6], y[7], y[8]}; g.Abb = {y[9], y[10], y[11]}; g.Aab = {y[12], y[13], y[14]};
@@ -472,429 +397,269 @@ __host__ __device__ __forceinline__ ElemGeom<T> elem_geom(const T y[15], const E
   const T cn = dsqrt(dot(cr, cr));
   const T icn = one / cn;
   g.n = scl(icn, cr);
-  const V3<T> t1 = cross(g.a2, g.n);
-  g.gc1 = scl(one / dot(g.a1, t1), t1);
-  const V3<T> t2 = cross(g.n, g.a1);
-  g.gc2 = scl(one / dot(g.a2, t2), t2);
-  g.a31 = scl(icn, cross(g.Aaa, g.a2) + cross(g.a1, g.Aab));
-  g.a32 = scl(icn, cross(g.Aab, g.a2) + cross(g.a1, g.Abb));
+  g.gc1 = scl(icn, cross(g.a2, g.n));       /* a1.(a2 x n) = a2.(n x a1) = |a1 x a2| */
+  g.gc2 = scl(icn, cross(g.n, g.a1));
+  g.a31 = scl(icn, cross2(g.Aaa, g.a2, g.a1, g.Aab));
+  g.a32 = scl(icn, cross2(g.Aab, g.a2, g.a1, g.Abb));
   if (p.tnormal) {   /* n_,alpha: drop the J_,alpha / J n part of the unnormalised derivative */
-    g.a31 = g.a31 - scl(dot(g.a31, g.n), g.n);
-    g.a32 = g.a32 - scl(dot(g.a32, g.n), g.n);
+    g.a31 = mad(-dot(g.a31, g.n), g.n, g.a31);
+    g.a32 = mad(-dot(g.a32, g.n), g.n, g.a32);
   }
   return g;
 }
 
-/* Primal geometry the FP64 tangent's chain rule reads, stored once per element
-   by the residual kernel of the same call (SoA over elements): n, 1/|a1 x a2|,
-   t1 = a2 x n, t2 = n x a1, 1/(a1.t1), 1/(a2.t2), u31 = Aaa x a2 + a1 x Aab,
-   u32 = Aab x a2 + a1 x Abb (elem_geom's intermediates); kGeomShape values,
-   followed by elem_res_store's. */
-
-template <class R>
-__host__ __device__ __forceinline__ void elem_geom_store(const R y[15], R *gp, size_t stride)
+/* Metric (00 11 01 02 12; the sixth, n.n, is 1) of the thickness point theta3 (ElemUpdateG). */
+template <class T>
+__host__ __device__ __forceinline__ void qp_metric(const ElemGeom<T> &g, T th3, T gm[5])
 {
-  const R one = R(1);
-  const V3<R> a1 = {y[0], y[1], y[2]}, a2 = {y[3], y[4], y[5]};
-  const V3<R> Aaa = {y[6], y[7], y[8]}, Abb = {y[9], y[10], y[11]}, Aab = {y[12], y[13], y[14]};
-  const V3<R> cr = cross(a1, a2);
-  const R cn = dsqrt(dot(cr, cr));
-  const R icn = one / cn;
-  const V3<R> n = scl(icn, cr);
-  const V3<R> t1 = cross(a2, n), t2 = cross(n, a1);
-  const R s1 = one / dot(a1, t1), s2 = one / dot(a2, t2);
-  const V3<R> u31 = cross(Aaa, a2) + cross(a1, Aab), u32 = cross(Aab, a2) + cross(a1, Abb);
-  const R v[kGeomPrimal] = {n.x, n.y, n.z, icn, t1.x, t1.y, t1.z, t2.x, t2.y, t2.z, s1, s2,
-                            u31.x, u31.y, u31.z, u32.x, u32.y, u32.z};
-#pragma unroll
-  for (int k = 0; k < kGeomShape; k++) gp[k * stride] = v[k];
-}
-
-/* The rest of the tangent's primal values (slots kGeomShape.. of the same
-   block): the pref0-scaled resultants N0 N1 N2 M0 M1 M2, Q, gc1.Q, gc2.Q,
-   gc1, gc2 (elem_out's intermediates, the same expressions). */
-template <class T, class R>
-__host__ __device__ __forceinline__ void elem_res_store(const ElemGeom<T> &g, T N0, T N1, T N2, T M0, T M1, T M2,
-                                                        R pref0, R *gp, size_t stride)
-{
-  const R two = R(2);
-  N0 = pref0 * N0; N1 = pref0 * N1; N2 = pref0 * N2;
-  M0 = pref0 * M0; M1 = pref0 * M1; M2 = pref0 * M2;
-  const T twoM2 = two * M2;
-  const V3<T> Q = scl(M0, g.Aaa) + scl(M1, g.Abb) + scl(twoM2, g.Aab);
-  const R v[kGeomPrimal - kGeomShape] = {
-      val(N0), val(N1), val(N2), val(M0), val(M1), val(M2), val(Q.x), val(Q.y), val(Q.z),
-      val(dot(g.gc1, Q)), val(dot(g.gc2, Q)),
-      val(g.gc1.x), val(g.gc1.y), val(g.gc1.z), val(g.gc2.x), val(g.gc2.y), val(g.gc2.z)};
-#pragma unroll
-  for (int k = 0; k < kGeomPrimal - kGeomShape; k++) gp[(kGeomShape + k) * stride] = v[k];
-}
-
-/* Metric (00 11 01 02 12 22) of the thickness point theta3 (ElemUpdateG). */
-template <class T, class R>
-__host__ __device__ __forceinline__ void qp_metric(const ElemGeom<T> &g, R th3, T gm[6])
-{
-  const V3<T> g1 = g.a1 + scl(th3, g.a31), g2 = g.a2 + scl(th3, g.a32);
+  const V3<T> g1 = mad(th3, g.a31, g.a1), g2 = mad(th3, g.a32, g.a2);
   gm[0] = dot(g1, g1); gm[1] = dot(g2, g2); gm[2] = dot(g1, g2);
-  gm[3] = dot(g1, g.n); gm[4] = dot(g2, g.n); gm[5] = dot(g.n, g.n);
-}
-
-template <class R>
-__host__ __device__ __forceinline__ QpRef<R> load_qpref(const R *ref, int stride, int q)
-{
-  QpRef<R> r;
-  const R *rq = ref + (size_t)kRefPerQp * q * stride;
-  r.gc00 = rq[0]; r.gc11 = rq[(size_t)1 * stride]; r.gc01 = rq[(size_t)2 * stride]; r.gc22 = rq[(size_t)3 * stride];
-  for (int k = 0; k < 3; k++) {
-    r.s[k] = rq[(size_t)(4 + k) * stride];
-    r.t[k] = rq[(size_t)(7 + k) * stride];
-    r.av[k] = rq[(size_t)(11 + k) * stride];
-    r.aw[k] = rq[(size_t)(14 + k) * stride];
-    r.ae[k] = rq[(size_t)(17 + k) * stride];
-  }
-  r.rho = rq[(size_t)10 * stride];
-  return r;
+  gm[3] = dot(g1, g.n); gm[4] = dot(g2, g.n);
 }
 
 /* The 15 force components from the resultants (ElemUpdFint, Nᵀ applied by the caller). */
-template <class T, class R>
-__host__ __device__ __forceinline__ void elem_out(const ElemGeom<T> &g, T N0, T N1, T N2, T M0, T M1, T M2, R pref0,
-                                                  T f[15])
+template <class R>
+__host__ __device__ __forceinline__ void elem_out(const ElemGeom<R> &g, const R N[3], const R M[3], R f[15])
 {
-  const R two = R(2);
-  N0 = pref0 * N0; N1 = pref0 * N1; N2 = pref0 * N2;
-  M0 = pref0 * M0; M1 = pref0 * M1; M2 = pref0 * M2;
-  const T twoM2 = two * M2;
-  const V3<T> Q = scl(M0, g.Aaa) + scl(M1, g.Abb) + scl(twoM2, g.Aab);
-  const V3<T> f1 = scl(N0, g.a1) + scl(N2, g.a2) - scl(dot(g.gc1, Q), g.n);
-  const V3<T> f2 = scl(N1, g.a2) + scl(N2, g.a1) - scl(dot(g.gc2, Q), g.n);
+  const R twoM2 = pow2(M[2], 2.f);
+  const V3<R> Q = lin3(M[0], g.Aaa, M[1], g.Abb, twoM2, g.Aab);
+  const V3<R> f1 = lin3(N[0], g.a1, N[2], g.a2, -dot(g.gc1, Q), g.n);
+  const V3<R> f2 = lin3(N[1], g.a2, N[2], g.a1, -dot(g.gc2, Q), g.n);
   f[0] = f1.x; f[1] = f1.y; f[2] = f1.z;
   f[3] = f2.x; f[4] = f2.y; f[5] = f2.z;
-  f[6] = -(M0 * g.n.x); f[7] = -(M0 * g.n.y); f[8] = -(M0 * g.n.z);
-  f[9] = -(M1 * g.n.x); f[10] = -(M1 * g.n.y); f[11] = -(M1 * g.n.z);
+  f[6] = -(M[0] * g.n.x); f[7] = -(M[0] * g.n.y); f[8] = -(M[0] * g.n.z);
+  f[9] = -(M[1] * g.n.x); f[10] = -(M[1] * g.n.y); f[11] = -(M[1] * g.n.z);
   f[12] = -(twoM2 * g.n.x); f[13] = -(twoM2 * g.n.y); f[14] = -(twoM2 * g.n.z);
 }
 
-/* f(y): the 15 force components of the element.
-   ref points at the element's first SoA constant (type R); stride = ne. */
-template <class T, class R>
-__host__ __device__ __forceinline__ void elem_forces(const T y[15], const EPar<R> &p, const R *ref, int stride,
-                                                     T f[15], int &status, R *gm_out = nullptr, R *tape_out = nullptr,
-                                                     R *gp_out = nullptr)
+/* The thickness-integrated resultants N = (N11, N22, N12) and M, scaled by
+   pref0; ref is the element's column of constants.  With
+   `grad`, out(q, w, th3, C) receives each thickness point's stress gradient
+   (qp_stress), w the point's weight times pref0. */
+template <class R, class Grad>
+__host__ __device__ __forceinline__ void elem_resultants(const ElemGeom<R> &g, const EPar<R> &p, const RefCol<R> &ref,
+                                                         R N[3], R M[3], int &status, bool final_update,
+                                                         bool grad, Grad out)
 {
-  const ElemGeom<T> g = elem_geom<T, R>(y, p);
   const int nq = p.nq;
-  const R gam = ref[(size_t)(kRefPerQp * nq + 0) * stride];
-  const R gamp = ref[(size_t)(kRefPerQp * nq + 1) * stride];
-  const R c1 = ref[(size_t)(kRefPerQp * nq + 2) * stride];
-  const R pref0 = ref[(size_t)(kRefPerQp * nq + 3) * stride];
-  const T zero = T{R(0)};
-  T N0 = zero, N1 = zero, N2 = zero, M0 = zero, M1 = zero, M2 = zero;
+  const R pref0 = ref(kRefPerQp * nq);
+  for (int i = 0; i < 3; i++) N[i] = M[i] = R(0);
   for (int q = 0; q < nq; q++) {
-    const QpRef<R> r = load_qpref(ref, stride, q);
     const R th3 = p.hhalf * p.theta[q];
-    T gm[6];
+    R gm[5], sv[3] = {R(0), R(0), R(0)};
     qp_metric(g, th3, gm);
-    if (gm_out)   /* the metric of every thickness point, SoA over elements, for the tangent */
-      for (int c = 0; c < 6; c++) gm_out[(size_t)(6 * q + c) * stride] = val(gm[c]);
-    T sv[3];
-    qp_stress(gm, r, gam, gamp, c1, p.mu, p.K, p.iters, sv, status, (T *)nullptr, true,
-              tape_out ? tape_out + (size_t)q * tape_per_qp(p.iters) * stride : nullptr, (size_t)stride);
+    R C[3][5] = {};
+    qp_stress<R>(gm, ref.at(kRefPerQp * q), p.mu, p.K, p.iters, sv, status, nullptr, final_update, grad, C);
+    if (grad) out(q, pref0 * p.w[q], th3, C);
     const R wq = p.w[q], wt = p.w[q] * th3;
-    N0 = N0 + wq * sv[0]; N1 = N1 + wq * sv[1]; N2 = N2 + wq * sv[2];
-    M0 = M0 + wt * sv[0]; M1 = M1 + wt * sv[1]; M2 = M2 + wt * sv[2];
+    for (int i = 0; i < 3; i++) { N[i] = mad(wq, sv[i], N[i]); M[i] = mad(wt, sv[i], M[i]); }
   }
-  if (gp_out) elem_res_store(g, N0, N1, N2, M0, M1, M2, pref0, gp_out, (size_t)stride);
-  elem_out(g, N0, N1, N2, M0, M1, M2, pref0, f);
+  for (int i = 0; i < 3; i++) { N[i] = pref0 * N[i]; M[i] = pref0 * M[i]; }
+}
+
+/* f(y): the 15 force components of the element. */
+template <class R>
+__host__ __device__ __forceinline__ void elem_forces(const R y[15], const EPar<R> &p, const RefCol<R> &ref, R f[15],
+                                                     int &status)
+{
+  const ElemGeom<R> g = elem_geom<R>(y, p);
+  R N[3], M[3];
+  elem_resultants<R>(g, p, ref, N, M, status, true, false, [](int, R, R, R(*)[5]) {});
+  elem_out(g, N, M, f);
 }
 
 /* UpdateElementThickness (active_strain.c:2198-2224): h0 sqrt(C33) with C33
    the mean over the thickness points of C33 after the sub-iterations (1 when
    that mean is not positive). */
 template <class R>
-__host__ __device__ __forceinline__ R elem_thickness(const R y[15], const EPar<R> &p, const R *ref, int stride, R h0,
+__host__ __device__ __forceinline__ R elem_thickness(const R y[15], const EPar<R> &p, const RefCol<R> &ref, R h0,
                                                      int &status)
 {
-  const ElemGeom<R> g = elem_geom<R, R>(y, p);
+  const ElemGeom<R> g = elem_geom<R>(y, p);
   const int nq = p.nq;
-  const R gam = ref[(size_t)(kRefPerQp * nq + 0) * stride];
-  const R gamp = ref[(size_t)(kRefPerQp * nq + 1) * stride];
-  const R c1 = ref[(size_t)(kRefPerQp * nq + 2) * stride];
   R sum = R(0);
   for (int q = 0; q < nq; q++) {
-    const QpRef<R> r = load_qpref(ref, stride, q);
-    R gm[6], sv[3], c33 = R(1);
+    R gm[5], sv[3], c33 = R(1);
     qp_metric(g, p.hhalf * p.theta[q], gm);
-    qp_stress(gm, r, gam, gamp, c1, p.mu, p.K, p.iters, sv, status, &c33);
+    qp_stress<R>(gm, ref.at(kRefPerQp * q), p.mu, p.K, p.iters, sv, status, &c33);
     sum += c33;
   }
   const R C33 = nq > 0 ? sum / (R)nq : R(1);
   return h0 * (C33 > R(0) ? sqrt(C33) : R(1));
 }
 
-/* Metric components the stress is differentiated along: 00 11 01 02 12.  The
-   sixth, g33 = n.n, is 1 for every y (d(n.n) = 2 n.dn = 0), so its column of
-   the constitutive derivative is never used; with the tangential thickness
-   metric g_alpha.n = (a_alpha + th a3,alpha).n is 0 for every y as well, which
-   leaves 00 11 01. */
-template <class R>
-__host__ __device__ __forceinline__ int metric_dirs(const EPar<R> &p) { return p.tnormal ? 3 : 5; }
+/* ---------------- element tangent D = df/dy ---------------- */
+/* The stress of every thickness point depends on y only through eight
+   scalars: the mid-surface metric a11, a22, a12, the curvature components
+   b11 = n.Aaa, b22 = n.Abb, b12 = n.Aab and kappa1, kappa2, the normal parts
+   of a3,alpha:
+     a3,1 = kappa1 n - b11 gc1 - b12 gc2,  a3,2 = kappa2 n - b12 gc1 - b22 gc2,
+     kappa1 = G^1_11 + G^2_12,  kappa2 = G^1_12 + G^2_22,  G^c_ab = gc_c . A_ab
+   (kappa = 0 with the tangential thickness metric), so that
+     g00 = a11 - 2 th b11 + th^2 h11 (g11, g01 alike),  g02 = th kappa1,
+     g12 = th kappa2,  h_ab = kappa_a kappa_b + b_ac a^cd b_db,
+   and the force is f.dy = N:da/2 - M:db, i.e. f1 = N11 a1 + N12 a2 - q1 n,
+   f3 = -M11 n, ..., q_c = M:G^c.  Hence D needs the 6 x 8 derivative H of the
+   resultants along the eight scalars, whose y-derivatives are short
+   combinations of a1, a2, n, gc1, gc2 (dn = -gc_c (n.da_c),
+   dgc_c = -gc_d (gc_c.da_d) + a^cd n (n.da_d)), and rank-one terms:
+     D = sum_m phi_m (x) dR_m  +  terms with the resultants held fixed.
+   tangent_coefs forms H and the combination coefficients once per element
+   (one thread), tangent_block the 15 x 3 block of columns of one of
+   a1, a2, Aaa, Abb, Aab (one lane each).  About 1,300 + 5 x 245 operations
+   at three thickness points; the forward-mode form this replaced took 16
+   lanes of 600 instructions per element. */
+enum {   /* per resultant m = N11, N22, N12, M11, M22, 2 M12 (base kTcRow m) */
+  kTcA1 = 0, kTcA2, kTcA12, kTcZ1, kTcZ2, kTcX11, kTcX12, kTcX21, kTcX22, kTcB11, kTcB22, kTcB12, kTcK1, kTcK2
+};
+constexpr int kTcRow = 14;
+constexpr int kTcVec = 6 * kTcRow;       /* a1, a2, n, gc1, gc2 */
+constexpr int kTcRes = kTcVec + 15;      /* N11 N22 N12 M11 M22 2M12 */
+constexpr int kTcQ = kTcRes + 6;         /* q1 q2 */
+constexpr int kTcGam = kTcQ + 2;         /* G^1_11 G^1_22 G^1_12, G^2_11 G^2_22 G^2_12 */
+constexpr int kTcE = kTcGam + 6;         /* (M:b) times a^11, a^12, a^22 */
+static_assert(kTcE + 3 == kTanCoefs, "tangent coefficient block");
 
-/* Jobs (q, k0..k0+KD-1) of the split tangent: stress of thickness point q
-   with KD metric directions (the last job of a point may carry unused
-   directions); jac layout as in elem_forces_split. */
-template <class R, int KD>
-__device__ __forceinline__ void constitutive_jobs(const ElemGeom<R> *g0, const R *gmq, const EPar<R> &p, const R *ref,
-                                                  int stride, int lane, R gam, R gamp, R c1, R *jac, int &status)
-{
-  typedef DK<R, KD> T;
-  const int ndirs = metric_dirs(p);
-  const int per_q = (ndirs + KD - 1) / KD;
-  for (int job = lane; job < per_q * p.nq; job += 16) {
-    const int q = job / per_q, k0 = (job - per_q * q) * KD;
-    R gmv[6];
-    if (gmq) {
-#pragma unroll
-      for (int c = 0; c < 6; c++) gmv[c] = gmq[(size_t)(6 * q + c) * stride];
-    } else {
-      qp_metric(*g0, p.hhalf * p.theta[q], gmv);
-    }
-    T gm[6];
-#pragma unroll
-    for (int c = 0; c < 6; c++) {
-      gm[c].v = gmv[c];
-#pragma unroll
-      for (int i = 0; i < KD; i++) gm[c].d[i] = (c == k0 + i && c < ndirs) ? R(1) : R(0);
-    }
-    T sv[3];
-    /* the stress only: the residual kernel of the same call checks the last CC3333 */
-    qp_stress(gm, load_qpref(ref, stride, q), gam, gamp, c1, p.mu, p.K, p.iters, sv, status, (T *)nullptr, false);
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-#pragma unroll
-      for (int t = 0; t < KD; t++)
-        if (k0 + t < ndirs) jac[q * 21 + 6 * i + k0 + t] = sv[i].d[t];
-    }
-    if (k0 == 0) {
-#pragma unroll
-      for (int i = 0; i < 3; i++) jac[q * 21 + 18 + i] = sv[i].v;
-    }
-  }
-}
-
-/* Element forces and their derivative along y_lane, for a group of 16 lanes
-   sharing one element (lane l < 15 carries direction l of y).  The
-   constitutive update depends on y only through the 6 metric components of
-   each thickness point, so it is differentiated along those: job (q, k) =
-   derivative of the stress of point q along metric component k, one job per
-   lane per round; each lane then applies the chain rule with its own metric
-   derivative.  That is 5 nq (3 nq with the tangential thickness metric)
-   constitutive derivative directions per element instead of 16 nq.  The primal values are the plain R-precision evaluation.
-   jac: this group's scratch, kMaxQp * 21 values; the 16 lanes of the group
-   and the other group of the warp must all call this (it synchronises the
-   warp). */
-template <class R>
-__device__ __forceinline__ void elem_forces_split(const R y[15], const EPar<R> &p, const R *ref, int stride, int lane,
-                                                  R *jac, D1<R> f[15], int &status, const R *gmq = nullptr)
-{
-  typedef D1<R> T;
-  const int nq = p.nq;
-  const R gam = ref[(size_t)(kRefPerQp * nq + 0) * stride];
-  const R gamp = ref[(size_t)(kRefPerQp * nq + 1) * stride];
-  const R c1 = ref[(size_t)(kRefPerQp * nq + 2) * stride];
-  const R pref0 = ref[(size_t)(kRefPerQp * nq + 3) * stride];
-  /* constitutive derivatives: jac[q*21 + 6*i + k] = d sv_i / d gm_k (k < ndirs),
-     jac[q*21 + 18 + i] = sv_i; FP64: KD metric directions per job, the fewest
-     for which the ceil(ndirs / KD) nq jobs fit one round of 16 lanes */
+/* Moments of the stress gradients over the thickness points:
+   T[k][3 i + c] = sum w th^k C_i,c (c = 00, 11, 01), U[k][2 i + c] the same
+   of the 02 and 12 columns for th^1 and th^2. */
+template <class R> struct TanMoments {
+  R T[4][9], U[2][6];
+  __host__ __device__ __forceinline__ void clear()
   {
-    /* the primal metric of each thickness point: stored by the residual
-       kernel of the same call (gmq), or from the element geometry here */
-    ElemGeom<R> g0;
-    if (!gmq) g0 = elem_geom<R, R>(y, p);
-    if constexpr (sizeof(R) == 4) {
-      /* FP32: one direction per job (wider duals spill under the FP32 kernel's register cap) */
-      constitutive_jobs<R, 1>(&g0, gmq, p, ref, stride, lane, gam, gamp, c1, jac, status);
-    } else {
-      const int ndirs = metric_dirs(p);
-      if (ndirs * nq <= 16) constitutive_jobs<R, 1>(&g0, gmq, p, ref, stride, lane, gam, gamp, c1, jac, status);
-      else if (((ndirs + 1) / 2) * nq <= 16) constitutive_jobs<R, 2>(&g0, gmq, p, ref, stride, lane, gam, gamp, c1, jac, status);
-      else constitutive_jobs<R, 3>(&g0, gmq, p, ref, stride, lane, gam, gamp, c1, jac, status);
-    }
-  }
-  __syncwarp();
-  const int ndirs = metric_dirs(p);
-  T yd[15];
 #pragma unroll
-  for (int c = 0; c < 15; c++) yd[c] = T{y[c], c == lane ? R(1) : R(0)};
-  const ElemGeom<T> g = elem_geom<T, R>(yd, p);
-  const T zero = T{R(0), R(0)};
-  T N0 = zero, N1 = zero, N2 = zero, M0 = zero, M1 = zero, M2 = zero;
-  for (int q = 0; q < nq; q++) {
-    const R th3 = p.hhalf * p.theta[q];
-    T gm[6];
-    qp_metric(g, th3, gm);
-    T sv[3];
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int i = 0; i < 9; i++) T[k][i] = R(0);
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+#pragma unroll
+      for (int i = 0; i < 6; i++) U[k][i] = R(0);
+  }
+  __host__ __device__ __forceinline__ void add(R w, R th, const R C[3][5])
+  {
+    const R w1 = w * th, w2 = w1 * th, w3 = w2 * th;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-      R d = R(0);
 #pragma unroll
-      for (int c = 0; c < 5; c++)
-        if (c < ndirs) d += jac[q * 21 + 6 * i + c] * gm[c].d;
-      sv[i] = T{jac[q * 21 + 18 + i], d};
+      for (int c = 0; c < 3; c++) {
+        T[0][3 * i + c] += w * C[i][c]; T[1][3 * i + c] += w1 * C[i][c];
+        T[2][3 * i + c] += w2 * C[i][c]; T[3][3 * i + c] += w3 * C[i][c];
+      }
+#pragma unroll
+      for (int c = 0; c < 2; c++) { U[0][2 * i + c] += w1 * C[i][3 + c]; U[1][2 * i + c] += w2 * C[i][3 + c]; }
     }
-    const R wq = p.w[q], wt = p.w[q] * th3;
-    N0 = N0 + wq * sv[0]; N1 = N1 + wq * sv[1]; N2 = N2 + wq * sv[2];
-    M0 = M0 + wt * sv[0]; M1 = M1 + wt * sv[1]; M2 = M2 + wt * sv[2];
   }
-  elem_out(g, N0, N1, N2, M0, M1, M2, pref0, f);
+};
+
+/* st(k, value) for every k < kTanCoefs */
+template <class R, class Store>
+__host__ __device__ __forceinline__ void tangent_coefs(const ElemGeom<R> &g, const R N[3], const R M[3],
+                                                       const TanMoments<R> &mo, int tnormal, Store st)
+{
+  const R two = R(2);
+  const R b11 = dot(g.n, g.Aaa), b22 = dot(g.n, g.Abb), b12 = dot(g.n, g.Aab);
+  const R G11 = dot(g.gc1, g.gc1), G22 = dot(g.gc2, g.gc2), G12 = dot(g.gc1, g.gc2);
+  const R s111 = dot(g.gc1, g.Aaa), s122 = dot(g.gc1, g.Abb), s112 = dot(g.gc1, g.Aab);   /* G^1_11 G^1_22 G^1_12 */
+  const R s211 = dot(g.gc2, g.Aaa), s222 = dot(g.gc2, g.Abb), s212 = dot(g.gc2, g.Aab);
+  const R k1 = tnormal ? R(0) : s111 + s212, k2 = tnormal ? R(0) : s112 + s222;
+  /* b^c_a = a^cd b_da */
+  const R m11 = G11 * b11 + G12 * b12, m21 = G12 * b11 + G22 * b12;
+  const R m12 = G11 * b12 + G12 * b22, m22 = G12 * b12 + G22 * b22;
+  /* dh along (a11, a22, a12) and (b11, b22, b12), rows h11, h22, h12 */
+  const R ha[3][3] = {{-(m11 * m11), -(m21 * m21), -(two * m11 * m21)},
+                      {-(m12 * m12), -(m22 * m22), -(two * m12 * m22)},
+                      {-(m11 * m12), -(m21 * m22), -(m11 * m22 + m21 * m12)}};
+  const R hb[3][3] = {{two * m11, R(0), two * m21}, {R(0), two * m22, two * m12}, {m12, m21, m11 + m22}};
+#pragma unroll
+  for (int m = 0; m < 6; m++) {
+    const int i = m % 3, t = m / 3;                 /* N rows take th^0..2, M rows th^1..3 */
+    const R sc = m == 5 ? two : R(1);
+    R Ha[3], Hb[3];
+    const R h0 = mo.T[t + 2][3 * i], h1 = mo.T[t + 2][3 * i + 1], h2 = mo.T[t + 2][3 * i + 2];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      Ha[c] = sc * (mo.T[t][3 * i + c] + (h0 * ha[0][c] + h1 * ha[1][c] + h2 * ha[2][c]));
+      Hb[c] = sc * ((h0 * hb[0][c] + h1 * hb[1][c] + h2 * hb[2][c]) - two * mo.T[t + 1][3 * i + c]);
+    }
+    const R Hk1 = tnormal ? R(0) : sc * (mo.U[t][2 * i] + two * k1 * h0 + k2 * h2);
+    const R Hk2 = tnormal ? R(0) : sc * (mo.U[t][2 * i + 1] + two * k2 * h1 + k1 * h2);
+    const int o = kTcRow * m;
+    st(o + kTcA1, two * Ha[0]); st(o + kTcA2, two * Ha[1]); st(o + kTcA12, Ha[2]);
+    st(o + kTcZ1, (Hk1 * m11 + Hk2 * m12) - (Hb[0] * s111 + Hb[1] * s122 + Hb[2] * s112));
+    st(o + kTcZ2, (Hk1 * m21 + Hk2 * m22) - (Hb[0] * s211 + Hb[1] * s222 + Hb[2] * s212));
+    st(o + kTcX11, -(Hk1 * s111 + Hk2 * s112)); st(o + kTcX12, -(Hk1 * s112 + Hk2 * s122));
+    st(o + kTcX21, -(Hk1 * s211 + Hk2 * s212)); st(o + kTcX22, -(Hk1 * s212 + Hk2 * s222));
+    st(o + kTcB11, Hb[0]); st(o + kTcB22, Hb[1]); st(o + kTcB12, Hb[2]);
+    st(o + kTcK1, Hk1); st(o + kTcK2, Hk2);
+  }
+  const V3<R> v[5] = {g.a1, g.a2, g.n, g.gc1, g.gc2};
+#pragma unroll
+  for (int k = 0; k < 5; k++) { st(kTcVec + 3 * k, v[k].x); st(kTcVec + 3 * k + 1, v[k].y); st(kTcVec + 3 * k + 2, v[k].z); }
+  const R M2 = two * M[2];
+  st(kTcRes, N[0]); st(kTcRes + 1, N[1]); st(kTcRes + 2, N[2]);
+  st(kTcRes + 3, M[0]); st(kTcRes + 4, M[1]); st(kTcRes + 5, M2);
+  st(kTcQ, M[0] * s111 + M[1] * s122 + M2 * s112); st(kTcQ + 1, M[0] * s211 + M[1] * s222 + M2 * s212);
+  st(kTcGam, s111); st(kTcGam + 1, s122); st(kTcGam + 2, s112);
+  st(kTcGam + 3, s211); st(kTcGam + 4, s222); st(kTcGam + 5, s212);
+  const R mb = M[0] * b11 + M[1] * b22 + M2 * b12;
+  st(kTcE, mb * G11); st(kTcE + 1, mb * G12); st(kTcE + 2, mb * G22);
 }
 
-/* constitutive_jobs in derivative-only form: the primal metric (gmq) and the
-   primal C33 sub-iteration values (tape) come from the residual kernel. */
-template <class R, int KD>
-__device__ __forceinline__ void constitutive_jobs_tl(const R *gmq, const R *tape, const EPar<R> &p, const R *ref,
-                                                     int stride, int lane, R gam, R gamp, R c1, R *jac)
+/* Columns 3 s .. 3 s + 2 of D (s = 0..4: a1, a2, Aaa, Abb, Aab) from the
+   coefficients ld(k): D[row][j]. */
+template <class R, class Load>
+__host__ __device__ __forceinline__ void tangent_block(int s, Load ld, R D[15][3])
 {
-  const int ndirs = metric_dirs(p);
-  const int per_q = (ndirs + KD - 1) / KD;
-  const int tq = tape_per_qp(p.iters);
-  for (int job = lane; job < per_q * p.nq; job += 16) {
-    const int q = job / per_q, k0 = (job - per_q * q) * KD;
-    R gmv[6], dgm[6][KD];
+  auto vec = [&](int k) { return V3<R>{ld(kTcVec + 3 * k), ld(kTcVec + 3 * k + 1), ld(kTcVec + 3 * k + 2)}; };
+  const V3<R> a1 = vec(0), a2 = vec(1), n = vec(2), g1 = vec(3), g2 = vec(4);
+  const R zero = R(0);
+  const bool t = s < 2;                              /* a tangent's columns */
+  /* dR_m along the columns = c1 a1 + c2 a2 + c3 n + c4 gc1 + c5 gc2 */
+  const int i1 = s == 0 ? kTcA1 : kTcA12, i2 = s == 0 ? kTcA12 : kTcA2;
+  const int i3 = s == 0 ? kTcZ1 : s == 1 ? kTcZ2 : s == 2 ? kTcB11 : s == 3 ? kTcB22 : kTcB12;
+  const int i4 = s == 0 ? kTcX11 : s == 1 ? kTcX21 : s == 2 ? kTcK1 : kTcK2;
+  const int i5 = s == 0 ? kTcX12 : s == 1 ? kTcX22 : s == 3 ? kTcK2 : kTcK1;
+  V3<R> dR[6];
 #pragma unroll
-    for (int c = 0; c < 6; c++) {
-      gmv[c] = gmq[(size_t)(6 * q + c) * stride];
+  for (int m = 0; m < 6; m++) {
+    const int o = kTcRow * m;
+    const R c1 = t ? ld(o + i1) : zero, c2 = t ? ld(o + i2) : zero, c3 = ld(o + i3);
+    const R c4 = s == 3 ? zero : ld(o + i4), c5 = s == 2 ? zero : ld(o + i5);
+    dR[m] = scl(c1, a1) + scl(c2, a2) + scl(c3, n) + scl(c4, g1) + scl(c5, g2);
+  }
+  const R q1 = ld(kTcQ), q2 = ld(kTcQ + 1);
+  /* dq_c = sum_m G^c_m dM_m, plus M:dG^c: -q_s gc_c + (M:b) a^cs n for a tangent, M_m gc_c for A_m */
+  const R kg = s == 0 ? -q1 : s == 1 ? -q2 : ld(kTcRes + 1 + s);
+  const R n1 = t ? ld(kTcE + s) : zero, n2 = t ? ld(kTcE + 1 + s) : zero;
+  V3<R> dq1 = scl(kg, g1) + scl(n1, n), dq2 = scl(kg, g2) + scl(n2, n);
 #pragma unroll
-      for (int i = 0; i < KD; i++) dgm[c][i] = (c == k0 + i && c < ndirs) ? R(1) : R(0);
-    }
-    R sv[3], dsv[3][KD];
-    qp_stress_tl<R, KD>(gmv, dgm, load_qpref(ref, stride, q), gam, gamp, c1, p.mu, p.K, p.iters,
-                        tape + (size_t)q * tq * stride, (size_t)stride, sv, dsv);
-    /* columns g00 and g11 doubled: the chain rule forms d g00 / 2 = dg1.g1 and d g11 / 2 = dg2.g2 */
+  for (int m = 0; m < 3; m++) {
+    dq1 = dq1 + scl(ld(kTcGam + m), dR[3 + m]);
+    dq2 = dq2 + scl(ld(kTcGam + 3 + m), dR[3 + m]);
+  }
+  const V3<R> gs = t ? (s == 0 ? g1 : g2) : V3<R>{zero, zero, zero};
+  const R a1c[3] = {a1.x, a1.y, a1.z}, a2c[3] = {a2.x, a2.y, a2.z}, nc[3] = {n.x, n.y, n.z}, gc[3] = {gs.x, gs.y, gs.z};
+  auto row = [&](const V3<R> &v, int j) { return j == 0 ? v.x : j == 1 ? v.y : v.z; };
+  const R N0 = ld(kTcRes), N1 = ld(kTcRes + 1), N2 = ld(kTcRes + 2);
+  const R M0 = ld(kTcRes + 3), M1 = ld(kTcRes + 4), M2 = ld(kTcRes + 5);
+  const R e1 = s == 0 ? N0 : s == 1 ? N2 : zero, e2 = s == 0 ? N2 : s == 1 ? N1 : zero;
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    /* minus the coefficient of n_i, and of gc_s,i */
+    const R nj = row(n, j);
+    const R p1 = row(dq1, j), p2 = row(dq2, j), p3 = row(dR[3], j), p4 = row(dR[4], j), p5 = row(dR[5], j);
+    const R w1 = q1 * nj, w2 = q2 * nj, w3 = M0 * nj, w4 = M1 * nj, w5 = M2 * nj;
+    const R v0 = row(dR[0], j), v1 = row(dR[1], j), v2 = row(dR[2], j);
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-#pragma unroll
-      for (int t = 0; t < KD; t++)
-        if (k0 + t < ndirs) jac[q * 21 + 6 * i + k0 + t] = k0 + t < 2 ? R(2) * dsv[i][t] : dsv[i][t];
-    }
-    if (k0 == 0) {
-#pragma unroll
-      for (int i = 0; i < 3; i++) jac[q * 21 + 18 + i] = sv[i];
+      D[i][j] = a1c[i] * v0 + a2c[i] * v2 + gc[i] * w1 - nc[i] * p1 + (i == j ? e1 : zero);
+      D[3 + i][j] = a2c[i] * v1 + a1c[i] * v2 + gc[i] * w2 - nc[i] * p2 + (i == j ? e2 : zero);
+      D[6 + i][j] = gc[i] * w3 - nc[i] * p3;
+      D[9 + i][j] = gc[i] * w4 - nc[i] * p4;
+      D[12 + i][j] = gc[i] * w5 - nc[i] * p5;
     }
   }
-}
-
-/* The chain rule of elem_forces_split along y_lane in tangent-linear form: the
-   primal geometry and resultants come from the residual kernel (gp, SoA
-   stride: elem_geom_store, elem_res_store), the stress derivatives from the
-   constitutive jobs (jac), so only derivatives are computed here.  Lane
-   3 r + c carries the unit direction of component c of the r-th of
-   (a1, a2, Aaa, Abb, Aab) (lane 15: none), and every product with it is a
-   selection (one-hot helpers above).  The derivatives follow elem_geom,
-   qp_metric and elem_out operation by operation:
-     dcr = da1 x a2 + a1 x da2,  d|cr| = n.dcr (= t1_c or t2_c),
-     dn = (dcr - n d|cr|)/|cr|,  d(1/|cr|) = -d|cr|/|cr|^2,
-     dt1 = da2 x n + a2 x dn,  d(1/(a1.t1)) = -(da1.t1 + a1.dt1)/(a1.t1)^2, ...
-   df holds d f_r / d y_lane. */
-template <class R>
-__device__ __forceinline__ void elem_forces_split_tl(const R y[15], const EPar<R> &p, const R *ref, int stride,
-                                                     const R *gp, int lane, R *jac, R df[15], const R *gmq,
-                                                     const R *tape)
-{
-  const int nq = p.nq;
-  const R gam = ref[(size_t)(kRefPerQp * nq + 0) * stride];
-  const R gamp = ref[(size_t)(kRefPerQp * nq + 1) * stride];
-  const R c1 = ref[(size_t)(kRefPerQp * nq + 2) * stride];
-  const R pref0 = ref[(size_t)(kRefPerQp * nq + 3) * stride];
-  const int ndirs = metric_dirs(p);
-  if (ndirs * nq <= 16) constitutive_jobs_tl<R, 1>(gmq, tape, p, ref, stride, lane, gam, gamp, c1, jac);
-  else if (((ndirs + 1) / 2) * nq <= 16) constitutive_jobs_tl<R, 2>(gmq, tape, p, ref, stride, lane, gam, gamp, c1, jac);
-  else constitutive_jobs_tl<R, 3>(gmq, tape, p, ref, stride, lane, gam, gamp, c1, jac);
-  __syncwarp();
-  const R zero = R(0), one = R(1), two = R(2);
-  R g[kGeomPrimal];
-#pragma unroll
-  for (int k = 0; k < kGeomPrimal; k++) g[k] = gp[(size_t)k * stride];
-  const V3<R> n = {g[0], g[1], g[2]}, t1 = {g[4], g[5], g[6]}, t2 = {g[7], g[8], g[9]};
-  const R icn = g[3], s1 = g[10], s2 = g[11];
-  const V3<R> u31 = {g[12], g[13], g[14]}, u32 = {g[15], g[16], g[17]};
-  const R N0 = g[18], N1 = g[19], N2 = g[20], M0 = g[21], M1 = g[22], M2 = g[23];   /* pref0-scaled */
-  const V3<R> Q = {g[24], g[25], g[26]};
-  const R q1 = g[27], q2 = g[28];
-  const V3<R> gc1 = {g[29], g[30], g[31]}, gc2 = {g[32], g[33], g[34]};
-  const V3<R> a1 = {y[0], y[1], y[2]}, a2 = {y[3], y[4], y[5]};
-  const V3<R> Aaa = {y[6], y[7], y[8]}, Abb = {y[9], y[10], y[11]}, Aab = {y[12], y[13], y[14]};
-  const int r = lane / 3, c = lane - 3 * r;
-  /* geometry */
-  const V3<R> dcr = sel_sign(ecross(c, r == 0 ? a2 : a1), r < 2, r == 1);
-  const R dcn = r == 0 ? comp(t1, c) : (r == 1 ? comp(t2, c) : zero);
-  const V3<R> dn = scl(icn, dcr - scl(dcn, n));
-  const R dicn = -(icn * icn) * dcn;
-  const V3<R> dt1 = cross_acc(a2, dn, sel_sign(ecross(c, n), r == 1, false));
-  const R ds1 = -(s1 * s1) * dot_acc(a1, dt1, r == 0 ? comp(t1, c) : zero);
-  const V3<R> dgc1 = scl(ds1, t1) + scl(s1, dt1);
-  const V3<R> dt2 = cross_acc(dn, a1, sel_sign(ecross(c, n), r == 0, true));
-  const R ds2 = -(s2 * s2) * dot_acc(a2, dt2, r == 1 ? comp(t2, c) : zero);
-  const V3<R> dgc2 = scl(ds2, t2) + scl(s2, dt2);
-  /* du31 = dAaa x a2 + Aaa x da2 + da1 x Aab + a1 x dAab and
-     du32 = dAab x a2 + Aab x da2 + da1 x Abb + a1 x dAbb: one term each */
-  const V3<R> v31 = r == 0 ? Aab : (r == 1 ? Aaa : (r == 2 ? a2 : a1));
-  const V3<R> du31 = sel_sign(ecross(c, v31), r < 3 || r == 4, r == 1 || r == 4);
-  const V3<R> v32 = r == 0 ? Abb : (r == 1 ? Aab : (r == 3 ? a1 : a2));
-  const V3<R> du32 = sel_sign(ecross(c, v32), r < 2 || r == 3 || r == 4, r == 1 || r == 3);
-  V3<R> a31 = scl(icn, u31), a32 = scl(icn, u32);
-  V3<R> da31 = scl(icn, du31) + scl(dicn, u31), da32 = scl(icn, du32) + scl(dicn, u32);
-  if (p.tnormal) {   /* a3,alpha - (a3,alpha . n) n */
-    const R p31 = dot(a31, n), p32 = dot(a32, n);
-    const R dp31 = dot(da31, n) + dot(a31, dn), dp32 = dot(da32, n) + dot(a32, dn);
-    da31 = da31 - scl(dp31, n) - scl(p31, dn);
-    da32 = da32 - scl(dp32, n) - scl(p32, dn);
-    a31 = a31 - scl(p31, n);
-    a32 = a32 - scl(p32, n);
-  }
-  const V3<R> da1 = {r == 0 && c == 0 ? one : zero, r == 0 && c == 1 ? one : zero, r == 0 && c == 2 ? one : zero};
-  const V3<R> da2 = {r == 1 && c == 0 ? one : zero, r == 1 && c == 1 ? one : zero, r == 1 && c == 2 ? one : zero};
-  /* resultant derivatives by the chain rule through each thickness point's metric */
-  R dN0 = zero, dN1 = zero, dN2 = zero, dM0 = zero, dM1 = zero, dM2 = zero;
-  for (int q = 0; q < nq; q++) {
-    const R th3 = p.hhalf * p.theta[q];
-    const V3<R> g1 = a1 + scl(th3, a31), g2 = a2 + scl(th3, a32);
-    const V3<R> dg1 = da1 + scl(th3, da31), dg2 = da2 + scl(th3, da32);
-    /* halves of d g00 and d g11: their stress columns are stored doubled */
-    const R dgm[5] = {dot(dg1, g1), dot(dg2, g2), dot_acc(g1, dg2, dot(dg1, g2)), dot_acc(g1, dn, dot(dg1, n)),
-                      dot_acc(g2, dn, dot(dg2, n))};
-    R dsv[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      R d = zero;
-#pragma unroll
-      for (int k = 0; k < 5; k++)
-        if (k < ndirs) d += jac[q * 21 + 6 * i + k] * dgm[k];
-      dsv[i] = d;
-    }
-    const R wq = p.w[q], wt = p.w[q] * th3;
-    dN0 = dN0 + wq * dsv[0]; dN1 = dN1 + wq * dsv[1]; dN2 = dN2 + wq * dsv[2];
-    dM0 = dM0 + wt * dsv[0]; dM1 = dM1 + wt * dsv[1]; dM2 = dM2 + wt * dsv[2];
-  }
-  /* elem_out */
-  dN0 = pref0 * dN0; dN1 = pref0 * dN1; dN2 = pref0 * dN2; dM0 = pref0 * dM0; dM1 = pref0 * dM1; dM2 = pref0 * dM2;
-  const R twoM2 = two * M2, dtwoM2 = two * dM2;
-  /* dQ = dM0 Aaa + M0 dAaa + dM1 Abb + M1 dAbb + d(2 M2) Aab + 2 M2 dAab */
-  const V3<R> dQ = add_at(scl(dM0, Aaa) + scl(dM1, Abb) + scl(dtwoM2, Aab), c,
-                          r == 2 ? M0 : (r == 3 ? M1 : (r == 4 ? twoM2 : zero)));
-  const R dq1 = dot_acc(gc1, dQ, dot(dgc1, Q)), dq2 = dot_acc(gc2, dQ, dot(dgc2, Q));
-  /* df1 = dN0 a1 + N0 da1 + dN2 a2 + N2 da2 - dq1 n - q1 dn,
-     df2 = dN1 a2 + N1 da2 + dN2 a1 + N2 da1 - dq2 n - q2 dn */
-  const V3<R> df1 = add_at(scl(dN0, a1) + scl(dN2, a2) - scl(dq1, n) - scl(q1, dn), c,
-                           r == 0 ? N0 : (r == 1 ? N2 : zero));
-  const V3<R> df2 = add_at(scl(dN1, a2) + scl(dN2, a1) - scl(dq2, n) - scl(q2, dn), c,
-                           r == 1 ? N1 : (r == 0 ? N2 : zero));
-  df[0] = df1.x; df[1] = df1.y; df[2] = df1.z;
-  df[3] = df2.x; df[4] = df2.y; df[5] = df2.z;
-  const V3<R> dm0 = scl(dM0, n) + scl(M0, dn), dm1 = scl(dM1, n) + scl(M1, dn), dm2 = scl(dtwoM2, n) + scl(twoM2, dn);
-  df[6] = -dm0.x; df[7] = -dm0.y; df[8] = -dm0.z;
-  df[9] = -dm1.x; df[10] = -dm1.y; df[11] = -dm1.z;
-  df[12] = -dm2.x; df[13] = -dm2.y; df[14] = -dm2.z;
 }
 
 /* ---------------- tangent contraction (row assembly) ---------------- */

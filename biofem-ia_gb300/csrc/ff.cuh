@@ -189,6 +189,33 @@ __host__ __device__ __forceinline__ double ff_widen(float f)
 /* hi + lo as a double: two exact widenings and one double addition. */
 __host__ __device__ __forceinline__ double ff_to_double_bits(FF a) { return ff_widen(a.hi) + ff_widen(a.lo); }
 
+/* A sum of products of float-float numbers, the heads' sum carried by two-sum
+   and every error (of the head product, the cross products, the two-sums) in
+   one float: 12 instructions a term against 27 for a product and a sum of
+   normalised numbers, with the same error bound, a few 2^-47 of the sum of the
+   terms' magnitudes. */
+struct FFAcc {
+  float hi, lo;
+  __host__ __device__ __forceinline__ FFAcc(FF c) : hi(c.hi), lo(c.lo) {}
+  __host__ __device__ __forceinline__ FFAcc(FF a, FF b)
+  {
+    hi = a.hi * b.hi;
+    lo = fmaf(a.lo, b.hi, fmaf(a.hi, b.lo, fmaf(a.hi, b.hi, -hi)));
+  }
+  __host__ __device__ __forceinline__ void add(FF a, FF b)
+  {
+    const float p = a.hi * b.hi;
+    const float e = fmaf(a.lo, b.hi, fmaf(a.hi, b.lo, fmaf(a.hi, b.hi, -p)));
+    const FF t = ff_two_sum(hi, p);
+    hi = t.hi;
+    lo += t.lo + e;
+  }
+  __host__ __device__ __forceinline__ FF get() const { return ff_two_sum(hi, lo); }
+};
+
+/* c x for a power of two c */
+__host__ __device__ __forceinline__ FF pow2(FF x, float c) { return FF(x.hi * c, x.lo * c); }
+
 /* s += a x for a float a and a float-float x: the head product a x.hi exact
    (two-product), added to s.hi by two-sum; the tails and a x.lo go to the
    low word (the accumulation of the float-float matvec). */

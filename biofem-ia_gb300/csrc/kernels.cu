@@ -8,15 +8,13 @@
  *   k_elem_residual  one thread per element: geometry, closed-form stress,
  *                    element forces Fb (ElemUpdFint) and the follower-pressure
  *                    corner force (SurfaceNormalPressure, external.c:589-624)
- *                    (and, for the FP64 tangent, the primal values its
- *                    derivative-only form reads: thickness-point metrics,
- *                    geometry, resultants, C33 sub-iteration values)
- *   k_elem_tangent   16 lanes per element: the stress is differentiated along
- *                    the metric components of each thickness point (one job
- *                    per lane), then lane j carries d/dy_j through the
- *                    geometry and the chain rule, giving column j of
- *                    D = df/dy, stored per element (kDeStride values, with the
- *                    follower-pressure corner vectors) for the row assembly
+ *                    (and, for the FP64 tangent, the stress gradients and the
+ *                    coefficients k_elem_tangent combines)
+ *   k_elem_tangent   five lanes per element, one per column block of
+ *                    D = df/dy, combined from the element's coefficients
+ *                    (element.cuh, tangent_block) and stored, with the
+ *                    follower-pressure corner vectors, for the row assembly
+ *   k_elem_tangent_f32  the FP32-bulk tangent, one thread per element
  *   k_elem_residual_ff  the FP32-bulk residual: k_elem_residual's element math
  *                    in float-float numbers on the FP32 pipe
  *   k_node_gather    one thread per node: Fint / Fext (and FDynamic's Fdyn)
@@ -78,23 +76,6 @@ __device__ __forceinline__ void gather_y(const double *pos, const int *patch, in
       y[3 * r] += c * x; y[3 * r + 1] += c * yy; y[3 * r + 2] += c * z;
     }
   }
-}
-
-/* gather_y for a group of 16 lanes sharing one element: lane l < 15 sums
-   component l (row l / 3, coordinate l % 3) in gather_y's order, then the
-   group exchanges the 15 sums, so every lane ends with gather_y's y at one
-   fifteenth of the FP64 work. */
-__device__ __forceinline__ void gather_y_group(const double *pos, const int *patch, int e, int nen, const double *tab,
-                                               int lane, double y[15])
-{
-  double s = 0.0;
-  if (lane < 15) {
-    const int r = lane / 3, d = lane - 3 * r;
-    const int *pe = patch + 16 * (size_t)e;
-    for (int i = 0; i < nen; i++) s += tab[r * 16 + i] * __ldg(pos + 4 * (size_t)__ldg(pe + i) + d);
-  }
-#pragma unroll
-  for (int c = 0; c < 15; c++) y[c] = __shfl_sync(0xffffffffu, s, c, 16);
 }
 
 /* ---------------- positions / ghosts ---------------- */
@@ -219,17 +200,33 @@ __global__ void k_ref_prep(DevMesh m, KParams p, const double *__restrict__ fib,
     double av[3], aw[3], ae[3];
     const double e3[3] = {0.0, 0.0, 1.0};
     aT(v, av); aT(w, aw); aT(e3, ae);
+    /* the stress's forms in (c00, c11, c01, c22): S^ij = mu (G^ij + c1 s_i s_j)
+       + alpha/2 (Ci + A Ci H)^ij with A = I - gam s t^T, H = I + gam' t s^T,
+       and Q_xy = (A^T x)^T Ci (A^T y) */
     double *o = eref + (size_t)kRefPerQp * q * ne + e;
-    o[0] = Gi[0][0] * ia2; o[1 * ne] = Gi[1][1] * ia2; o[2 * ne] = 0.5 * (Gi[0][1] + Gi[1][0]) * ia2;
-    o[3 * ne] = Gi[2][2] * ia2;
-    for (int k = 0; k < 3; k++) {
-      o[(4 + k) * ne] = s[k]; o[(7 + k) * ne] = t[k];
-      o[(11 + k) * ne] = av[k]; o[(14 + k) * ne] = aw[k]; o[(17 + k) * ne] = ae[k];
-    }
-    o[10 * ne] = rho;
+    auto form = [&](int k, double f00, double f11, double f01, double f22) {
+      o[(size_t)k * ne] = f00; o[(size_t)(k + 1) * ne] = f11; o[(size_t)(k + 2) * ne] = f01; o[(size_t)(k + 3) * ne] = f22;
+    };
+    auto quad = [&](int k, const double x[3], const double y[3]) {
+      form(k, x[0] * y[0], x[1] * y[1], x[0] * y[1] + x[1] * y[0], x[2] * y[2]);
+    };
+    const double gg = gam * gamp, dg = gamp - gam;
+    const double t00 = t[0] * t[0], t11 = t[1] * t[1], t01 = 2.0 * t[0] * t[1], t22 = t[2] * t[2];
+    const double g33 = gg * s[2] * s[2], g00 = gg * s[0] * s[0], g11 = gg * s[1] * s[1], g01 = gg * s[0] * s[1];
+    o[(size_t)kRfS33 * ne] = p.mu * (Gi[2][2] * ia2 + c1 * s[2] * s[2]);
+    o[(size_t)kRfS00 * ne] = p.mu * (Gi[0][0] * ia2 + c1 * s[0] * s[0]);
+    o[(size_t)kRfS11 * ne] = p.mu * (Gi[1][1] * ia2 + c1 * s[1] * s[1]);
+    o[(size_t)kRfS01 * ne] = p.mu * (0.5 * (Gi[0][1] + Gi[1][0]) * ia2 + c1 * s[0] * s[1]);
+    form(kRfB33, -g33 * t00, -g33 * t11, -g33 * t01, 2.0 + dg * s[2] * t[2] - g33 * t22);
+    form(kRfB00, 2.0 + dg * s[0] * t[0] - g00 * t00, -g00 * t11, dg * s[0] * t[1] - g00 * t01, -g00 * t22);
+    form(kRfB11, -g11 * t00, 2.0 + dg * s[1] * t[1] - g11 * t11, dg * s[1] * t[0] - g11 * t01, -g11 * t22);
+    form(kRfB01, gamp * s[1] * t[0] - g01 * t00, -gam * s[0] * t[1] - g01 * t11,
+         2.0 + gamp * s[1] * t[1] - gam * s[0] * t[0] - g01 * t01, -g01 * t22);
+    quad(kRfQvv, av, av); quad(kRfQww, aw, aw); quad(kRfQee, ae, ae);
+    quad(kRfQvw, av, aw); quad(kRfQve, av, ae); quad(kRfQwe, aw, ae);
+    o[(size_t)kRfRho * ne] = rho;
   }
-  double *o = eref + (size_t)kRefPerQp * p.nq * ne + e;
-  o[0] = gam; o[ne] = gamp; o[2 * ne] = c1; o[3 * ne] = 0.5 * (2.0 * p.hhalf) * dA0;
+  eref[(size_t)kRefPerQp * p.nq * ne + e] = 0.5 * (2.0 * p.hhalf) * dA0;   /* pref0 */
 }
 
 /* ---------------- residual element kernel ---------------- */
@@ -256,8 +253,29 @@ __device__ __forceinline__ void elem_pressure_force(const DevMesh &m, const KPar
   m.fp[2 * ne + e] = (ca.z / nrm) * p.pressure * dA / 3.;
 }
 
-__global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, double *__restrict__ gm_out,
-                                                       double *__restrict__ gp_out, double *__restrict__ tape_out)
+/* The pressure block vectors of one element (follower-pressure load
+   stiffness): every corner carries P/6 (x2-x1)x(x3-x1), so d/dx1 = [b-a]x,
+   d/dx2 = -[b]x, d/dx3 = [a]x with a = x2-x1, b = x3-x1; stored after D in
+   the element's block for the row assembly. */
+template <class R>
+__device__ __forceinline__ void store_pressure_vectors(const R av[3], const R bv[3], R *dst)
+{
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    dst[d] = bv[d] - av[d];
+    dst[3 + d] = -bv[d];
+    dst[6 + d] = av[d];
+  }
+}
+
+/* One thread per element.  For the R + K call (tan) it also evaluates the
+   stress gradients (about 300 FP64 operations a thickness point beside the
+   400 of the stress itself), keeps them in cq between the thickness loop and
+   the moments (its own column: 15 values a point would not fit in registers
+   beside the stress), and stores the kTanCoefs tangent coefficients
+   k_elem_tangent reads.  One kernel serves both calls, so that R is bit for
+   bit the same: two instances would contract multiply-adds differently. */
+__global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, bool tan)
 {
   __shared__ double tabs[kNumTables * 80];
   for (int i = threadIdx.x; i < kNumTables * 80; i += blockDim.x) tabs[i] = m.ntab[i];
@@ -272,12 +290,17 @@ __global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, dou
   double f[15];
   int st = 0;
   const EPar<double> ep = epar<double>(p);
-  elem_forces<double, double>(y, ep, m.eref + e, p.ne, f, st, gm_out ? gm_out + e : nullptr,
-                              tape_out ? tape_out + e : nullptr, gp_out ? gp_out + e : nullptr);
-  if (gp_out) elem_geom_store<double>(y, gp_out + e, (size_t)p.ne);   /* the tangent's primal geometry */
+  const size_t ne = p.ne;
+  const ElemGeom<double> g = elem_geom<double>(y, ep);
+  double N[3], M[3];
+  elem_resultants<double>(g, ep, RefCol<double>{m.eref + e, ne}, N, M, st, true, tan, [&](int q, double w, double, double C[3][5]) {
+    double *cq = m.cq + e;
+    for (int i = 0; i < 3; i++)
+      for (int k = 0; k < 5; k++) cq[(size_t)(15 * q + 5 * i + k) * ne] = w * C[i][k];
+  });
+  elem_out(g, N, M, f);
   set_status(m.status, st);
   /* Fb_a = sum_r N[r][a] f_r, stored slot-major: fb[(3a+d)*ne + e] */
-  const size_t ne = p.ne;
   for (int a = 0; a < nen; a++) {
     double fx = 0.0, fy = 0.0, fz = 0.0;
 #pragma unroll
@@ -290,6 +313,25 @@ __global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, dou
     m.fb[(3 * a + 2) * ne + e] = fz;
   }
   if (p.pressure != 0.0) elem_pressure_force(m, p, e);
+  if (tan) {
+    TanMoments<double> mo;
+    mo.clear();
+    for (int q = 0; q < ep.nq; q++) {
+      double C[3][5];
+      for (int i = 0; i < 3; i++)
+        for (int k = 0; k < 5; k++) C[i][k] = m.cq[(size_t)(15 * q + 5 * i + k) * ne + e];
+      mo.add(1.0, ep.hhalf * ep.theta[q], C);
+    }
+    double *tc = m.tcoef + e;
+    tangent_coefs<double>(g, N, M, mo, ep.tnormal, [&](int k, double v) { tc[(size_t)k * ne] = v; });
+    if (p.pressure != 0.0 && !p.pres_dead) {
+      double X[3][3];
+      for (int k = 0; k < 3; k++) load_node(m.pos, m.etri[3 * (size_t)e + k], X[k][0], X[k][1], X[k][2]);
+      const double av[3] = {X[1][0] - X[0][0], X[1][1] - X[0][1], X[1][2] - X[0][2]};
+      const double bv[3] = {X[2][0] - X[0][0], X[2][1] - X[0][1], X[2][2] - X[0][2]};
+      store_pressure_vectors<double>(av, bv, m.De + (size_t)kDeStride * e + kDePres);
+    }
+  }
 }
 
 /* ---------------- FP32-bulk residual (float-float) ---------------- */
@@ -317,181 +359,156 @@ __global__ void __launch_bounds__(128, 3) k_elem_residual_ff(DevMesh m, KParams 
   load_node(m.pos, m.etri[3 * (size_t)e], xc[0], xc[1], xc[2]);
   FF y[15];
   {
-    const FF c[3] = {ff_split(xc[0]), ff_split(xc[1]), ff_split(xc[2])};
+    FFAcc acc[15] = {
+#define BIOFEM_Y0(r) FFAcc(tsum[r], ff_split(xc[0])), FFAcc(tsum[r], ff_split(xc[1])), FFAcc(tsum[r], ff_split(xc[2]))
+        BIOFEM_Y0(0), BIOFEM_Y0(1), BIOFEM_Y0(2), BIOFEM_Y0(3), BIOFEM_Y0(4)
+#undef BIOFEM_Y0
+    };
+    const int *pe = m.patch + 16 * (size_t)e;
+    for (int i = 0; i < nen; i++) {
+      double X, Y, Z;
+      load_node(m.pos, __ldg(pe + i), X, Y, Z);
+      const FF d[3] = {ff_split(X - xc[0]), ff_split(Y - xc[1]), ff_split(Z - xc[2])};
 #pragma unroll
-    for (int r = 0; r < 5; r++)
+      for (int r = 0; r < 5; r++) {
+        const FF c = tab[r * 16 + i];
 #pragma unroll
-      for (int d = 0; d < 3; d++) y[3 * r + d] = tsum[r] * c[d];
-  }
-  const int *pe = m.patch + 16 * (size_t)e;
-  for (int i = 0; i < nen; i++) {
-    double X, Y, Z;
-    load_node(m.pos, __ldg(pe + i), X, Y, Z);
-    const FF d[3] = {ff_split(X - xc[0]), ff_split(Y - xc[1]), ff_split(Z - xc[2])};
-#pragma unroll
-    for (int r = 0; r < 5; r++) {
-      const FF c = tab[r * 16 + i];
-#pragma unroll
-      for (int k = 0; k < 3; k++) y[3 * r + k] = y[3 * r + k] + c * d[k];
+        for (int k = 0; k < 3; k++) acc[3 * r + k].add(c, d[k]);
+      }
     }
+#pragma unroll
+    for (int k = 0; k < 15; k++) y[k] = acc[k].get();
   }
   FF f[15];
   int st = 0;
   const EPar<FF> ep = epar<FF>(p);
-  elem_forces<FF, FF>(y, ep, static_cast<const FF *>(m.erefFF) + e, p.ne, f, st);
+  elem_forces<FF>(y, ep, RefCol<FF>{m.erefF + e, (size_t)p.ne, (size_t)p.ne * (kRefPerQp * p.nq + kRefPerElem)}, f, st);
   set_status(m.status, st);
   const size_t ne = p.ne;
   for (int a = 0; a < nen; a++) {
-    FF fx = FF(0.f, 0.f), fy = FF(0.f, 0.f), fz = FF(0.f, 0.f);
+    const FF c0 = tab[a];
+    FFAcc fx(c0, f[0]), fy(c0, f[1]), fz(c0, f[2]);
 #pragma unroll
-    for (int r = 0; r < 5; r++) {
+    for (int r = 1; r < 5; r++) {
       const FF c = tab[r * 16 + a];
-      fx = fx + c * f[3 * r]; fy = fy + c * f[3 * r + 1]; fz = fz + c * f[3 * r + 2];
+      fx.add(c, f[3 * r]); fy.add(c, f[3 * r + 1]); fz.add(c, f[3 * r + 2]);
     }
-    m.fb[(3 * a) * ne + e] = ff_to_double_bits(fx);
-    m.fb[(3 * a + 1) * ne + e] = ff_to_double_bits(fy);
-    m.fb[(3 * a + 2) * ne + e] = ff_to_double_bits(fz);
+    m.fb[(3 * a) * ne + e] = ff_to_double_bits(fx.get());
+    m.fb[(3 * a + 1) * ne + e] = ff_to_double_bits(fy.get());
+    m.fb[(3 * a + 2) * ne + e] = ff_to_double_bits(fz.get());
   }
   if (p.pressure != 0.0) elem_pressure_force(m, p, e);
 }
 
-__global__ void k_to_ff(const double *__restrict__ a, FF *__restrict__ b, long long n)
+/* heads, then tails, of the float-float form of a */
+__global__ void k_to_ff(const double *__restrict__ a, float *__restrict__ b, long long n)
 {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) b[t] = FF(a[t]);
+  if (t >= n) return;
+  const FF f(a[t]);
+  b[t] = f.hi;
+  b[n + t] = f.lo;
 }
 
 /* ---------------- tangent element kernel ---------------- */
-constexpr int kTanElemsPerCta = 8;   /* 16 lanes per element, 128 threads */
+/* Five lanes per element (six elements a warp), lane s forming the 15 x 3
+   block of columns of D along the s-th of a1, a2, Aaa, Abb, Aab from the
+   element's coefficients (tangent_block).  FP64-pipe bound: 245 FP64
+   instructions a lane, 0.27 ms on the 98,304-triangle sheet (with the
+   residual kernel's 0.32 ms of gradients and coefficients: 0.59 ms; the
+   16-lane forward-mode form took 1.99 ms). */
+constexpr int kTanElems = 6;         /* elements per warp */
 
-/* The pressure block vectors of one element (follower-pressure load
-   stiffness): every corner carries P/6 (x2-x1)x(x3-x1), so d/dx1 = [b-a]x,
-   d/dx2 = -[b]x, d/dx3 = [a]x with a = x2-x1, b = x3-x1; stored after D in
-   the element's block for the row assembly. */
-template <class R>
-__device__ __forceinline__ void store_pressure_vectors(const R av[3], const R bv[3], R *dst)
+__global__ void __launch_bounds__(128) k_elem_tangent(DevMesh m, KParams p)
 {
+  const int lane = threadIdx.x & 31;
+  const int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kTanElems + lane / 5;
+  if (lane >= 5 * kTanElems || e >= p.ne) return;
+  const int s = lane % 5;
+  const size_t ne = p.ne;
+  const double *tc = m.tcoef + e;
+  double D[15][3];
+  tangent_block<double>(s, [&](int k) { return __ldg(tc + (size_t)k * ne); }, D);
+  double *De = m.De + (size_t)kDeStride * e + 3 * s;
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    dst[d] = bv[d] - av[d];
-    dst[3 + d] = -bv[d];
-    dst[6 + d] = av[d];
-  }
-}
-
-__global__ void __launch_bounds__(128, 3) k_elem_tangent(DevMesh m, KParams p)
-{
-  __shared__ double tabs[kNumTables * 80];
-  __shared__ double Jsh[kTanElemsPerCta][kMaxQp * 21]; /* constitutive derivatives per thickness point */
-  for (int i = threadIdx.x; i < kNumTables * 80; i += blockDim.x) tabs[i] = m.ntab[i];
-  __syncthreads();
-  const int lane = threadIdx.x & 15;
-  const int slot = threadIdx.x >> 4;
-  const int e = blockIdx.x * kTanElemsPerCta + slot;
-  const bool live = e < p.ne;
-  const int ee = live ? e : p.ne - 1;
-  const int info = m.einfo[ee];
-  const int nen = info & 0xff, tabi = info >> 8;
-  const double *tab = tabs + tabi * 80;
-  double y[15];
-  gather_y_group(m.pos, m.patch, ee, nen, tab, lane, y);
-  double fd[15];
-  const EPar<double> ep = epar<double>(p);
-  /* the thickness-point metrics, the primal geometry and resultants and the
-     primal C33 sub-iteration values come from k_elem_residual, launched
-     before this kernel (which also performs the CC3333 checks) */
-  elem_forces_split_tl<double>(y, ep, m.eref + ee, p.ne, m.gpr + ee, lane, Jsh[slot], fd, m.gmq + ee, m.gtape + ee);
-  if (!live) return;
-  /* column `lane` of D = df/dy, row-major in the element's block */
-  double *De = m.De + (size_t)kDeStride * e;
-  if (lane < 15) {
+  for (int r = 0; r < 15; r++)
 #pragma unroll
-    for (int r = 0; r < 15; r++) De[r * 15 + lane] = fd[r];
-  } else if (p.pressure != 0.0 && !p.pres_dead) {
-    double X[3][3];
-    for (int k = 0; k < 3; k++) load_node(m.pos, m.etri[3 * (size_t)e + k], X[k][0], X[k][1], X[k][2]);
-    const double av[3] = {X[1][0] - X[0][0], X[1][1] - X[0][1], X[1][2] - X[0][2]};
-    const double bv[3] = {X[2][0] - X[0][0], X[2][1] - X[0][1], X[2][2] - X[0][2]};
-    store_pressure_vectors<double>(av, bv, De + kDePres);
-  }
+    for (int j = 0; j < 3; j++) De[15 * r + j] = D[r][j];
 }
 
 /* ---------------- FP32-bulk tangent ---------------- */
-/* Same element math as k_elem_tangent in single precision.  Node positions
-   are shifted to the element's first corner in FP64 (one node per lane, then
-   shared by shuffles) and rounded to FP32, so the FP32 values carry the
+/* The element tangent in single precision, one thread per element: stress
+   gradients, coefficients and all five column blocks in registers, D staged
+   through shared memory (225 floats a lane, an odd stride) so that it leaves
+   in whole cache lines.  Node positions are shifted to the element's first
+   corner in FP64 and rounded to FP32, so the FP32 values carry the
    element-size digits; the shift is put back through (sum_i N_r[i]) * x_c,
    which is not zero for the truncated second-derivative rows (their rows sum
-   to -1e-4 / -1e-4 / +2e-4).  D = df/dy is written in FP32 for the row assembly. */
-__global__ void __launch_bounds__(128, 5) k_elem_tangent_f32(DevMesh m, KParams p)
+   to -1e-4 / -1e-4 / +2e-4). */
+__global__ void __launch_bounds__(32) k_elem_tangent_f32(DevMesh m, KParams p)
 {
-  __shared__ float tabs[kNumTables * 80];
-  __shared__ float tsum[kNumTables * 5];
-  __shared__ float JshF[kTanElemsPerCta][kMaxQp * 21];
-  for (int i = threadIdx.x; i < kNumTables * 85; i += blockDim.x) {
-    if (i < kNumTables * 80) tabs[i] = m.ntabF[i]; else tsum[i - kNumTables * 80] = m.ntabF[i];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 15;
-  const int slot = threadIdx.x >> 4;
-  const int e = blockIdx.x * kTanElemsPerCta + slot;
-  const bool live = e < p.ne;
-  const int ee = live ? e : p.ne - 1;
-  const int info = m.einfo[ee];
+  __shared__ float Dsh[32 * 225];
+  const int lane = threadIdx.x;
+  const int e0 = blockIdx.x * 32;
+  const int e = min(e0 + lane, p.ne - 1);          /* the last block's spare lanes repeat the last element */
+  const int info = m.einfo[e];
   const int nen = info & 0xff, tabi = info >> 8;
-  const float *tab = tabs + tabi * 80;
-  /* shifted coordinates: lane i < nen owns patch node i */
-  const int c0 = m.etri[3 * (size_t)ee];
+  const float *tab = m.ntabF + tabi * 80, *tsum = m.ntabF + kNumTables * 80 + tabi * 5;
+  int corner[3];
+  for (int k = 0; k < 3; k++) corner[k] = m.etri[3 * (size_t)e + k];
   double xc, yc, zc;
-  load_node(m.pos, c0, xc, yc, zc);
-  float dx = 0.f, dy = 0.f, dz = 0.f;
-  if (lane < nen) {
-    const int node = m.patch[16 * (size_t)ee + lane];
-    double X, Y, Z;
-    load_node(m.pos, node, X, Y, Z);
-    dx = (float)(X - xc); dy = (float)(Y - yc); dz = (float)(Z - zc);
-  }
+  load_node(m.pos, corner[0], xc, yc, zc);
   float y[15];
 #pragma unroll
   for (int r = 0; r < 5; r++) {
-    const float sr = tsum[tabi * 5 + r];
+    const float sr = __ldg(tsum + r);
     y[3 * r] = sr * (float)xc; y[3 * r + 1] = sr * (float)yc; y[3 * r + 2] = sr * (float)zc;
   }
-  const unsigned hmask = 0xffffffffu;
-  for (int i = 0; i < 16; i++) {
-    const float ax = __shfl_sync(hmask, dx, i, 16), ay = __shfl_sync(hmask, dy, i, 16), az = __shfl_sync(hmask, dz, i, 16);
-    if (i < nen) {
+  const int *pe = m.patch + 16 * (size_t)e;
+#pragma unroll 4
+  for (int i = 0; i < nen; i++) {
+    double X, Y, Z;
+    load_node(m.pos, __ldg(pe + i), X, Y, Z);
+    const float ax = (float)(X - xc), ay = (float)(Y - yc), az = (float)(Z - zc);
 #pragma unroll
-      for (int r = 0; r < 5; r++) {
-        const float c = tab[r * 16 + i];
-        y[3 * r] = fmaf(c, ax, y[3 * r]); y[3 * r + 1] = fmaf(c, ay, y[3 * r + 1]); y[3 * r + 2] = fmaf(c, az, y[3 * r + 2]);
-      }
+    for (int r = 0; r < 5; r++) {
+      const float c = __ldg(tab + r * 16 + i);
+      y[3 * r] = fmaf(c, ax, y[3 * r]); y[3 * r + 1] = fmaf(c, ay, y[3 * r + 1]); y[3 * r + 2] = fmaf(c, az, y[3 * r + 2]);
     }
   }
-  D1f fd[15];
-  int st = 0;
   const EPar<float> ep = epar<float>(p);
-  elem_forces_split<float>(y, ep, m.erefF + ee, p.ne, lane, JshF[slot], fd, st);
-  if (live) set_status(m.status, st);
-  /* pressure vectors from the shifted corner coordinates */
-  const int cs = m.ecorner[ee];
-  const int cslot[3] = {cs & 31, (cs >> 5) & 31, (cs >> 10) & 31};
-  float xk[3][3];
-  for (int k = 0; k < 3; k++) {
-    xk[k][0] = __shfl_sync(hmask, dx, cslot[k], 16);
-    xk[k][1] = __shfl_sync(hmask, dy, cslot[k], 16);
-    xk[k][2] = __shfl_sync(hmask, dz, cslot[k], 16);
-  }
-  if (!live) return;
-  float *De = m.DeF + (size_t)kDeStride * e;
-  if (lane < 15) {
+  const ElemGeom<float> g = elem_geom<float>(y, ep);
+  float N[3], M[3];
+  int st = 0;
+  TanMoments<float> mo;
+  mo.clear();
+  /* the stress only: the residual kernel of the same call checks the last CC3333 */
+  elem_resultants<float>(g, ep, RefCol<float>{m.erefF + e, (size_t)p.ne}, N, M, st, false, true,
+                         [&](int, float w, float th, float C[3][5]) { mo.add(w, th, C); });
+  if (e0 + lane < p.ne) set_status(m.status, st);
+  float tc[kTanCoefs];
+  tangent_coefs<float>(g, N, M, mo, ep.tnormal, [&](int k, float v) { tc[k] = v; });
+  float *Dl = Dsh + 225 * lane;
 #pragma unroll
-    for (int r = 0; r < 15; r++) De[r * 15 + lane] = fd[r].d;
-  } else if (p.pres6f != 0.f && !p.pres_dead) {
-    const float av[3] = {xk[1][0] - xk[0][0], xk[1][1] - xk[0][1], xk[1][2] - xk[0][2]};
-    const float bv[3] = {xk[2][0] - xk[0][0], xk[2][1] - xk[0][1], xk[2][2] - xk[0][2]};
-    store_pressure_vectors<float>(av, bv, De + kDePres);
+  for (int s = 0; s < 5; s++) {
+    float D[15][3];
+    tangent_block<float>(s, [&](int k) { return tc[k]; }, D);
+#pragma unroll
+    for (int r = 0; r < 15; r++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) Dl[15 * r + 3 * s + j] = D[r][j];
   }
+  if (p.pres6f != 0.f && !p.pres_dead && e0 + lane < p.ne) {
+    double X[3][3];
+    for (int k = 0; k < 3; k++) load_node(m.pos, corner[k], X[k][0], X[k][1], X[k][2]);
+    const float av[3] = {(float)(X[1][0] - xc), (float)(X[1][1] - yc), (float)(X[1][2] - zc)};
+    const float bv[3] = {(float)(X[2][0] - xc), (float)(X[2][1] - yc), (float)(X[2][2] - zc)};
+    store_pressure_vectors<float>(av, bv, m.DeF + (size_t)kDeStride * e + kDePres);
+  }
+  __syncwarp();
+  const int n = min(32, p.ne - e0);
+  float *out = m.DeF + (size_t)kDeStride * e0;
+  for (int t = lane; t < 225 * n; t += 32) out[(size_t)kDeStride * (t / 225) + t % 225] = Dsh[t];
 }
 
 /* ---------------- node gather (residual assembly) ---------------- */
@@ -1109,11 +1126,9 @@ int launch_positions(const DevMesh &m, const KParams &p, const double *x, void *
   return (int)cudaGetLastError();
 }
 
-int launch_elem_residual(const DevMesh &m, const KParams &p, void *stream, bool store_metric)
+int launch_elem_residual(const DevMesh &m, const KParams &p, void *stream, bool tangent)
 {
-  k_elem_residual<<<blocks_for(p.ne, 128), 128, 0, (cudaStream_t)stream>>>(m, p, store_metric ? m.gmq : nullptr,
-                                                                          store_metric ? m.gpr : nullptr,
-                                                                          store_metric ? m.gtape : nullptr);
+  k_elem_residual<<<blocks_for(p.ne, 128), 128, 0, (cudaStream_t)stream>>>(m, p, tangent);
   return (int)cudaGetLastError();
 }
 
@@ -1123,34 +1138,21 @@ int launch_elem_residual_ff(const DevMesh &m, const KParams &p, void *stream)
   return (int)cudaGetLastError();
 }
 
-int launch_to_ff(const double *a, void *b, long long n, void *stream)
+int launch_to_ff(const double *a, float *b, long long n, void *stream)
 {
-  k_to_ff<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(a, static_cast<FF *>(b), n);
+  k_to_ff<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(a, b, n);
   return (int)cudaGetLastError();
 }
 
 int launch_elem_tangent(const DevMesh &m, const KParams &p, void *stream)
 {
-  k_elem_tangent<<<blocks_for(p.ne, kTanElemsPerCta), 128, 0, (cudaStream_t)stream>>>(m, p);
+  k_elem_tangent<<<blocks_for(p.ne, 4 * kTanElems), 128, 0, (cudaStream_t)stream>>>(m, p);
   return (int)cudaGetLastError();
 }
 
 int launch_elem_tangent_f32(const DevMesh &m, const KParams &p, void *stream)
 {
-  k_elem_tangent_f32<<<blocks_for(p.ne, kTanElemsPerCta), 128, 0, (cudaStream_t)stream>>>(m, p);
-  return (int)cudaGetLastError();
-}
-
-
-__global__ void k_to_float(const double *__restrict__ a, float *__restrict__ b, long long n)
-{
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) b[t] = (float)a[t];
-}
-
-int launch_to_float(const double *a, float *b, long long n, void *stream)
-{
-  k_to_float<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(a, b, n);
+  k_elem_tangent_f32<<<blocks_for(p.ne, 32), 32, 0, (cudaStream_t)stream>>>(m, p);
   return (int)cudaGetLastError();
 }
 
@@ -1170,7 +1172,7 @@ __global__ void __launch_bounds__(128) k_elem_thickness(DevMesh m, KParams p, do
   gather_y(m.pos, m.patch, e, nen, tabs + tabi * 80, y);
   int st = 0;
   const EPar<double> ep = epar<double>(p);
-  th[e] = elem_thickness<double>(y, ep, m.eref + e, p.ne, h0, st);
+  th[e] = elem_thickness<double>(y, ep, RefCol<double>{m.eref + e, (size_t)p.ne}, h0, st);
   set_status(m.status, st);
 }
 
