@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/biofem_gpu.h"
+#include "fx.cuh"
 
 namespace biofem {
 
@@ -21,8 +22,8 @@ constexpr int kRefPerElem = 1;    /* pref0 */
 constexpr int kTanCoefs = 116;    /* per-element coefficients of the FP64 tangent (tangent_coefs) */
 constexpr int kCapTable = 11;     /* flat apex-cap triangle: a1 = x2 - x1, a2 = x3 - x1, no curvature */
 constexpr int kNumTables = 12;    /* 0 = regular 12-node patch, v = 3..10 irregular, kCapTable */
-constexpr int kDeStride = 240;    /* per-element tangent block: D = df/dy (15 x 15, row-major), */
-constexpr int kDePres = 225;      /* then the three follower-pressure corner vectors (9) */
+constexpr int kDeStride = 244;    /* per-element tangent block: D = df/dy (25 x 9, with padding), then */
+constexpr int kDePres = 234;      /* the three follower-pressure corner vectors (9); 16-byte aligned */
 constexpr int kMaxRowBlocks = 1023;   /* tangent blocks per row the row assembly handles (10-bit slot targets) */
 constexpr int kRowRec = 20;           /* ints per row-assembly record (80 bytes, 16-byte aligned) */
 constexpr unsigned kRowSlotGhost = 1u << 31;   /* record slot target of a ghost slot: three packed parents */
@@ -74,6 +75,7 @@ struct DevMesh {
   const double *eref;        /* (kRefPerQp*nq + kRefPerElem) * ne, SoA */
   const float *erefF;        /* FP32-bulk handles: the same as float-float, the plane of heads then the plane of tails */
   const void *ntabFF;        /* basis tables and their row sums as float-float pairs (FP32-bulk handles) */
+  const int *ntabFx;         /* the basis tables in fixed point (fx.cuh): kNumTables x 16 columns x 6 pairs */
   const double *ntab;        /* kNumTables * 5 * 16 basis-derivative tables */
   const float *ntabF;        /* the same in FP32, followed by the kNumTables*5 row sums */
   const int *etri;           /* 3*ne triangle corners (pressure) */
@@ -82,25 +84,27 @@ struct DevMesh {
   const unsigned char *rowkind; /* nt: 0 free real row, 1 clamped row, 2 ghost row */
   /* residual gather lists */
   const int *rptr, *ridx;    /* nt+1, into fb scratch (slot*3*ne + e) */
-  const int *rrec;           /* kRowRec ints per contribution (same order): e | slot << 27, einfo, ecorner, 0,
+  const int *rrec;           /* kRowRec ints per contribution (same order): e | slot << 27, einfo, ecorner, 0 for a
+                                regular patch of real, distinct nodes,
                                 the slot targets in the row (row assembly of the tangent) */
+  const unsigned char *rgrow; /* FP64 handles: nt, growth bits of the fixed-point row assembly (fx.cuh) */
   const int *pptr, *pidx;    /* nt+1, elements whose corner is the node */
   /* tangent pattern */
   const int *rowptr, *colind;   /* BSR pattern, columns sorted per row */
   long long nnzb;
   int maxblk;                /* most blocks in one row */
-  int ntabs;                 /* basis tables the row assembly stages: kCapTable, or kNumTables with cap elements */
   /* work arrays */
   double *pos;               /* 4*nt padded positions */
   double *fb;                /* 48*ne element forces */
   double *fp;                /* 3*ne element pressure forces */
-  double *De;                /* kDeStride*ne element tangent blocks df/dy (FP64 handles) */
+  double *De;                /* kDeStride*ne element tangent blocks df/dy in fixed point (FP64 handles) */
   float *DeF;                /* the same in FP32 (FP32-bulk handles) */
   int *status;               /* device error flag */
   double *dA0;               /* n_elmt flat reference areas of the real triangles (AreaNormal at Init) */
   int *dptr, *didx;          /* per node, the real triangles with that corner, in triangle order */
   double *xn, *xnm1, *xd, *xdd;   /* 3*nt dynamic state (previous positions, velocity, acceleration) */
   double *dyn_diag;          /* nt: d Fdyn / d x on the diagonal of each free row */
+  unsigned short *dexp;      /* FP64 handles: 16*ne exponent fields of D, one per Cartesian pair (fx.cuh) */
   double *cq;                /* FP64 handles: 15 nq x ne stress gradients d S / d metric (k_elem_residual's own scratch) */
   double *tcoef;             /* FP64 handles: kTanCoefs x ne tangent coefficients, k_elem_residual -> k_elem_tangent */
   unsigned long long *fmax;  /* max |Fext| as ordered bits */
@@ -114,11 +118,16 @@ int launch_elem_tangent(const DevMesh &m, const KParams &p, void *stream);
 int launch_node_gather(const DevMesh &m, const KParams &p, const double *x, double *R, void *stream,
                        double *parts = nullptr);
 int launch_elem_thickness(const DevMesh &m, const KParams &p, double h0, double *th, void *stream);
-int launch_row_assemble(const DevMesh &m, const KParams &p, void *K, bool f32, bool colmajor, void *stream);
+/* the regular table as the row assembly's kernel parameter (constant-bank operands), of either precision */
+struct RowTableF { float n[12][5]; };
+struct RowTables { FxRegular x; RowTableF f; };
+bool regular_tables(const double *tab0, int den, RowTables &t);
+int launch_row_assemble(const DevMesh &m, const KParams &p, const RowTables &t, void *K, bool f32, bool colmajor, void *stream);
 int launch_row_records(const DevMesh &m, const KParams &p, int *rrec, void *stream);   /* once per mesh */
+int launch_row_growth(const DevMesh &m, const KParams &p, unsigned char *rgrow, void *stream);   /* once per mesh, after the records */
 extern thread_local bool t_blocking_waits;   /* solver host waits sleep instead of spinning (serving workers) */
-int row_assemble_configure(int maxblk, bool f32, int ntabs);   /* dynamic shared memory of the row assembly */
-size_t row_assemble_smem(int maxblk, bool f32, int ntabs);
+int row_assemble_configure(int maxblk, bool f32);   /* dynamic shared memory of the row assembly */
+size_t row_assemble_smem(int maxblk, bool f32);
 int row_assemble_max_blocks(bool f32);             /* blocks per row each row assembly handles */
 int launch_scale(const DevMesh &m, const KParams &p, double *R, void *stream);
 int launch_elem_tangent_f32(const DevMesh &m, const KParams &p, void *stream);

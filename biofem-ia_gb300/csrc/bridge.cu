@@ -153,6 +153,7 @@ struct BiofemGpuMesh_ {
   HostTopo topo;
   BiofemParams prm{};
   KParams kp{};
+  RowTables rtab{};
   std::vector<double> dA0;
   std::vector<int> rowptr, colind;
   long long nnzb = 0, ncontrib = 0;
@@ -538,6 +539,8 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
     tabsF[kNumTables * 80 + i] = (float)acc;
     tabsFF[kNumTables * 80 + i] = FF(acc);
   }
+  const int den = params->basis == BIOFEM_BASIS_EXACT ? 31 * 324 : 10000;   /* the regular table's common denominator (fx.cuh) */
+  if (!regular_tables(tabs.data(), den, m->rtab)) { free_mesh(m); return fail(77, "the regular basis table is not what the row assembly expects"); }
   std::vector<double> fib(mesh->n_fib, mesh->n_fib + 3 * (size_t)ne), gsc(mesh->gamma_scale, mesh->gamma_scale + ne);
 
 #define UP(field, vec) do { rc = dupload(m, const_cast<std::remove_const<std::remove_pointer<decltype(dm.field)>::type>::type **>(&dm.field), vec); if (rc) { free_mesh(m); return rc; } } while (0)
@@ -552,13 +555,12 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
   }
   dm.nnzb = m->nnzb;
   dm.maxblk = m->maxblk;
-  dm.ntabs = (T.n_elmt_base > 0 && T.n_elmt_base < ne) ? kNumTables : kCapTable;
   if (m->maxblk > row_assemble_max_blocks(params->precision != BIOFEM_FP64)) {
     free_mesh(m);
     return fail(63, "a tangent row has more blocks than the FP32 row assembly holds in registers");
   }
   {
-    cudaError_t ce = (cudaError_t)row_assemble_configure(m->maxblk, params->precision != BIOFEM_FP64, dm.ntabs);
+    cudaError_t ce = (cudaError_t)row_assemble_configure(m->maxblk, params->precision != BIOFEM_FP64);
     if (ce != cudaSuccess) { free_mesh(m); return fail(76, std::string("row assembly configuration: ") + cudaGetErrorString(ce)); }
   }
   double *d_fib = nullptr, *d_gsc = nullptr, *d_eref = nullptr;
@@ -574,11 +576,28 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
   float *d_erefF = nullptr;
   if (params->precision == BIOFEM_FP64) {
     double *dK = nullptr;
-    if ((rc = dalloc(m, &dm.De, (size_t)kDeStride * ne)) || (rc = dalloc(m, &dK, 9 * (size_t)m->nnzb)) ||
+    std::vector<int> tabsFx(kNumTables * 16 * 12, 0);   /* per table column five (lo, hi) pairs and the column sum */
+    for (int tb = 0; tb < kNumTables; tb++)
+      for (int b = 0; b < 16; b++) {
+        double col[5];
+        for (int r = 0; r < 5; r++) {
+          col[r] = tabs[tb * 80 + r * 16 + b];
+          const Fx f = fx_table(col[r], den);
+          tabsFx[(tb * 16 + b) * 12 + 2 * r] = f.lo;
+          tabsFx[(tb * 16 + b) * 12 + 2 * r + 1] = f.hi;
+        }
+        tabsFx[(tb * 16 + b) * 12 + 10] = fx_column_sum(col);
+      }
+    int *d_ntabFx = nullptr;
+    unsigned char *d_rgrow = nullptr;
+    if ((rc = dupload(m, &d_ntabFx, tabsFx)) || (rc = dalloc(m, &d_rgrow, (size_t)nt)) || (rc = dalloc(m, &dm.dexp, 16 * (size_t)ne)) ||
+        (rc = dalloc(m, &dm.De, (size_t)kDeStride * ne)) || (rc = dalloc(m, &dK, 9 * (size_t)m->nnzb)) ||
         (rc = dalloc(m, &dm.cq, 15 * (size_t)kp.nq * ne)) || (rc = dalloc(m, &dm.tcoef, (size_t)kTanCoefs * ne))) {
       free_mesh(m);
       return rc;
     }
+    dm.ntabFx = d_ntabFx;
+    dm.rgrow = d_rgrow;
     m->d_K = dK;
   } else {
     float *dK = nullptr;
@@ -598,7 +617,8 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
   CUDA_TRY(cudaMemsetAsync(dm.fp, 0, 3 * sizeof(double) * (size_t)ne, m->st));
   /* reference positions (ghosts included) -> one-time reference geometry */
   if ((rc = launch_positions(dm, kp, dm.X, m->st)) || (rc = launch_ref_prep(dm, kp, d_fib, d_gsc, d_eref, m->st)) ||
-      (rc = launch_row_records(dm, kp, const_cast<int *>(dm.rrec), m->st))) {
+      (rc = launch_row_records(dm, kp, const_cast<int *>(dm.rrec), m->st)) ||
+      (dm.rgrow && (rc = launch_row_growth(dm, kp, const_cast<unsigned char *>(dm.rgrow), m->st)))) {
     free_mesh(m);
     return fail(76, std::string("reference preparation launch: ") + cudaGetErrorString((cudaError_t)rc));
   }
@@ -772,7 +792,7 @@ static int residual_jacobian(BiofemGpuMesh *m, const double *d_x, double *d_R, v
       if (!rc) { rc = launch_elem_tangent(m->dm, m->kp, st); tmark(m, st, 3); }
       if (!rc) { rc = launch_node_gather(m->dm, m->kp, d_x, d_R, st); tmark(m, st, 4); }
     }
-    if (!rc) { rc = launch_row_assemble(m->dm, m->kp, K, false, colmajor, st); tmark(m, st, 5); }
+    if (!rc) { rc = launch_row_assemble(m->dm, m->kp, m->rtab, K, false, colmajor, st); tmark(m, st, 5); }
     if (!rc) { rc = launch_scale(m->dm, m->kp, d_R, st); tmark(m, st, 6); }
   } else {
     /* FP32-bulk: residual in float-float, tangent (D, K) in FP32 */
@@ -789,7 +809,7 @@ static int residual_jacobian(BiofemGpuMesh *m, const double *d_x, double *d_R, v
       if (!rc) { rc = launch_elem_tangent_f32(m->dm, m->kp, st); tmark(m, st, 3); }
       if (!rc) { rc = launch_node_gather(m->dm, m->kp, d_x, d_R, st); tmark(m, st, 4); }
     }
-    if (!rc) { rc = launch_row_assemble(m->dm, m->kp, K, true, colmajor, st); tmark(m, st, 5); }
+    if (!rc) { rc = launch_row_assemble(m->dm, m->kp, m->rtab, K, true, colmajor, st); tmark(m, st, 5); }
     if (!rc) { rc = launch_scale(m->dm, m->kp, d_R, st); tmark(m, st, 6); }
   }
   if (rc) return fail(76, std::string("jacobian launch: ") + cudaGetErrorString((cudaError_t)rc));

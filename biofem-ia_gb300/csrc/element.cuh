@@ -139,6 +139,18 @@ template <> struct RefCol<FF> {
   __host__ __device__ __forceinline__ RefCol at(int k) const { return {p + (size_t)k * stride, stride, tail}; }
 };
 
+/* One thickness point's constants in registers, loaded together (the FP32
+   tangent waits for memory, not for arithmetic). */
+template <class R> struct RefRegs {
+  R v[kRefPerQp];
+  __host__ __device__ __forceinline__ explicit RefRegs(const RefCol<R> &r)
+  {
+#pragma unroll
+    for (int k = 0; k < kRefPerQp; k++) v[k] = r(k);
+  }
+  __host__ __device__ __forceinline__ R operator()(int k) const { return v[k]; }
+};
+
 /* Material / quadrature constants in the working precision R. */
 template <class R> struct EPar {
   R mu, K, hhalf;
@@ -212,8 +224,8 @@ __host__ __device__ __forceinline__ void inverse_rows(R c00, R c11, R c01, R c02
    dc = -c dg c and d ln det = c:dg.  The damping factor of a bisected update
    is constant, as in the update itself.  About 0.3 of the arithmetic of five
    forward directions. */
-template <class R>
-__host__ __device__ __forceinline__ void qp_stress(const R gm[5] /* 00 11 01 02 12 */, const RefCol<R> &r, R mu, R K,
+template <class R, class Ref>
+__host__ __device__ __forceinline__ void qp_stress(const R gm[5] /* 00 11 01 02 12 */, const Ref &r, R mu, R K,
                                                    int iters, R sv[3], int &status, R *c33_out = nullptr,
                                                    bool final_update = true, bool grad = false, R C[3][5] = nullptr)
 {
@@ -449,7 +461,10 @@ __host__ __device__ __forceinline__ void elem_resultants(const ElemGeom<R> &g, c
     R gm[5], sv[3] = {R(0), R(0), R(0)};
     qp_metric(g, th3, gm);
     R C[3][5] = {};
-    qp_stress<R>(gm, ref.at(kRefPerQp * q), p.mu, p.K, p.iters, sv, status, nullptr, final_update, grad, C);
+    if constexpr (sizeof(R) == 4)
+      qp_stress<R>(gm, RefRegs<R>(ref.at(kRefPerQp * q)), p.mu, p.K, p.iters, sv, status, nullptr, final_update, grad, C);
+    else
+      qp_stress<R>(gm, ref.at(kRefPerQp * q), p.mu, p.K, p.iters, sv, status, nullptr, final_update, grad, C);
     if (grad) out(q, pref0 * p.w[q], th3, C);
     const R wq = p.w[q], wt = p.w[q] * th3;
     for (int i = 0; i < 3; i++) { N[i] = mad(wq, sv[i], N[i]); M[i] = mad(wt, sv[i], M[i]); }

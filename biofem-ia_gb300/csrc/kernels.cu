@@ -22,10 +22,11 @@
  *                    order (the order FInternalAct's VecSetValues loop adds
  *                    them), R = Fint - Fext + Fdyn, clamp rows R = x - X,
  *                    ghost rows 0 (main.c:844-1016)
- *   k_row_assemble   one warp per row node: for every element holding the
+ *   k_row_assemble_* one warp per row node: for every element holding the
  *                    node, K_e's block row N_a^T D N (and the pressure blocks)
  *                    added into the row's blocks in shared memory in a fixed
- *                    order, then the row written once
+ *                    order, then the row written once; FP64 K in fixed point
+ *                    on the integer pipe (fx.cuh)
  *   k_scale          R *= 1 / max(|Fext|_inf, 1) (main.c:1020-1026); the row
  *                    assembly applies the same factor to K as it writes it
  *   k_elem_thickness UpdateElementThickness (output); k_dyn_diag / k_dyn_update
@@ -37,7 +38,10 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "element.cuh"
+#include "fx.cuh"
 
 namespace biofem {
 
@@ -255,16 +259,17 @@ __device__ __forceinline__ void elem_pressure_force(const DevMesh &m, const KPar
 
 /* The pressure block vectors of one element (follower-pressure load
    stiffness): every corner carries P/6 (x2-x1)x(x3-x1), so d/dx1 = [b-a]x,
-   d/dx2 = -[b]x, d/dx3 = [a]x with a = x2-x1, b = x3-x1; stored after D in
-   the element's block for the row assembly. */
+   d/dx2 = -[b]x, d/dx3 = [a]x with a = x2-x1, b = x3-x1, times psc = -P/6 (R
+   subtracts the load); stored after D in the element's block for the row
+   assembly. */
 template <class R>
-__device__ __forceinline__ void store_pressure_vectors(const R av[3], const R bv[3], R *dst)
+__device__ __forceinline__ void store_pressure_vectors(const R av[3], const R bv[3], R psc, R *dst)
 {
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    dst[d] = bv[d] - av[d];
-    dst[3 + d] = -bv[d];
-    dst[6 + d] = av[d];
+    dst[d] = psc * (bv[d] - av[d]);
+    dst[3 + d] = -(psc * bv[d]);
+    dst[6 + d] = psc * av[d];
   }
 }
 
@@ -329,7 +334,7 @@ __global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, boo
       for (int k = 0; k < 3; k++) load_node(m.pos, m.etri[3 * (size_t)e + k], X[k][0], X[k][1], X[k][2]);
       const double av[3] = {X[1][0] - X[0][0], X[1][1] - X[0][1], X[1][2] - X[0][2]};
       const double bv[3] = {X[2][0] - X[0][0], X[2][1] - X[0][1], X[2][2] - X[0][2]};
-      store_pressure_vectors<double>(av, bv, m.De + (size_t)kDeStride * e + kDePres);
+      store_pressure_vectors<double>(av, bv, -p.pressure / 6.0, m.De + (size_t)kDeStride * e + kDePres);
     }
   }
 }
@@ -416,41 +421,94 @@ __global__ void k_to_ff(const double *__restrict__ a, float *__restrict__ b, lon
    element's coefficients (tangent_block).  FP64-pipe bound: 245 FP64
    instructions a lane, 0.27 ms on the 98,304-triangle sheet (with the
    residual kernel's 0.32 ms of gradients and coefficients: 0.59 ms; the
-   16-lane forward-mode form took 1.99 ms). */
+   16-lane forward-mode form took 1.99 ms).  D leaves in the row assembly's fixed-point form
+   (fx.cuh): per Cartesian pair (i, j) the largest exponent over the element's
+   25 entries, then every entry as two 32-bit words; an element with an
+   infinity or NaN keeps its doubles and is marked kFxRaw. */
 constexpr int kTanElems = 6;         /* elements per warp */
+
+/* place of entry (k = 5 r + s, q = 3 i + j) of D in an FP64 element block, see the
+   row assembly.  FP32 blocks hold float4s of rows r = 0..3: (s, q) at 9 s + q;
+   then, row 4, a float4 of s = 0..3 for each q (45 + q) and s = 4 (float 216 + q). */
+__host__ __device__ __forceinline__ int fx_place(int k, int q) { return (k / 2) * 18 + 2 * q + k % 2; }
 
 __global__ void __launch_bounds__(128) k_elem_tangent(DevMesh m, KParams p)
 {
   const int lane = threadIdx.x & 31;
-  const int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kTanElems + lane / 5;
-  if (lane >= 5 * kTanElems || e >= p.ne) return;
-  const int s = lane % 5;
+  const int g = lane < 5 * kTanElems ? lane / 5 : kTanElems - 1, s = lane % 5;
+  const int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kTanElems + g;
+  const bool live = lane < 5 * kTanElems && e < p.ne;
+  const int ee = min(e, p.ne - 1);
   const size_t ne = p.ne;
-  const double *tc = m.tcoef + e;
+  const double *tc = m.tcoef + ee;
   double D[15][3];
   tangent_block<double>(s, [&](int k) { return __ldg(tc + (size_t)k * ne); }, D);
-  double *De = m.De + (size_t)kDeStride * e + 3 * s;
+  const bool pres_live = p.pressure != 0.0 && !p.pres_dead;
+  const double *pv = m.De + (size_t)kDeStride * ee + kDePres + 3 * min(s, 2);
+  /* exponent of each (i, j) over this lane's five rows, two to a register, then over the element's five lanes */
+  unsigned eb[5];
 #pragma unroll
-  for (int r = 0; r < 15; r++)
+  for (int q = 0; q < 9; q++) {
+    int h = 0;
 #pragma unroll
-    for (int j = 0; j < 3; j++) De[15 * r + j] = D[r][j];
+    for (int r = 0; r < 5; r++) h = max(h, __double2hiint(D[3 * r + q / 3][q % 3]) & 0x7fffffff);
+    /* the pressure block's entry (i, j) is component 3 - i - j of the three corner vectors, one of them read here */
+    const int i = q / 3, j = q % 3;
+    if (i != j && pres_live && s < 3) h = max(h, __double2hiint(pv[3 - i - j]) & 0x7fffffff);
+    h >>= 20;
+    eb[q / 2] = q % 2 ? eb[q / 2] | ((unsigned)h << 16) : (unsigned)h;
+  }
+#pragma unroll
+  for (int k = 1; k < 5; k++) {
+    const int src = lane < 5 * kTanElems ? 5 * g + (s + k) % 5 : lane;
+#pragma unroll
+    for (int q = 0; q < 5; q++) eb[q] = __vmaxu2(eb[q], __shfl_sync(0xffffffffu, eb[q], src));
+  }
+  bool raw = false;
+#pragma unroll
+  for (int q = 0; q < 5; q++) raw |= (eb[q] & 0xffffu) == (unsigned)kFxRaw || (eb[q] >> 16) == (unsigned)kFxRaw;
+  if (!live) return;
+  if (s == 0) {
+    const unsigned bad = kFxRaw | (kFxRaw << 16);
+    uint4 *dst = reinterpret_cast<uint4 *>(m.dexp + 16 * (size_t)e);
+    dst[0] = raw ? make_uint4(bad, bad, bad, bad) : make_uint4(eb[0], eb[1], eb[2], eb[3]);
+    dst[1] = make_uint4(raw ? bad : eb[4], 0u, 0u, 0u);
+  }
+  double *De = m.De + (size_t)kDeStride * e;
+#pragma unroll
+  for (int r = 0; r < 5; r++)
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+      const double d = D[3 * r + q / 3][q % 3];
+      const Fx v = fx_split(fx_from_double(d, (int)(q % 2 ? eb[q / 2] >> 16 : eb[q / 2] & 0xffffu)));
+      const int2 w = raw ? make_int2(__double2loint(d), __double2hiint(d)) : make_int2(v.lo, v.hi);
+      *reinterpret_cast<int2 *>(De + fx_place(5 * r + s, q)) = w;
+    }
 }
 
 /* ---------------- FP32-bulk tangent ---------------- */
 /* The element tangent in single precision, one thread per element: stress
-   gradients, coefficients and all five column blocks in registers, D staged
-   through shared memory (225 floats a lane, an odd stride) so that it leaves
-   in whole cache lines.  Node positions are shifted to the element's first
-   corner in FP64 and rounded to FP32, so the FP32 values carry the
-   element-size digits; the shift is put back through (sum_i N_r[i]) * x_c,
-   which is not zero for the truncated second-derivative rows (their rows sum
-   to -1e-4 / -1e-4 / +2e-4). */
-__global__ void __launch_bounds__(32) k_elem_tangent_f32(DevMesh m, KParams p)
+   gradients, coefficients and the five column blocks in registers, each block
+   leaving through shared memory as the row assembly's 16-byte pieces, nine
+   neighbouring lanes an element.  Node positions
+   are shifted to the element's first corner in FP64 and rounded to FP32, so
+   the FP32 values carry the element-size digits; the shift is put back through
+   (sum_i N_r[i]) * x_c, which is not zero for the truncated second-derivative
+   rows (their rows sum to -1e-4 / -1e-4 / +2e-4).
+   Bound by the loads of the constants and the stores of D (1.1 KB an element):
+   0.18 -> 0.08 ms on the 98,304-triangle sheet; staging all of D in one go
+   took 0.09, a thread storing its own 0.10. */
+constexpr int kTanF32Block = 64;
+
+__global__ void __launch_bounds__(kTanF32Block, 6) k_elem_tangent_f32(DevMesh m, KParams p)
 {
-  __shared__ float Dsh[32 * 225];
-  const int lane = threadIdx.x;
-  const int e0 = blockIdx.x * 32;
-  const int e = min(e0 + lane, p.ne - 1);          /* the last block's spare lanes repeat the last element */
+  __shared__ float stage[kTanF32Block * 37];       /* rows r = 0..3 of one column block, [q][r], an odd stride */
+  __shared__ float row4[kTanF32Block * 45];        /* row r = 4 of the blocks, [q][s], until all five are known */
+  const int lane = threadIdx.x & 31, w0 = threadIdx.x & ~31;
+  const int e0 = blockIdx.x * kTanF32Block + w0;   /* the warp's elements e0 .. e0 + 31 */
+  if (e0 >= p.ne) return;
+  const int nw = min(32, p.ne - e0);
+  const int e = e0 + min(lane, nw - 1);            /* the last warp's spare lanes repeat its last element */
   const int info = m.einfo[e];
   const int nen = info & 0xff, tabi = info >> 8;
   const float *tab = m.ntabF + tabi * 80, *tsum = m.ntabF + kNumTables * 80 + tabi * 5;
@@ -485,30 +543,42 @@ __global__ void __launch_bounds__(32) k_elem_tangent_f32(DevMesh m, KParams p)
   /* the stress only: the residual kernel of the same call checks the last CC3333 */
   elem_resultants<float>(g, ep, RefCol<float>{m.erefF + e, (size_t)p.ne}, N, M, st, false, true,
                          [&](int, float w, float th, float C[3][5]) { mo.add(w, th, C); });
-  if (e0 + lane < p.ne) set_status(m.status, st);
+  if (lane < nw) set_status(m.status, st);
   float tc[kTanCoefs];
   tangent_coefs<float>(g, N, M, mo, ep.tnormal, [&](int k, float v) { tc[k] = v; });
-  float *Dl = Dsh + 225 * lane;
+  float4 *out = reinterpret_cast<float4 *>(m.DeF + (size_t)kDeStride * e0);
+  float *sd = stage + 37 * threadIdx.x, *r4 = row4 + 45 * threadIdx.x;
 #pragma unroll
   for (int s = 0; s < 5; s++) {
     float D[15][3];
     tangent_block<float>(s, [&](int k) { return tc[k]; }, D);
 #pragma unroll
-    for (int r = 0; r < 15; r++)
+    for (int q = 0; q < 9; q++) {
 #pragma unroll
-      for (int j = 0; j < 3; j++) Dl[15 * r + 3 * s + j] = D[r][j];
+      for (int r = 0; r < 4; r++) sd[4 * q + r] = D[3 * r + q / 3][q % 3];
+      r4[5 * q + s] = D[12 + q / 3][q % 3];
+    }
+    __syncwarp();
+    for (int t = lane; t < 9 * nw; t += 32) {
+      const int g = t / 9, q = t - 9 * g;
+      const float *v = stage + 37 * (w0 + g) + 4 * q;
+      out[(kDeStride / 4) * g + 9 * s + q] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    __syncwarp();
   }
-  if (p.pres6f != 0.f && !p.pres_dead && e0 + lane < p.ne) {
+  for (int t = lane; t < 9 * nw; t += 32) {
+    const int g = t / 9, q = t - 9 * g;
+    const float *v = row4 + 45 * (w0 + g) + 5 * q;
+    out[(kDeStride / 4) * g + 45 + q] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float *>(out + (kDeStride / 4) * g)[216 + q] = v[4];
+  }
+  if (p.pres6f != 0.f && !p.pres_dead && lane < nw) {
     double X[3][3];
     for (int k = 0; k < 3; k++) load_node(m.pos, corner[k], X[k][0], X[k][1], X[k][2]);
     const float av[3] = {(float)(X[1][0] - xc), (float)(X[1][1] - yc), (float)(X[1][2] - zc)};
     const float bv[3] = {(float)(X[2][0] - xc), (float)(X[2][1] - yc), (float)(X[2][2] - zc)};
-    store_pressure_vectors<float>(av, bv, m.DeF + (size_t)kDeStride * e + kDePres);
+    store_pressure_vectors<float>(av, bv, -p.pres6f, m.DeF + (size_t)kDeStride * e + kDePres);
   }
-  __syncwarp();
-  const int n = min(32, p.ne - e0);
-  float *out = m.DeF + (size_t)kDeStride * e0;
-  for (int t = lane; t < 225 * n; t += 32) out[(size_t)kDeStride * (t / 225) + t % 225] = Dsh[t];
 }
 
 /* ---------------- node gather (residual assembly) ---------------- */
@@ -589,15 +659,35 @@ __global__ void k_node_gather(DevMesh m, KParams p, const double *__restrict__ x
    patch, K_ib += (N[:,a] (x) I3)^T D_e (N[:,b] (x) I3), with D_e = df/dy the
    element kernel stored, plus the follower-pressure block when a and b are
    corner slots; a ghost slot b adds to the blocks of its parents with signs
-   +, +, - (x_g = x_nv2 + x_nv1 - x_nv3).  The row's blocks accumulate in
-   shared memory in a fixed order (contributions in element order; within an
-   element the real slots, then the ghost slots in slot order), so K is
-   deterministic; FP32 sums are compensated (Kahan).  Clamped and ghost rows
-   are identity rows.  K is scaled by 1/max(|Fext|_inf, 1) as it is written
+   +, +, - (x_g = x_nv2 + x_nv1 - x_nv3).  Clamped and ghost rows are identity
+   rows.  K is scaled by 1/max(|Fext|_inf, 1) as it is written
    (main.c:1020-1026; k_node_gather, launched before, found the max); with
-   colmajor each 3x3 block is stored column by column. */
-constexpr int kRowWarps = 4;
-constexpr int kRowChunk = 4;          /* contributions whose slots and w are formed together */
+   colmajor each 3x3 block is stored column by column.
+
+   Three contributions at a time, lane (c, q) = (contribution, entry q = 3 i + j
+   of the 3x3 blocks), 27 lanes: the lane forms its five values
+   w_s = sum_r N[r][a] D_rs[q] (D is stored so that the nine lanes of a
+   contribution read neighbouring 16-byte pieces: two values (5 r + s, 5 r + s
+   + 1) of an entry in FP64, four in FP32), then for every slot b its
+   entry sum_s N[s][b] w_s, and adds it to block target(b) of the
+   contribution's own copy of the row in shared memory (three copies: two
+   contributions may share a block; their sum is taken at the write-out).  Block
+   t's three copies lie in 32 consecutive words, entry (c, q) at 32 t + lane, so
+   every access is free of bank conflicts whatever the targets.
+   Nothing is exchanged between lanes, and on a regular patch N[s][b] is a
+   constant-bank operand of the multiply (the kernel parameter `reg`), its
+   eight zeros left out: shared memory sees one read and one write an entry.  Forms that shared w through
+   shared memory were bound by it (FP64: 0.75 ms, FP32: 0.34 ms on the
+   98,304-triangle sheet).  The order of every sum is fixed, so K is
+   deterministic. */
+constexpr int kRowCopies = 3;
+constexpr int kRowWords = 32;        /* words of one block: 3 x 9 entries and padding */
+/* N[s][b] = 0 on the regular patch (both kinds of tables; regular_tables checks it) */
+__host__ __device__ constexpr bool row_reg_zero(int s, int b)
+{
+  return (s == 0 && (b == 2 || b == 7)) || (s == 1 && (b == 4 || b == 6)) || (s == 2 && (b == 8 || b == 11)) ||
+         (s == 3 && (b == 5 || b == 9));
+}
 
 __device__ __forceinline__ int row_find(const int *cols, int nb, int node)
 {
@@ -611,306 +701,300 @@ __device__ __forceinline__ int row_find(const int *cols, int nb, int node)
 
 __host__ __device__ __forceinline__ size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
 
-/* one warp's shared buffers; every part starts on 16 bytes */
-template <class R> struct RowAsmBuf {
-  R *acc, *comp;      /* the row's 9 nb block values (and their compensations, FP32) */
-  R *wT;              /* kRowChunk x 9 x 8: w of each contribution of the chunk */
-  R *gv;              /* 9 x 16 values of the ghost slots of one contribution */
-  int *cols;          /* the row's block columns */
-  int *rec;           /* kRowChunk row-assembly records (kRowRec ints each) */
-};
+/* FP64 row assembly in fixed point (fx.cuh); the follower-pressure vectors
+   are converted to the row's units and added with it.  A row with an element
+   whose D is not finite takes row_assemble_raw, plain FP64.
 
-__host__ __device__ __forceinline__ size_t row_buf_bytes(int maxblk, size_t rsize)
+   Why integers: the FP64 form of this sum ran at 93 % of the FP64 pipe
+   (1.94 ms on the 98,304-triangle sheet, q = 3); K's error against a 64-bit
+   reference is measured no larger (see fx.cuh for the bound).  Now 0.49 ms,
+   bound by the integer multiplies (IMAD.WIDE, four cycles a warp).  Fetching
+   the next contributions' D early, as the FP32 form does, needs 126 registers
+   and halves the warps: 0.58 ms. */
+struct FxRowBuf {
+  long long *acc;     /* kRowWords maxblk */
+  int *rec;           /* kRowCopies records */
+  double *sc;         /* 9 units of K */
+  int *eb;            /* 9 exponents */
+};
+constexpr int kFxTab = 6;            /* table column: 5 values and fx_column_sum, 48 bytes */
+
+__host__ __device__ __forceinline__ size_t fx_row_bytes(int maxblk)
 {
-  const size_t nacc = 9 * (size_t)maxblk * (rsize == 4 ? 2 : 1);
-  return align16(nacc * rsize) + kRowChunk * 9 * kRowPad * rsize + 144 * rsize + align16(4 * (size_t)maxblk) +
-         kRowChunk * kRowRec * 4;
+  return (size_t)kRowWords * maxblk * 8 + kRowCopies * kRowRec * 4 + 80 + 48;
 }
 
-template <class R>
-__device__ __forceinline__ RowAsmBuf<R> row_buf(unsigned char *base, int maxblk)
+__device__ __forceinline__ FxRowBuf fx_row_buf(unsigned char *q, int maxblk)
 {
-  RowAsmBuf<R> b;
-  const size_t nacc = 9 * (size_t)maxblk;
-  b.acc = reinterpret_cast<R *>(base);
-  b.comp = b.acc + nacc;
-  unsigned char *q = base + align16(nacc * (sizeof(R) == 4 ? 2 : 1) * sizeof(R));
-  b.wT = reinterpret_cast<R *>(q);
-  q += kRowChunk * 9 * kRowPad * sizeof(R);
-  b.gv = reinterpret_cast<R *>(q);
-  q += 144 * sizeof(R);
-  b.cols = reinterpret_cast<int *>(q);
-  q += align16(4 * (size_t)maxblk);
+  FxRowBuf b;
+  b.acc = reinterpret_cast<long long *>(q);
+  q += (size_t)kRowWords * maxblk * 8;
   b.rec = reinterpret_cast<int *>(q);
+  q += kRowCopies * kRowRec * 4;
+  b.sc = reinterpret_cast<double *>(q);
+  q += 80;
+  b.eb = reinterpret_cast<int *>(q);
   return b;
 }
 
-/* The records of the contributions [cb, cb + CH) of a row ending at c1, one
-   16-byte piece per lane (lanes < 5 np); zero past the row. */
-template <int CH>
-__device__ __forceinline__ int4 row_rec_load(const int *rrec, int cb, int c1, int lane)
+/* one entry of the block of column n */
+__device__ __forceinline__ long long fx_entry(const Fx n[5], const Fx w[5])
 {
-  static_assert(kRowRec % 4 == 0 && (kRowRec / 4) * CH <= 32, "a chunk's records must fit one piece per lane");
-  const int np = min(CH, c1 - cb);
-  if (np <= 0 || lane >= (kRowRec / 4) * np) return make_int4(0, 0, 0, 0);
-  return __ldg(reinterpret_cast<const int4 *>(rrec) + (size_t)(kRowRec / 4) * cb + lane);
+  FxSum<63> sum;
+#pragma unroll
+  for (int s = 0; s < 5; s++) sum.add(n[s], w[s]);
+  return sum.value();
 }
 
-template <class R>
-__device__ __forceinline__ void row_add(R *acc, R *comp, int idx, R v)
+/* the same of the regular table's column B, whose values are small integers over a common denominator */
+template <int B>
+__device__ __forceinline__ long long fx_entry_reg(const FxRegular &reg, const Fx w[5])
 {
-  if constexpr (sizeof(R) == 4) {
-    const R s = acc[idx], yv = v - comp[idx];
-    const R t = s + yv;
-    comp[idx] = (t - s) - yv;
-    acc[idx] = t;
-  } else {
-    acc[idx] += v;
-  }
+  FxIntSum<15> sum;
+#pragma unroll
+  for (int s = 0; s < 5; s++)
+    if (!row_reg_zero(s, B)) sum.add(reg.n[B][s], w[s]);
+  return sum.value();
 }
 
-/* The row's contributions are taken kRowChunk at a time: one pass forms the
-   slot targets of all their patch slots (a binary search in the row's block
-   columns; a ghost slot packs its three parents' targets), one pass forms
-   all their w (45 values each, so the chunk's D loads are in flight
-   together), then the contributions are added one after another in element
-   order: lane t of 9 nen takes block b = t / 9, entry q = t % 9.  FP64
-   values are fused into the block accumulator (acc + sum_s N[s][b] wT[q][s]
-   as one FMA chain), FP32 values are formed alone and added with Kahan
-   compensation; a ghost slot's values go to its parents after the real
-   slots, in slot order, and so do a repeated real node's (a patch at an open
-   boundary that is no ring holds some node twice: kRowSlotDup, one target),
-   so that no two lanes add into one block at once. */
-template <class R>
-__global__ void __launch_bounds__(32 * kRowWarps) k_row_assemble(DevMesh m, KParams p, const R *__restrict__ De,
-                                                                 const R *__restrict__ ntab, R psc, R *__restrict__ K,
-                                                                 int maxblk, int colmajor)
+/* The row's sum in FP64, one contribution after another in element order:
+   for rows with an infinite or NaN element, or of magnitudes near the smallest
+   double (neither in a converging solve).  Lane q < 9 forms entry q. */
+__device__ __noinline__ void row_assemble_raw(const DevMesh &m, int c0, int c1, bool pres_live, double *acc,
+                                              int nb, int lane)
+{
+  for (int t = lane; t < 9 * nb; t += 32) acc[t] = 0.0;
+  __syncwarp();
+  if (lane < 9)
+    for (int c = c0; c < c1; c++) {
+      const int *rc = m.rrec + (size_t)kRowRec * c;
+      const int e = rc[0] & ((1 << 27) - 1), a = rc[0] >> 27, info = rc[1], cs = rc[2], nen = info & 0xff;
+      const double *tab = m.ntab + (info >> 8) * 80;
+      const double *De = m.De + (size_t)kDeStride * e;
+      const int eb = m.dexp[16 * (size_t)e + lane];
+      double w[5];
+      for (int s = 0; s < 5; s++) {
+        w[s] = 0.0;
+        for (int r = 0; r < 5; r++) {
+          const double d = De[fx_place(5 * r + s, lane)];
+          w[s] = fma(tab[16 * r + a], eb == kFxRaw ? d : fx_to_double(Fx{__double2loint(d), __double2hiint(d)}, eb), w[s]);
+        }
+      }
+      const int corner[3] = {cs & 31, (cs >> 5) & 31, (cs >> 10) & 31};
+      const bool acorner = pres_live && (a == corner[0] || a == corner[1] || a == corner[2]);
+      for (int b = 0; b < nen; b++) {
+        const unsigned sl = (unsigned)rc[4 + b];
+        const int np = (sl & kRowSlotGhost) && !(sl & kRowSlotDup) ? 3 : 1;
+        double v = 0.0;
+        for (int s = 0; s < 5; s++) v = fma(tab[16 * s + b], w[s], v);
+        if (acorner)
+          for (int k = 0; k < 3; k++)
+            if (b == corner[k]) v += skew_entry(lane / 3, lane % 3, De + kDePres + 3 * k, 1.0);
+        for (int k = 0; k < np; k++) acc[9 * ((sl >> (10 * k)) & 1023u) + lane] += k == 2 ? -v : v;
+      }
+    }
+}
+
+__global__ void __launch_bounds__(256, 3) k_row_assemble_fx(DevMesh m, KParams p, FxRegular reg, double *__restrict__ K,
+                                                            int maxblk, int colmajor)
 {
   extern __shared__ __align__(16) unsigned char row_smem[];
-  R *tabsT = reinterpret_cast<R *>(row_smem);       /* m.ntabs x 16 x 8: N[s][b] at 8 b + s */
-  for (int t = threadIdx.x; t < m.ntabs * 16 * kRowPad; t += blockDim.x) {
-    const int tb = t / (16 * kRowPad), r = t - tb * 16 * kRowPad, b = r / kRowPad, sidx = r - b * kRowPad;
-    tabsT[t] = sidx < 5 ? ntab[tb * 80 + sidx * 16 + b] : R(0);
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int i = blockIdx.x * kRowWarps + wid;
+  const int i = blockIdx.x * (blockDim.x >> 5) + wid;
   if (i >= p.nt) return;
-  RowAsmBuf<R> B = row_buf<R>(row_smem + align16(m.ntabs * 16 * kRowPad * sizeof(R)) +
-                              (size_t)wid * row_buf_bytes(maxblk, sizeof(R)), maxblk);
+  const FxRowBuf B = fx_row_buf(row_smem + (size_t)wid * fx_row_bytes(maxblk), maxblk);
   const int k0 = m.rowptr[i], nb = m.rowptr[i + 1] - k0;
-  const int kind = m.rowkind[i];
-  R *Kr = K + 9 * (size_t)k0;
-  if (kind != 0) {   /* clamped (R = x - X) and ghost (R = 0) rows: identity */
+  double *Kr = K + 9 * (size_t)k0;
+  if (m.rowkind[i] != 0) {   /* clamped (R = x - X) and ghost (R = 0) rows: identity */
     for (int t = lane; t < 9 * nb; t += 32) {
       const int q = t % 9;
-      Kr[t] = (m.colind[k0 + t / 9] == i && (q == 0 || q == 4 || q == 8)) ? R(1) : R(0);
+      Kr[t] = (m.colind[k0 + t / 9] == i && (q == 0 || q == 4 || q == 8)) ? 1.0 : 0.0;
     }
     return;
   }
-  for (int t = lane; t < nb; t += 32) B.cols[t] = m.colind[k0 + t];
-  for (int t = lane; t < 9 * nb; t += 32) {
-    B.acc[t] = R(0);
-    if constexpr (sizeof(R) == 4) B.comp[t] = R(0);
-  }
+  const int c0 = m.rptr[i], c1 = m.rptr[i + 1];
+  const int4 *rrec4 = reinterpret_cast<const int4 *>(m.rrec);
   const bool pres_live = p.pressure != 0.0 && !p.pres_dead;
-  const int c1 = m.rptr[i + 1];
-  int4 nrec = row_rec_load<kRowChunk>(m.rrec, m.rptr[i], c1, lane);
-  for (int cb = m.rptr[i]; cb < c1; cb += kRowChunk) {
-    const int np = min(kRowChunk, c1 - cb);
-    if (lane < (kRowRec / 4) * np) reinterpret_cast<int4 *>(B.rec)[lane] = nrec;
-    nrec = row_rec_load<kRowChunk>(m.rrec, cb + kRowChunk, c1, lane);   /* the next chunk's, in flight meanwhile */
-    __syncwarp();   /* also orders the cols / acc set-up and the previous chunk's reads */
-    /* w of the chunk: lane u -> contribution u / 45, entry u % 45 */
-    for (int u = lane; u < 45 * np; u += 32) {
-      const int pc = u / 45, t = u - 45 * pc;
-      const int *rc = B.rec + kRowRec * pc;
+  const int pc = lane / 9, q = lane - 9 * pc;       /* contribution and entry; lanes 27..31 idle */
+  int4 nrec = make_int4(0, 0, 0, 0);
+  if (lane < (kRowRec / 4) * min(kRowCopies, c1 - c0)) nrec = __ldg(rrec4 + (size_t)(kRowRec / 4) * c0 + lane);
+  /* the row's exponent of entry q, over all contributions */
+  int eb = 0;
+  for (int c = c0 + pc; c < c1; c += kRowCopies)
+    if (pc < kRowCopies) eb = max(eb, (int)m.dexp[16 * (size_t)(__ldg(m.rrec + (size_t)kRowRec * c) & ((1 << 27) - 1)) + q]);
+  {
+    const int l1 = lane >= 27 ? lane : (lane + 9) % 27, l2 = lane >= 27 ? lane : (lane + 18) % 27;
+    const int x1 = __shfl_sync(0xffffffffu, eb, l1), x2 = __shfl_sync(0xffffffffu, eb, l2);
+    eb = max(eb, max(x1, x2));
+  }
+  const bool raw = __any_sync(0xffffffffu, (eb > 0 && eb < kFxMinExp) || eb > kFxMaxExp);
+  if (raw) {
+    row_assemble_raw(m, c0, c1, pres_live, reinterpret_cast<double *>(B.acc), nb, lane);
+  } else {
+    eb += m.rgrow[i];
+    if (lane < 9) { B.sc[lane] = ldexp(reg.unit, eb - 1022); B.eb[lane] = eb; }
+    long long *acc = B.acc + lane;
+    for (int t = 0; t < nb; t++) acc[kRowWords * t] = 0;
+    for (int cb = c0; cb < c1; cb += kRowCopies) {
+      const int np = min(kRowCopies, c1 - cb);
+      if (lane < (kRowRec / 4) * np) reinterpret_cast<int4 *>(B.rec)[lane] = nrec;
+      if (lane < (kRowRec / 4) * min(kRowCopies, c1 - cb - kRowCopies))
+        nrec = __ldg(rrec4 + (size_t)(kRowRec / 4) * (cb + kRowCopies) + lane);
+      __syncwarp();   /* also orders the set-up */
+      const bool on = pc < np;
+      const int *rc = B.rec + kRowRec * (on ? pc : 0);
       const int e = rc[0] & ((1 << 27) - 1), a = rc[0] >> 27, info = rc[1];
-      int pos;
-      const R v = row_wt_entry(De + (size_t)kDeStride * e, tabsT + (info >> 8) * 16 * kRowPad + kRowPad * a, t, &pos);
-      B.wT[9 * kRowPad * pc + pos] = v;
-    }
-    __syncwarp();
-    for (int pc = 0; pc < np; pc++) {
-      const int *rc = B.rec + kRowRec * pc;
-      const int e = rc[0] & ((1 << 27) - 1), a = rc[0] >> 27, info = rc[1], cs = rc[2];
-      const int nen = info & 0xff;
-      const R *tabT = tabsT + (info >> 8) * 16 * kRowPad;
-      const R *wT = B.wT + 9 * kRowPad * pc;
-      const unsigned *slot = reinterpret_cast<const unsigned *>(rc + 4);
-      const int cslot0 = cs & 31, cslot1 = (cs >> 5) & 31, cslot2 = (cs >> 10) & 31;
-      const bool acorner = pres_live && (a == cslot0 || a == cslot1 || a == cslot2);
-      const bool ghost_lane = lane < nen && (slot[lane] & kRowSlotGhost);
-      const unsigned gmask = __ballot_sync(0xffffffffu, ghost_lane);
-      for (int t = lane; t < 9 * nen; t += 32) {
-        const int b = t / 9, q = t - 9 * b;
-        const unsigned sl = slot[b];
-        const bool ghost = (sl & kRowSlotGhost) != 0;
-        const int idx = 9 * (int)(sl & 1023u) + q;
-        R v;
-        if constexpr (sizeof(R) == 8) v = row_block_accum(wT + kRowPad * q, tabT + kRowPad * b, ghost ? R(0) : B.acc[idx]);
-        else v = row_block_accum(wT + kRowPad * q, tabT + kRowPad * b, R(0));
-        if (acorner) {
-          const int kc = b == cslot0 ? 0 : (b == cslot1 ? 1 : (b == cslot2 ? 2 : -1));
-          if (kc >= 0) v += skew_entry(q / 3, q % 3, De + (size_t)kDeStride * e + kDePres + 3 * kc, psc);
-        }
-        if (ghost) B.gv[t] = v;
-        else if constexpr (sizeof(R) == 8) B.acc[idx] = v;
-        else row_add(B.acc, B.comp, idx, v);
-      }
-      if (gmask) {
-        __syncwarp();
-        /* ghost slots, in slot order: lane 9k + q adds to entry q of parent k */
-        for (unsigned gm = gmask; gm; gm &= gm - 1) {
-          const int b = __ffs(gm) - 1;
-          if (lane < ((slot[b] & kRowSlotDup) ? 9 : 27)) {   /* a repeated real node has one target */
-            const int k = lane / 9, q = lane - 9 * k;
-            const int pos = (int)((slot[b] >> (10 * k)) & 1023u);
-            const R v = B.gv[9 * b + q];
-            row_add(B.acc, B.comp, 9 * pos + q, k == 2 ? -v : v);
+      const int2 *tab = reinterpret_cast<const int2 *>(m.ntabFx) + (info >> 8) * 16 * kFxTab;
+      Fx w[5];
+      if (on) {
+        const int4 *D = reinterpret_cast<const int4 *>(m.De + (size_t)kDeStride * e) + q;
+        const int sh = eb - (int)m.dexp[16 * (size_t)e + q];
+        if ((info >> 8) == 0) {
+          const int *nr = reg.n[a];
+          const int n[5] = {nr[0], nr[1], nr[2], nr[3], nr[4]};
+          FxIntSum<14> sum[5];
+#pragma unroll
+          for (int g = 0; g < 13; g++) {
+            const int4 d = __ldg(D + 9 * g);
+            sum[(2 * g) % 5].add(n[(2 * g) / 5], Fx{d.x, d.y});
+            if (2 * g + 1 < 25) sum[(2 * g + 1) % 5].add(n[(2 * g + 1) / 5], Fx{d.z, d.w});
           }
-          __syncwarp();
+#pragma unroll
+          for (int s = 0; s < 5; s++) w[s] = fx_split(fx_shift(sum[s].value(), sh));
+        } else {
+          Fx n[5];
+#pragma unroll
+          for (int r = 0; r < 5; r++) {
+            const int2 x = __ldg(tab + a * kFxTab + r);
+            n[r] = Fx{x.x, x.y};
+          }
+          FxSum<62> sum[5];
+#pragma unroll
+          for (int g = 0; g < 13; g++) {
+            const int4 d = __ldg(D + 9 * g);
+            sum[(2 * g) % 5].add(n[(2 * g) / 5], Fx{d.x, d.y});
+            if (2 * g + 1 < 25) sum[(2 * g + 1) % 5].add(n[(2 * g + 1) / 5], Fx{d.z, d.w});
+          }
+#pragma unroll
+          for (int s = 0; s < 5; s++) w[s] = fx_split(fx_shift(sum[s].value(), sh));
         }
       }
-      __syncwarp();
+      if (__all_sync(0xffffffffu, rc[3] == 0)) {    /* regular patches without ghost or repeated slots */
+        if (on) {
+          const int4 *sl4 = reinterpret_cast<const int4 *>(rc + 4);
+          const int4 t0 = sl4[0], t1 = sl4[1], t2 = sl4[2];
+          acc[kRowWords * t0.x] += fx_entry_reg<0>(reg, w);
+          acc[kRowWords * t0.y] += fx_entry_reg<1>(reg, w);
+          acc[kRowWords * t0.z] += fx_entry_reg<2>(reg, w);
+          acc[kRowWords * t0.w] += fx_entry_reg<3>(reg, w);
+          acc[kRowWords * t1.x] += fx_entry_reg<4>(reg, w);
+          acc[kRowWords * t1.y] += fx_entry_reg<5>(reg, w);
+          acc[kRowWords * t1.z] += fx_entry_reg<6>(reg, w);
+          acc[kRowWords * t1.w] += fx_entry_reg<7>(reg, w);
+          acc[kRowWords * t2.x] += fx_entry_reg<8>(reg, w);
+          acc[kRowWords * t2.y] += fx_entry_reg<9>(reg, w);
+          acc[kRowWords * t2.z] += fx_entry_reg<10>(reg, w);
+          acc[kRowWords * t2.w] += fx_entry_reg<11>(reg, w);
+        }
+      } else if (on) {
+        const int nen = info & 0xff;
+        for (int b = 0; b < nen; b++) {
+          const unsigned sl = (unsigned)rc[4 + b];
+          Fx n[5];
+#pragma unroll
+          for (int s = 0; s < 5; s++) {
+            const int2 x = __ldg(tab + b * kFxTab + s);
+            n[s] = Fx{x.x, x.y};
+          }
+          const long long v = fx_entry(n, w);
+          acc[kRowWords * (int)(sl & 1023u)] += v;
+          if ((sl & kRowSlotGhost) && !(sl & kRowSlotDup)) {   /* a repeated real node has one target */
+            acc[kRowWords * (int)((sl >> 10) & 1023u)] += v;
+            acc[kRowWords * (int)((sl >> 20) & 1023u)] -= v;
+          }
+        }
+      }
+      if (pres_live) __syncwarp();                   /* the contributions' own adds are done */
+      if (pres_live && on) {
+        /* lane (c, 3 k + d): component d of corner k's vector, entries (i, j) and (j, i) of its cross-product matrix */
+        const int cs = rc[2], s0 = cs & 31, s1 = (cs >> 5) & 31, s2 = (cs >> 10) & 31;
+        if (a == s0 || a == s1 || a == s2) {
+          const int k = q / 3, d = q - 3 * k;
+          const unsigned sl = (unsigned)rc[4 + (k == 0 ? s0 : k == 1 ? s1 : s2)];
+          const double v = m.De[(size_t)kDeStride * e + kDePres + q];
+          const int qm = d == 0 ? 5 : d == 1 ? 6 : 1, qp = d == 0 ? 7 : d == 1 ? 2 : 3;
+          long long *dst = acc - q + kRowWords * (int)(sl & 1023u);
+          dst[qm] -= fx_shift(fx_from_double(v * reg.den2, B.eb[qm] + kFxDenBits), 60 - kFxDenBits - kFxUnit);
+          dst[qp] += fx_shift(fx_from_double(v * reg.den2, B.eb[qp] + kFxDenBits), 60 - kFxDenBits - kFxUnit);
+        }
+      }
+      __syncwarp();   /* the records are rewritten by the next three */
     }
   }
   __syncwarp();
   /* dynamic term diagonal, scale, write-out */
   const double fmax = __longlong_as_double((long long)*m.fmax);
-  const R sc = fmax > 1.0 ? R(1.0 / fmax) : R(1);
-  const int pd = row_find(B.cols, nb, i);
+  const double sc = fmax > 1.0 ? 1.0 / fmax : 1.0;
+  const int pd = p.dyn ? row_find(m.colind + k0, nb, i) : -1;
+  const double dd = p.dyn ? m.dyn_diag[i] : 0.0;
+  int blk = lane / 9, qq = lane - 9 * blk;
   for (int t = lane; t < 9 * nb; t += 32) {
-    R v = B.acc[t];
-    const int q = t % 9;
-    if (p.dyn && t / 9 == pd && (q == 0 || q == 4 || q == 8)) v += R(m.dyn_diag[i]);
-    if (fmax > 1.0) {
-      if constexpr (sizeof(R) == 4) v = (R)((double)v * (1.0 / fmax)); else v = v * sc;
-    }
-    Kr[colmajor ? t - q + 3 * (q % 3) + q / 3 : t] = v;
+    const long long *c = B.acc + kRowWords * blk + qq;
+    double v = raw ? reinterpret_cast<const double *>(B.acc)[t] : (double)(c[0] + c[9] + c[18]) * B.sc[qq];
+    if (blk == pd && qq % 4 == 0) v += dd;
+    if (fmax > 1.0) v *= sc;
+    Kr[colmajor ? t - qq + 3 * (qq % 3) + qq / 3 : t] = v;
+    blk += 3; qq += 5;
+    if (qq >= 9) { qq -= 9; blk++; }
   }
 }
 
-/* FP32 row assembly with the row's blocks owned by lanes: lane k owns block k
-   of the row in registers (9 values) and, in rows of more than 32 blocks
-   (most interior rows: 36 on average in a regular mesh), block 32 + k in
-   shared memory.  One pass over the row's contributions, kRowChunk at a
-   time: slot targets and an inverse map (owned block -> real patch slot) in
-   shared memory, then w of each contribution (lane t and t + 32 of its 45
-   entries), then each owned block's values formed by its owner lane (N[.][b]
-   from the table, the 9 x 5 values of w read by every lane at once) and fused
-   into a per-chunk partial sum; a ghost slot's values go to the lanes owning
-   its parents, after the real slots, in slot order, and so do those of a
-   slot repeating an earlier slot's real node (kRowSlotDup, one owner).  The partial sums are
-   added into the row with Kahan compensation once per chunk, in element
-   order; the second 32 blocks' pass is skipped for a chunk that touches none
-   of them. */
+/* FP32 row assembly, the same way in single precision, each entry with its
+   Kahan compensation beside it.  Latency and the L1 data path bound it:
+   0.38 -> 0.26 ms on the 98,304-triangle sheet (0.31 without the early loads
+   of D). */
 constexpr int kRowRegMax = 64;
 
-struct RowRegBuf {
-  float *wT;          /* kRowChunk x 9 x 8 */
-  float *acc1;        /* 32 x 9 values of the owned blocks 32..63 ([lane][q]); the write-out staging */
-  float *comp;        /* 9 x 32 Kahan compensations of the owned blocks 0..31 ([q][lane]) */
-  float *comp1;       /* 32 x 9 compensations of the owned blocks 32..63 ([lane][q]) */
-  int *cols;          /* kRowRegMax */
-  int *rec;           /* kRowChunk row-assembly records */
-  unsigned char *inv; /* kRowChunk x 64: real slot of each owned block, 255 none */
-};
-
-__host__ __device__ __forceinline__ size_t row_reg_bytes()
+__host__ __device__ __forceinline__ size_t row_f32_bytes(int maxblk)
 {
-  return kRowChunk * 9 * kRowPad * 4 + 3 * 9 * 32 * 4 + kRowRegMax * 4 + kRowChunk * kRowRec * 4 + kRowChunk * 64;
+  return (size_t)kRowWords * maxblk * 8 + kRowCopies * kRowRec * 4;
 }
 
-__device__ __forceinline__ RowRegBuf row_reg_buf(unsigned char *q)
+__device__ __forceinline__ void kahan_add(float2 &a, float v)
 {
-  RowRegBuf b;
-  b.wT = reinterpret_cast<float *>(q);
-  q += kRowChunk * 9 * kRowPad * 4;
-  b.acc1 = reinterpret_cast<float *>(q);
-  q += 9 * 32 * 4;
-  b.comp = reinterpret_cast<float *>(q);
-  q += 9 * 32 * 4;
-  b.comp1 = reinterpret_cast<float *>(q);
-  q += 9 * 32 * 4;
-  b.cols = reinterpret_cast<int *>(q);
-  q += kRowRegMax * 4;
-  b.rec = reinterpret_cast<int *>(q);
-  q += kRowChunk * kRowRec * 4;
-  b.inv = q;
-  return b;
+  const float2 s = a;
+  const float y = v - s.y;
+  const float t = s.x + y;
+  a = make_float2(t, (t - s.x) - y);
 }
 
-/* tmp[q] += sum_s N[s] wT[8 q + s] for the nine entries of one block */
-__device__ __forceinline__ void row_reg_block(const float *wT, const float n[5], float tmp[9])
+template <int B> __device__ __forceinline__ float row_entry_reg(const RowTableF &reg, const float w[5])
 {
+  float v = 0.f;
 #pragma unroll
-  for (int q = 0; q < 9; q++) tmp[q] = row_block_accum(wT + kRowPad * q, n, tmp[q]);
+  for (int s = 0; s < 5; s++)
+    if (!row_reg_zero(s, B)) v = fmaf(reg.n[B][s], w[s], v);
+  return v;
 }
 
-/* The chunk's contributions to owned block k (k = lane or 32 + lane, inverse
-   map column kc) added into tmp: the real slot mapped to k (with its
-   follower-pressure term), then the ghost slots whose parents include k. */
-__device__ __forceinline__ void row_reg_chunk(const RowRegBuf &B, const float *tabsT, const float *De, float psc,
-                                              bool pres_live, int np, int lane, int k, int kc, float tmp[9])
+__device__ __forceinline__ float row_entry(const float n[5], const float w[5])
 {
-  for (int pc = 0; pc < np; pc++) {
-    const int *rc = B.rec + kRowRec * pc;
-    const int a = rc[0] >> 27, info = rc[1], cs = rc[2];
-    const int nen = info & 0xff;
-    const float *tabT = tabsT + (info >> 8) * 16 * kRowPad;
-    const float *wT = B.wT + 9 * kRowPad * pc;
-    const unsigned *slot = reinterpret_cast<const unsigned *>(rc + 4);
-    const int b = B.inv[64 * pc + kc];
-    if (b != 255) {
-      float n[5];
-      load5(tabT + kRowPad * b, n);
-      row_reg_block(wT, n, tmp);
-      const int cslot0 = cs & 31, cslot1 = (cs >> 5) & 31, cslot2 = (cs >> 10) & 31;
-      if (pres_live && (a == cslot0 || a == cslot1 || a == cslot2)) {
-        const int kcr = b == cslot0 ? 0 : (b == cslot1 ? 1 : (b == cslot2 ? 2 : -1));
-        if (kcr >= 0) {
-          const float *vv = De + (size_t)kDeStride * (rc[0] & ((1 << 27) - 1)) + kDePres + 3 * kcr;
+  float v = 0.f;
 #pragma unroll
-          for (int q = 0; q < 9; q++) tmp[q] += skew_entry(q / 3, q % 3, vv, psc);
-        }
-      }
-    }
-    /* ghost slots, in slot order: the owners of the three parents add +, +, - */
-    const bool ghost_lane = lane < nen && (slot[lane] & kRowSlotGhost);
-    for (unsigned gm = __ballot_sync(0xffffffffu, ghost_lane); gm; gm &= gm - 1) {
-      const int gb = __ffs(gm) - 1;
-      const unsigned sl = slot[gb];
-      const int pos0 = (int)(sl & 1023u), pos1 = (int)((sl >> 10) & 1023u), pos2 = (int)((sl >> 20) & 1023u);
-      if (k == pos0 || k == pos1 || k == pos2) {   /* a repeated real node: pos0 = pos1, pos2 none */
-        float n[5], v[9];
-        load5(tabT + kRowPad * gb, n);
-#pragma unroll
-        for (int q = 0; q < 9; q++) v[q] = 0.f;
-        row_reg_block(wT, n, v);
-        const float sg = k == pos2 ? -1.f : 1.f;
-#pragma unroll
-        for (int q = 0; q < 9; q++) tmp[q] = fmaf(sg, v[q], tmp[q]);
-      }
-    }
-  }
+  for (int s = 0; s < 5; s++) v = fmaf(n[s], w[s], v);
+  return v;
 }
 
-__global__ void __launch_bounds__(32 * kRowWarps, 8) k_row_assemble_f32(DevMesh m, KParams p, const float *__restrict__ De,
-                                                                     const float *__restrict__ ntab, float psc,
-                                                                     float *__restrict__ K, int colmajor)
+__global__ void __launch_bounds__(256, 2) k_row_assemble_f32(DevMesh m, KParams p, RowTableF reg,
+                                                             float *__restrict__ K, int maxblk, int colmajor)
 {
   extern __shared__ __align__(16) unsigned char row_smem[];
-  float *tabsT = reinterpret_cast<float *>(row_smem);
-  for (int t = threadIdx.x; t < m.ntabs * 16 * kRowPad; t += blockDim.x) {
-    const int tb = t / (16 * kRowPad), r = t - tb * 16 * kRowPad, b = r / kRowPad, sidx = r - b * kRowPad;
-    tabsT[t] = sidx < 5 ? ntab[tb * 80 + sidx * 16 + b] : 0.f;
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int i = blockIdx.x * kRowWarps + wid;
+  const int i = blockIdx.x * (blockDim.x >> 5) + wid;
   if (i >= p.nt) return;
-  RowRegBuf B = row_reg_buf(row_smem + align16(m.ntabs * 16 * kRowPad * 4) + (size_t)wid * row_reg_bytes());
+  unsigned char *base = row_smem + (size_t)wid * row_f32_bytes(maxblk);
+  float2 *racc = reinterpret_cast<float2 *>(base);                       /* kRowWords maxblk */
+  int *rec = reinterpret_cast<int *>(base + (size_t)kRowWords * maxblk * 8);
   const int k0 = m.rowptr[i], nb = m.rowptr[i + 1] - k0;
   float *Kr = K + 9 * (size_t)k0;
   if (m.rowkind[i] != 0) {   /* clamped and ghost rows: identity */
@@ -920,122 +1004,111 @@ __global__ void __launch_bounds__(32 * kRowWarps, 8) k_row_assemble_f32(DevMesh 
     }
     return;
   }
-  for (int t = lane; t < nb; t += 32) B.cols[t] = m.colind[k0 + t];
-  /* the two w entries of this lane: t0 = lane, t1 = lane + 32 (< 45) */
-  const int wi0 = lane / 15, wk0 = lane - 15 * wi0;
-  const int wpos0 = kRowPad * (3 * wi0 + wk0 % 3) + wk0 / 3, wd0 = wi0 * 15 + wk0;
-  const int t1 = lane + 32, wi1 = t1 / 15, wk1 = t1 - 15 * wi1;
-  const int wpos1 = kRowPad * (3 * wi1 + wk1 % 3) + wk1 / 3, wd1 = wi1 * 15 + wk1;
-  const bool has1 = t1 < 45;
+  const int c0 = m.rptr[i], c1 = m.rptr[i + 1];
+  const int4 *rrec4 = reinterpret_cast<const int4 *>(m.rrec);
   const bool pres_live = p.pressure != 0.0 && !p.pres_dead;
-  const bool two = nb > 32;
-  const double fmax = __longlong_as_double((long long)*m.fmax);
-  float acc[9], tmp[9];
+  const int pc = lane / 9, q = lane - 9 * pc;       /* contribution and entry; lanes 27..31 idle */
+  int4 nrec = make_int4(0, 0, 0, 0);
+  if (lane < (kRowRec / 4) * min(kRowCopies, c1 - c0)) nrec = __ldg(rrec4 + (size_t)(kRowRec / 4) * c0 + lane);
+  float2 *acc = racc + lane;
+  for (int t = 0; t < nb; t++) acc[kRowWords * t] = make_float2(0.f, 0.f);
+  /* D of the next three contributions is in flight while three are added */
+  float4 dn[6];
+  float dn24 = 0.f;
+  auto load_d = [&](int c) {
+    if (pc >= kRowCopies || c >= c1) return;
+    const int e = __ldg(m.rrec + (size_t)kRowRec * c) & ((1 << 27) - 1);
+    const float4 *D = reinterpret_cast<const float4 *>(m.DeF + (size_t)kDeStride * e) + q;
 #pragma unroll
-  for (int q = 0; q < 9; q++) {
-    acc[q] = 0.f;
-    B.comp[32 * q + lane] = 0.f;
-    B.acc1[9 * lane + q] = 0.f;
-    B.comp1[9 * lane + q] = 0.f;
-  }
-  __syncwarp();
-  const int pd = row_find(B.cols, nb, i);
-  const int c1 = m.rptr[i + 1];
-  int4 nrec = row_rec_load<kRowChunk>(m.rrec, m.rptr[i], c1, lane);
-  for (int cb = m.rptr[i]; cb < c1; cb += kRowChunk) {
-    const int np = min(kRowChunk, c1 - cb);
-    if (lane < (kRowRec / 4) * np) reinterpret_cast<int4 *>(B.rec)[lane] = nrec;
-    nrec = row_rec_load<kRowChunk>(m.rrec, cb + kRowChunk, c1, lane);   /* the next chunk's, in flight meanwhile */
-    for (int u = lane; u < kRowChunk * 16; u += 32) reinterpret_cast<unsigned *>(B.inv)[u] = 0xffffffffu;
-    __syncwarp();
-    /* inverse map: owned block -> real slot (lane u -> contribution u / 16, slot u % 16);
-       hi: the chunk reaches a block from 32 on (a real slot or a ghost's parent) */
-    bool hi = false;
-    for (int u = lane; u < 16 * np; u += 32) {
-      const int pc = u >> 4, b = u & 15;
-      const int *rc = B.rec + kRowRec * pc;
-      const unsigned sl = (unsigned)rc[4 + b];
-      if (b < (rc[1] & 0xff)) {
-        if (!(sl & kRowSlotGhost)) {
-          B.inv[64 * pc + sl] = (unsigned char)b;
-          hi |= sl >= 32u;
-        } else {
-          hi |= (sl & 1023u) >= 32u ||
-                (!(sl & kRowSlotDup) && (((sl >> 10) & 1023u) >= 32u || ((sl >> 20) & 1023u) >= 32u));
-        }
-      }
-    }
-    hi = __any_sync(0xffffffffu, hi);
-    for (int pc = 0; pc < np; pc++) {
-      const int *rc = B.rec + kRowRec * pc;
-      const int e = rc[0] & ((1 << 27) - 1), a = rc[0] >> 27, info = rc[1];
-      const float *D = De + (size_t)kDeStride * e;
-      float n[5];
-      load5(tabsT + (info >> 8) * 16 * kRowPad + kRowPad * a, n);
-      float v0 = 0.f, v1 = 0.f;
-#pragma unroll
-      for (int r = 0; r < 5; r++) v0 = fmaf(n[r], __ldg(D + 45 * r + wd0), v0);
-      B.wT[9 * kRowPad * pc + wpos0] = v0;
-      if (has1) {
-#pragma unroll
-        for (int r = 0; r < 5; r++) v1 = fmaf(n[r], __ldg(D + 45 * r + wd1), v1);
-        B.wT[9 * kRowPad * pc + wpos1] = v1;
-      }
-    }
-    __syncwarp();
-    /* h = 0: blocks 0..31, compensated into acc (registers); h = 1: blocks
-       32..63, into acc1 (each lane's own shared-memory column) */
-    for (int h = 0; h < (hi ? 2 : 1); h++) {
-#pragma unroll
-      for (int q = 0; q < 9; q++) tmp[q] = 0.f;
-      row_reg_chunk(B, tabsT, De, psc, pres_live, np, lane, 32 * h + lane, 32 * h + lane, tmp);
-      if (h == 0) {
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-          const float y = tmp[q] - B.comp[32 * q + lane];
-          const float t = acc[q] + y;
-          B.comp[32 * q + lane] = (t - acc[q]) - y;
-          acc[q] = t;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-          const float s = B.acc1[9 * lane + q];
-          const float y = tmp[q] - B.comp1[9 * lane + q];
-          const float t = s + y;
-          B.comp1[9 * lane + q] = (t - s) - y;
-          B.acc1[9 * lane + q] = t;
-        }
-      }
-    }
-    __syncwarp();   /* records, inverse map and wT are rewritten by the next chunk */
-  }
-  /* dynamic term diagonal, scale, block layout; blocks 32.. are written first
-     (from acc1, in place), then acc1 stages blocks 0..31 */
-  auto finish = [&](float v, int k, int q) {
-    if (p.dyn && k == pd && (q == 0 || q == 4 || q == 8)) v += (float)m.dyn_diag[i];
-    if (fmax > 1.0) v = (float)((double)v * (1.0 / fmax));
-    return v;
+    for (int s = 0; s < 6; s++) dn[s] = __ldg(D + 9 * s);
+    dn24 = __ldg(m.DeF + (size_t)kDeStride * e + 216 + q);
   };
-  if (two) {
-    if (32 + lane < nb) {
-      float v[9];
+  load_d(c0 + pc);
+  for (int cb = c0; cb < c1; cb += kRowCopies) {
+    const int np = min(kRowCopies, c1 - cb);
+    if (lane < (kRowRec / 4) * np) reinterpret_cast<int4 *>(rec)[lane] = nrec;
+    if (lane < (kRowRec / 4) * min(kRowCopies, c1 - cb - kRowCopies))
+      nrec = __ldg(rrec4 + (size_t)(kRowRec / 4) * (cb + kRowCopies) + lane);
+    __syncwarp();   /* also orders the set-up */
+    const bool on = pc < np;
+    const int *rc = rec + kRowRec * (on ? pc : 0);
+    const int e = rc[0] & ((1 << 27) - 1), a = rc[0] >> 27, info = rc[1];
+    const float *tab = m.ntabF + (info >> 8) * 80;
+    float w[5];
+    if (on) {
+      float n[5];
 #pragma unroll
-      for (int q = 0; q < 9; q++) v[q] = finish(B.acc1[9 * lane + q], 32 + lane, q);
+      for (int r = 0; r < 5; r++) n[r] = (info >> 8) == 0 ? reg.n[a][r] : __ldg(tab + 16 * r + a);
 #pragma unroll
-      for (int q = 0; q < 9; q++) B.acc1[9 * lane + (colmajor ? 3 * (q % 3) + q / 3 : q)] = v[q];
+      for (int s = 0; s < 5; s++) w[s] = fmaf(n[3], dn[s].w, fmaf(n[2], dn[s].z, fmaf(n[1], dn[s].y, n[0] * dn[s].x)));
+      w[0] = fmaf(n[4], dn[5].x, w[0]); w[1] = fmaf(n[4], dn[5].y, w[1]);
+      w[2] = fmaf(n[4], dn[5].z, w[2]); w[3] = fmaf(n[4], dn[5].w, w[3]);
+      w[4] = fmaf(n[4], dn24, w[4]);
     }
-    __syncwarp();
-    for (int t = lane; t < 9 * (nb - 32); t += 32) Kr[9 * 32 + t] = B.acc1[t];
-    __syncwarp();
-  }
-  if (lane < nb) {
+    load_d(cb + kRowCopies + pc);
+    if (__all_sync(0xffffffffu, rc[3] == 0)) {    /* regular patches without ghost or repeated slots */
+      if (on) {
+        const int4 *sl4 = reinterpret_cast<const int4 *>(rc + 4);
+        const int4 t0 = sl4[0], t1 = sl4[1], t2 = sl4[2];
+        kahan_add(acc[kRowWords * t0.x], row_entry_reg<0>(reg, w));
+        kahan_add(acc[kRowWords * t0.y], row_entry_reg<1>(reg, w));
+        kahan_add(acc[kRowWords * t0.z], row_entry_reg<2>(reg, w));
+        kahan_add(acc[kRowWords * t0.w], row_entry_reg<3>(reg, w));
+        kahan_add(acc[kRowWords * t1.x], row_entry_reg<4>(reg, w));
+        kahan_add(acc[kRowWords * t1.y], row_entry_reg<5>(reg, w));
+        kahan_add(acc[kRowWords * t1.z], row_entry_reg<6>(reg, w));
+        kahan_add(acc[kRowWords * t1.w], row_entry_reg<7>(reg, w));
+        kahan_add(acc[kRowWords * t2.x], row_entry_reg<8>(reg, w));
+        kahan_add(acc[kRowWords * t2.y], row_entry_reg<9>(reg, w));
+        kahan_add(acc[kRowWords * t2.z], row_entry_reg<10>(reg, w));
+        kahan_add(acc[kRowWords * t2.w], row_entry_reg<11>(reg, w));
+      }
+    } else if (on) {
+      const int nen = info & 0xff;
+      for (int b = 0; b < nen; b++) {
+        const unsigned sl = (unsigned)rc[4 + b];
+        float n[5];
 #pragma unroll
-    for (int q = 0; q < 9; q++) B.acc1[9 * lane + (colmajor ? 3 * (q % 3) + q / 3 : q)] = finish(acc[q], lane, q);
+        for (int s = 0; s < 5; s++) n[s] = __ldg(tab + 16 * s + b);
+        const float v = row_entry(n, w);
+        kahan_add(acc[kRowWords * (int)(sl & 1023u)], v);
+        if ((sl & kRowSlotGhost) && !(sl & kRowSlotDup)) {   /* a repeated real node has one target */
+          kahan_add(acc[kRowWords * (int)((sl >> 10) & 1023u)], v);
+          kahan_add(acc[kRowWords * (int)((sl >> 20) & 1023u)], -v);
+        }
+      }
+    }
+    if (pres_live) __syncwarp();                     /* the contributions' own adds are done */
+    if (pres_live && on) {
+      /* lane (c, 3 k + d): component d of corner k's vector, entries (i, j) and (j, i) of its cross-product matrix */
+      const int cs = rc[2], s0 = cs & 31, s1 = (cs >> 5) & 31, s2 = (cs >> 10) & 31;
+      if (a == s0 || a == s1 || a == s2) {
+        const int k = q / 3, d = q - 3 * k;
+        const unsigned sl = (unsigned)rc[4 + (k == 0 ? s0 : k == 1 ? s1 : s2)];
+        const float v = m.DeF[(size_t)kDeStride * e + kDePres + q];
+        float2 *dst = acc - q + kRowWords * (int)(sl & 1023u);
+        kahan_add(dst[d == 0 ? 5 : d == 1 ? 6 : 1], -v);
+        kahan_add(dst[d == 0 ? 7 : d == 1 ? 2 : 3], v);
+      }
+    }
+    __syncwarp();   /* the records are rewritten by the next three */
   }
   __syncwarp();
-  const int nw = 9 * min(32, nb);
-  for (int t = lane; t < nw; t += 32) Kr[t] = B.acc1[t];
+  /* dynamic term diagonal, scale, block layout */
+  const double fmax = __longlong_as_double((long long)*m.fmax);
+  const int pd = p.dyn ? row_find(m.colind + k0, nb, i) : -1;
+  const float dd = p.dyn ? (float)m.dyn_diag[i] : 0.f;
+  int blk = lane / 9, qq = lane - 9 * blk;
+  for (int t = lane; t < 9 * nb; t += 32) {
+    const float2 *c = racc + kRowWords * blk + qq;
+    const float2 s0 = c[0], s1 = c[9], s2 = c[18];
+    float v = ((s0.x + s1.x) + s2.x) - ((s0.y + s1.y) + s2.y);
+    if (blk == pd && qq % 4 == 0) v += dd;
+    if (fmax > 1.0) v = (float)((double)v * (1.0 / fmax));
+    Kr[colmajor ? t - qq + 3 * (qq % 3) + qq / 3 : t] = v;
+    blk += 3; qq += 5;
+    if (qq >= 9) { qq -= 9; blk++; }
+  }
 }
 
 /* Row-assembly records (see DevMesh::rrec), built on the device once per
@@ -1074,7 +1147,14 @@ __global__ void k_row_records(DevMesh m, KParams p, int *__restrict__ rrec)
       r[0] = live ? (e | (a << 27)) : 0;
       r[1] = live ? info : 0;
       r[2] = live ? m.ecorner[e] : 0;
-      r[3] = 0;
+      /* 0: a regular patch of real, distinct nodes */
+      const int *pe = m.patch + 16 * (size_t)e;
+      int general = info != 12;
+      for (int b1 = 0; b1 < nen; b1++) {
+        general |= pe[b1] >= p.nv;
+        for (int b2 = 0; b2 < b1; b2++) general |= pe[b2] == pe[b1];
+      }
+      r[3] = live ? general : 0;
     }
     unsigned sl = 0;
     if (live && b < nen) {
@@ -1092,6 +1172,47 @@ __global__ void k_row_records(DevMesh m, KParams p, int *__restrict__ rrec)
     }
     r[4 + b] = (int)sl;
   }
+}
+
+/* The growth bits of every row of the fixed-point assembly (fx_growth), once
+   per mesh: one warp per row, lane t the bound of block t. */
+__global__ void k_row_growth(DevMesh m, KParams p, unsigned char *__restrict__ rgrow)
+{
+  const int lane = threadIdx.x & 31;
+  const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (i >= p.nt) return;
+  const int nb = m.rowptr[i + 1] - m.rowptr[i];
+  const int c0 = m.rptr[i], c1 = m.rowkind[i] == 0 ? m.rptr[i + 1] : c0;
+  long long most = 0;
+  for (int t = lane; t < nb; t += 32) {
+    long long sum = 0;
+    for (int c = c0; c < c1; c++) {
+      const int *rc = m.rrec + (size_t)kRowRec * c;
+      const int *tab = m.ntabFx + (rc[1] >> 8) * 16 * 2 * kFxTab + 2 * kFxTab - 2;   /* the columns' sums */
+      const int nen = rc[1] & 0xff, a = rc[0] >> 27, cs = rc[2];
+      auto corner = [&](int b) { return b == (cs & 31) || b == ((cs >> 5) & 31) || b == ((cs >> 10) & 31); };
+      int s = 0;
+      for (int b = 0; b < nen; b++) {
+        const unsigned sl = (unsigned)rc[4 + b];
+        const unsigned u = t;
+        const bool hit = (sl & 1023u) == u ||
+                         ((sl & kRowSlotGhost) && !(sl & kRowSlotDup) && (((sl >> 10) & 1023u) == u || ((sl >> 20) & 1023u) == u));
+        if (hit) s += tab[2 * kFxTab * b];
+        if (hit && corner(a) && corner(b)) sum += 64 * 64;      /* the pressure block */
+      }
+      sum += (long long)s * tab[2 * kFxTab * a];
+    }
+    most = max(most, sum);
+  }
+  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+  if (lane == 0) rgrow[i] = (unsigned char)fx_growth(most);
+}
+
+int launch_row_growth(const DevMesh &m, const KParams &p, unsigned char *rgrow, void *stream)
+{
+  const long long threads = 32LL * p.nt;
+  k_row_growth<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m, p, rgrow);
+  return (int)cudaGetLastError();
 }
 
 int launch_row_records(const DevMesh &m, const KParams &p, int *rrec, void *stream)
@@ -1152,7 +1273,7 @@ int launch_elem_tangent(const DevMesh &m, const KParams &p, void *stream)
 
 int launch_elem_tangent_f32(const DevMesh &m, const KParams &p, void *stream)
 {
-  k_elem_tangent_f32<<<blocks_for(p.ne, 32), 32, 0, (cudaStream_t)stream>>>(m, p);
+  k_elem_tangent_f32<<<blocks_for(p.ne, kTanF32Block), kTanF32Block, 0, (cudaStream_t)stream>>>(m, p);
   return (int)cudaGetLastError();
 }
 
@@ -1234,34 +1355,69 @@ int launch_node_gather(const DevMesh &m, const KParams &p, const double *x, doub
   return (int)cudaGetLastError();
 }
 
-/* the staged tables (only the cap table when the mesh has cap elements),
-   then each warp's row buffer */
-size_t row_assemble_smem(int maxblk, bool f32, int ntabs)
+/* Warps a CTA: of 8, 4, 2, 1 the one that keeps most warps on an SM (24 by
+   registers at most for FP64, 32 for FP32; 227 KB shared, 1 KB of it reserved per CTA). */
+static size_t row_bytes(int maxblk, bool f32) { return f32 ? row_f32_bytes(maxblk) : fx_row_bytes(maxblk); }
+
+static int row_warps(int maxblk, bool f32)
 {
-  if (f32) return align16(ntabs * 16 * kRowPad * 4) + kRowWarps * row_reg_bytes();
-  return align16(ntabs * 16 * kRowPad * 8) + kRowWarps * row_buf_bytes(maxblk, 8);
+  int best = 1, most = 0;
+  for (int w = 8; w >= 1; w /= 2) {
+    const int ctas = (int)(228 * 1024 / (w * row_bytes(maxblk, f32) + 1024));
+    const int warps = std::min(w * ctas, f32 ? 32 : 24);
+    if (warps > most) { most = warps; best = w; }
+  }
+  return best;
+}
+
+size_t row_assemble_smem(int maxblk, bool f32) { return row_warps(maxblk, f32) * row_bytes(maxblk, f32); }
+
+/* The regular table for the row assemblies; false when it does not have the
+   zeros or (FP64) the common denominator that they rely on. */
+bool regular_tables(const double *tab0, int den, RowTables &t)
+{
+  bool ok = true;
+  for (int b = 0; b < 12; b++)
+    for (int s = 0; s < 5; s++) {
+      const double v = tab0[16 * s + b];
+      const int k = (int)llrint(v * den);
+      ok &= (double)k / den == v && (!row_reg_zero(s, b) || k == 0);
+      t.x.n[b][s] = k;
+      t.f.n[b][s] = (float)v;
+    }
+  t.x.den2 = (double)den * den;
+  t.x.unit = ldexp(1.0 / t.x.den2, -kFxUnit);
+  return ok;
 }
 
 int row_assemble_max_blocks(bool f32) { return f32 ? kRowRegMax : kMaxRowBlocks; }
 
-int launch_row_assemble(const DevMesh &m, const KParams &p, void *K, bool f32, bool colmajor, void *stream)
+int launch_row_assemble(const DevMesh &m, const KParams &p, const RowTables &t, void *K, bool f32, bool colmajor, void *stream)
 {
-  const int grid = blocks_for(p.nt, kRowWarps);
-  const size_t smem = row_assemble_smem(m.maxblk, f32, m.ntabs);
+  const int warps = row_warps(m.maxblk, f32);
+  const int grid = blocks_for(p.nt, warps);
+  const size_t smem = row_assemble_smem(m.maxblk, f32);
   if (f32)
-    k_row_assemble_f32<<<grid, 32 * kRowWarps, smem, (cudaStream_t)stream>>>(
-        m, p, m.DeF, m.ntabF, -p.pres6f, static_cast<float *>(K), (int)colmajor);
+    k_row_assemble_f32<<<grid, 32 * warps, smem, (cudaStream_t)stream>>>(
+        m, p, t.f, static_cast<float *>(K), m.maxblk, (int)colmajor);
   else
-    k_row_assemble<double><<<grid, 32 * kRowWarps, smem, (cudaStream_t)stream>>>(
-        m, p, m.De, m.ntab, -p.pressure / 6.0, static_cast<double *>(K), m.maxblk, (int)colmajor);
+    k_row_assemble_fx<<<grid, 32 * warps, smem, (cudaStream_t)stream>>>(
+        m, p, t.x, static_cast<double *>(K), m.maxblk, (int)colmajor);
   return (int)cudaGetLastError();
 }
 
-int row_assemble_configure(int maxblk, bool f32, int ntabs)
+/* The kernels' dynamic shared-memory limit is raised to the device's, once and
+   for every handle (a limit set to one handle's need would fail another's
+   larger launch); a row buffer that does not fit is refused here. */
+int row_assemble_configure(int maxblk, bool f32)
 {
-  const size_t smem = row_assemble_smem(maxblk, f32, ntabs);
-  cudaError_t e = f32 ? cudaFuncSetAttribute(k_row_assemble_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                      : cudaFuncSetAttribute(k_row_assemble<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess && row_assemble_smem(maxblk, f32) > (size_t)optin) e = cudaErrorInvalidValue;
+  if (e == cudaSuccess)
+    e = f32 ? cudaFuncSetAttribute(k_row_assemble_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)
+            : cudaFuncSetAttribute(k_row_assemble_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
   return (int)e;
 }
 
