@@ -447,16 +447,16 @@ __host__ __device__ __forceinline__ void elem_out(const ElemGeom<R> &g, const R 
 /* The thickness-integrated resultants N = (N11, N22, N12) and M, scaled by
    pref0; ref is the element's column of constants.  With
    `grad`, out(q, w, th3, C) receives each thickness point's stress gradient
-   (qp_stress), w the point's weight times pref0. */
+   (qp_stress), w the point's weight times pref0.  Points q0, q0 + dq, ... only. */
 template <class R, class Grad>
 __host__ __device__ __forceinline__ void elem_resultants(const ElemGeom<R> &g, const EPar<R> &p, const RefCol<R> &ref,
                                                          R N[3], R M[3], int &status, bool final_update,
-                                                         bool grad, Grad out)
+                                                         bool grad, Grad out, int q0 = 0, int dq = 1)
 {
   const int nq = p.nq;
   const R pref0 = ref(kRefPerQp * nq);
   for (int i = 0; i < 3; i++) N[i] = M[i] = R(0);
-  for (int q = 0; q < nq; q++) {
+  for (int q = q0; q < nq; q += dq) {
     const R th3 = p.hhalf * p.theta[q];
     R gm[5], sv[3] = {R(0), R(0), R(0)};
     qp_metric(g, th3, gm);
@@ -567,38 +567,46 @@ template <class R> struct TanMoments {
   }
 };
 
-/* st(k, value) for every k < kTanCoefs */
-template <class R, class Store>
-__host__ __device__ __forceinline__ void tangent_coefs(const ElemGeom<R> &g, const R N[3], const R M[3],
-                                                       const TanMoments<R> &mo, int tnormal, Store st)
-{
-  const R two = R(2);
-  const R b11 = dot(g.n, g.Aaa), b22 = dot(g.n, g.Abb), b12 = dot(g.n, g.Aab);
-  const R G11 = dot(g.gc1, g.gc1), G22 = dot(g.gc2, g.gc2), G12 = dot(g.gc1, g.gc2);
-  const R s111 = dot(g.gc1, g.Aaa), s122 = dot(g.gc1, g.Abb), s112 = dot(g.gc1, g.Aab);   /* G^1_11 G^1_22 G^1_12 */
-  const R s211 = dot(g.gc2, g.Aaa), s222 = dot(g.gc2, g.Abb), s212 = dot(g.gc2, g.Aab);
-  const R k1 = tnormal ? R(0) : s111 + s212, k2 = tnormal ? R(0) : s112 + s222;
-  /* b^c_a = a^cd b_da */
-  const R m11 = G11 * b11 + G12 * b12, m21 = G12 * b11 + G22 * b12;
-  const R m12 = G11 * b12 + G12 * b22, m22 = G12 * b12 + G22 * b22;
-  /* dh along (a11, a22, a12) and (b11, b22, b12), rows h11, h22, h12 */
-  const R ha[3][3] = {{-(m11 * m11), -(m21 * m21), -(two * m11 * m21)},
-                      {-(m12 * m12), -(m22 * m22), -(two * m12 * m22)},
-                      {-(m11 * m12), -(m21 * m22), -(m11 * m22 + m21 * m12)}};
-  const R hb[3][3] = {{two * m11, R(0), two * m21}, {R(0), two * m22, two * m12}, {m12, m21, m11 + m22}};
-#pragma unroll
-  for (int m = 0; m < 6; m++) {
-    const int i = m % 3, t = m / 3;                 /* N rows take th^0..2, M rows th^1..3 */
+/* What the tangent coefficients of every resultant share. */
+template <class R> struct TanShape {
+  R b11, b22, b12, G11, G22, G12;
+  R s111, s122, s112, s211, s222, s212;    /* G^1_11 G^1_22 G^1_12, G^2_.. */
+  R k1, k2;
+  R m11, m21, m12, m22;                    /* b^c_a = a^cd b_da */
+  int tnormal;
+
+  __host__ __device__ __forceinline__ TanShape(const ElemGeom<R> &g, int tn) : tnormal(tn)
+  {
+    b11 = dot(g.n, g.Aaa); b22 = dot(g.n, g.Abb); b12 = dot(g.n, g.Aab);
+    G11 = dot(g.gc1, g.gc1); G22 = dot(g.gc2, g.gc2); G12 = dot(g.gc1, g.gc2);
+    s111 = dot(g.gc1, g.Aaa); s122 = dot(g.gc1, g.Abb); s112 = dot(g.gc1, g.Aab);
+    s211 = dot(g.gc2, g.Aaa); s222 = dot(g.gc2, g.Abb); s212 = dot(g.gc2, g.Aab);
+    k1 = tn ? R(0) : s111 + s212; k2 = tn ? R(0) : s112 + s222;
+    m11 = G11 * b11 + G12 * b12; m21 = G12 * b11 + G22 * b12;
+    m12 = G11 * b12 + G12 * b22; m22 = G12 * b12 + G22 * b22;
+  }
+
+  /* the coefficients of resultant m = 3 t + i: T0..T2 the moments t .. t + 2 of
+     the i-th stress's 00, 11, 01 columns, U the moment t + 1 of 02, 12 */
+  template <class Store>
+  __host__ __device__ __forceinline__ void row(int m, const R T0[3], const R T1[3], const R T2[3], const R U[2], Store st) const
+  {
+    const R two = R(2);
+    /* dh along (a11, a22, a12) and (b11, b22, b12), rows h11, h22, h12 */
+    const R ha[3][3] = {{-(m11 * m11), -(m21 * m21), -(two * m11 * m21)},
+                        {-(m12 * m12), -(m22 * m22), -(two * m12 * m22)},
+                        {-(m11 * m12), -(m21 * m22), -(m11 * m22 + m21 * m12)}};
+    const R hb[3][3] = {{two * m11, R(0), two * m21}, {R(0), two * m22, two * m12}, {m12, m21, m11 + m22}};
     const R sc = m == 5 ? two : R(1);
     R Ha[3], Hb[3];
-    const R h0 = mo.T[t + 2][3 * i], h1 = mo.T[t + 2][3 * i + 1], h2 = mo.T[t + 2][3 * i + 2];
+    const R h0 = T2[0], h1 = T2[1], h2 = T2[2];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      Ha[c] = sc * (mo.T[t][3 * i + c] + (h0 * ha[0][c] + h1 * ha[1][c] + h2 * ha[2][c]));
-      Hb[c] = sc * ((h0 * hb[0][c] + h1 * hb[1][c] + h2 * hb[2][c]) - two * mo.T[t + 1][3 * i + c]);
+      Ha[c] = sc * (T0[c] + (h0 * ha[0][c] + h1 * ha[1][c] + h2 * ha[2][c]));
+      Hb[c] = sc * ((h0 * hb[0][c] + h1 * hb[1][c] + h2 * hb[2][c]) - two * T1[c]);
     }
-    const R Hk1 = tnormal ? R(0) : sc * (mo.U[t][2 * i] + two * k1 * h0 + k2 * h2);
-    const R Hk2 = tnormal ? R(0) : sc * (mo.U[t][2 * i + 1] + two * k2 * h1 + k1 * h2);
+    const R Hk1 = tnormal ? R(0) : sc * (U[0] + two * k1 * h0 + k2 * h2);
+    const R Hk2 = tnormal ? R(0) : sc * (U[1] + two * k2 * h1 + k1 * h2);
     const int o = kTcRow * m;
     st(o + kTcA1, two * Ha[0]); st(o + kTcA2, two * Ha[1]); st(o + kTcA12, Ha[2]);
     st(o + kTcZ1, (Hk1 * m11 + Hk2 * m12) - (Hb[0] * s111 + Hb[1] * s122 + Hb[2] * s112));
@@ -608,17 +616,37 @@ __host__ __device__ __forceinline__ void tangent_coefs(const ElemGeom<R> &g, con
     st(o + kTcB11, Hb[0]); st(o + kTcB22, Hb[1]); st(o + kTcB12, Hb[2]);
     st(o + kTcK1, Hk1); st(o + kTcK2, Hk2);
   }
-  const V3<R> v[5] = {g.a1, g.a2, g.n, g.gc1, g.gc2};
+
+  /* the rest: vectors, resultants and what is formed from them */
+  template <class Store>
+  __host__ __device__ __forceinline__ void rest(const ElemGeom<R> &g, const R N[3], const R M[3], Store st) const
+  {
+    const V3<R> v[5] = {g.a1, g.a2, g.n, g.gc1, g.gc2};
 #pragma unroll
-  for (int k = 0; k < 5; k++) { st(kTcVec + 3 * k, v[k].x); st(kTcVec + 3 * k + 1, v[k].y); st(kTcVec + 3 * k + 2, v[k].z); }
-  const R M2 = two * M[2];
-  st(kTcRes, N[0]); st(kTcRes + 1, N[1]); st(kTcRes + 2, N[2]);
-  st(kTcRes + 3, M[0]); st(kTcRes + 4, M[1]); st(kTcRes + 5, M2);
-  st(kTcQ, M[0] * s111 + M[1] * s122 + M2 * s112); st(kTcQ + 1, M[0] * s211 + M[1] * s222 + M2 * s212);
-  st(kTcGam, s111); st(kTcGam + 1, s122); st(kTcGam + 2, s112);
-  st(kTcGam + 3, s211); st(kTcGam + 4, s222); st(kTcGam + 5, s212);
-  const R mb = M[0] * b11 + M[1] * b22 + M2 * b12;
-  st(kTcE, mb * G11); st(kTcE + 1, mb * G12); st(kTcE + 2, mb * G22);
+    for (int k = 0; k < 5; k++) { st(kTcVec + 3 * k, v[k].x); st(kTcVec + 3 * k + 1, v[k].y); st(kTcVec + 3 * k + 2, v[k].z); }
+    const R M2 = R(2) * M[2];
+    st(kTcRes, N[0]); st(kTcRes + 1, N[1]); st(kTcRes + 2, N[2]);
+    st(kTcRes + 3, M[0]); st(kTcRes + 4, M[1]); st(kTcRes + 5, M2);
+    st(kTcQ, M[0] * s111 + M[1] * s122 + M2 * s112); st(kTcQ + 1, M[0] * s211 + M[1] * s222 + M2 * s212);
+    st(kTcGam, s111); st(kTcGam + 1, s122); st(kTcGam + 2, s112);
+    st(kTcGam + 3, s211); st(kTcGam + 4, s222); st(kTcGam + 5, s212);
+    const R mb = M[0] * b11 + M[1] * b22 + M2 * b12;
+    st(kTcE, mb * G11); st(kTcE + 1, mb * G12); st(kTcE + 2, mb * G22);
+  }
+};
+
+/* st(k, value) for every k < kTanCoefs */
+template <class R, class Store>
+__host__ __device__ __forceinline__ void tangent_coefs(const ElemGeom<R> &g, const R N[3], const R M[3],
+                                                       const TanMoments<R> &mo, int tnormal, Store st)
+{
+  const TanShape<R> sh(g, tnormal);
+#pragma unroll
+  for (int m = 0; m < 6; m++) {
+    const int i = m % 3, t = m / 3;                 /* N rows take th^0..2, M rows th^1..3 */
+    sh.row(m, mo.T[t] + 3 * i, mo.T[t + 1] + 3 * i, mo.T[t + 2] + 3 * i, mo.U[t] + 2 * i, st);
+  }
+  sh.rest(g, N, M, st);
 }
 
 /* Columns 3 s .. 3 s + 2 of D (s = 0..4: a1, a2, Aaa, Abb, Aab) from the

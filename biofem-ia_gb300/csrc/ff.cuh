@@ -77,9 +77,9 @@ __host__ __device__ __forceinline__ FF operator*(FF a, FF b)
 __host__ __device__ __forceinline__ FF operator/(FF a, FF b)
 {
   const float q1 = a.hi / b.hi;
-  const FF r = a - b * FF(q1, 0.f);
-  const float q2 = r.hi / b.hi;
-  return ff_fast_two_sum(q1, q2);
+  /* the remainder of a correctly rounded quotient is a float: exact by one fused multiply-add */
+  const float r = fmaf(-q1, b.lo, fmaf(-q1, b.hi, a.hi) + a.lo);
+  return ff_fast_two_sum(q1, r / b.hi);
 }
 
 __host__ __device__ __forceinline__ FF &operator+=(FF &a, FF b) { a = a + b; return a; }
@@ -96,8 +96,8 @@ __host__ __device__ __forceinline__ FF dsqrt(FF a)
 {
   if (!(a.hi > 0.f)) return FF(sqrtf(a.hi), 0.f);
   const float s = sqrtf(a.hi);
-  const FF r = a - ff_two_prod(s, s);
-  return ff_fast_two_sum(s, r.hi / (2.f * s));
+  const float r = fmaf(-s, s, a.hi) + a.lo;      /* a.hi - s^2 is exact */
+  return ff_fast_two_sum(s, r / (2.f * s));
 }
 
 __host__ __device__ __forceinline__ FF val(FF a) { return a; }

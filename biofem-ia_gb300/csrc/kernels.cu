@@ -250,7 +250,13 @@ __device__ __forceinline__ void elem_pressure_force(const DevMesh &m, const KPar
   const V3<double> d21 = {X[1][0] - X[0][0], X[1][1] - X[0][1], X[1][2] - X[0][2]};
   const V3<double> d31 = {X[2][0] - X[0][0], X[2][1] - X[0][1], X[2][2] - X[0][2]};
   const V3<double> ca = cross(d21, d31);
-  const double nrm = sqrt(ca.x * ca.x + ca.y * ca.y + ca.z * ca.z);
+  const double n2 = dot(ca, ca);
+  if (n2 > 1e-280 && n2 < 1e280) {   /* |ca| cancels; a square root and three divisions less */
+    const double sc = p.pressure * (1.0 / 6.0);
+    m.fp[e] = ca.x * sc; m.fp[ne + e] = ca.y * sc; m.fp[2 * ne + e] = ca.z * sc;
+    return;
+  }
+  const double nrm = sqrt(n2);       /* a triangle without area gives NaN */
   const double dA = 0.5 * nrm;
   m.fp[e] = (ca.x / nrm) * p.pressure * dA / 3.;
   m.fp[ne + e] = (ca.y / nrm) * p.pressure * dA / 3.;
@@ -273,25 +279,60 @@ __device__ __forceinline__ void store_pressure_vectors(const R av[3], const R bv
   }
 }
 
-/* One thread per element.  For the R + K call (tan) it also evaluates the
+/* L = 1: one thread per element.  For the R + K call (tan) it also evaluates the
    stress gradients (about 300 FP64 operations a thickness point beside the
    400 of the stress itself), keeps them in cq between the thickness loop and
    the moments (its own column: 15 values a point would not fit in registers
    beside the stress), and stores the kTanCoefs tangent coefficients
    k_elem_tangent reads.  One kernel serves both calls, so that R is bit for
-   bit the same: two instances would contract multiply-adds differently. */
-__global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, bool tan)
+   bit the same: two instances would contract multiply-adds differently.
+
+   L = 3: three lanes per element (ten elements a warp), for meshes that leave
+   FP64 units idle (residual_lanes).  Lane s gathers Cartesian component s of
+   y, takes thickness points s, s + 3, .., forms the tangent coefficients of
+   the two resultants of stress s (N11 and M11, ..) from their moments alone, and
+   scatters component s of the force; the geometry in between is formed by all
+   three.  A chain of 730 FP64 operations (1,280 with gradients) in place of
+   1,850 (3,820), at 64 cycles each. */
+template <int L> constexpr int kResElems = 32 / L;      /* elements a warp */
+constexpr int kResBlock = 128;
+
+/* lane s's component of the three lanes' doubles, in every lane */
+__device__ __forceinline__ double lane3(double v, int base, int s) { return __shfl_sync(0xffffffffu, v, base + s); }
+
+template <int L>
+__global__ void __launch_bounds__(kResBlock) k_elem_residual(DevMesh m, KParams p, bool tan)
 {
+  static_assert(L == 1 || L == 3, "one thread, or one lane per Cartesian component");
   __shared__ double tabs[kNumTables * 80];
   for (int i = threadIdx.x; i < kNumTables * 80; i += blockDim.x) tabs[i] = m.ntab[i];
   __syncthreads();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= p.ne) return;
+  const int lane = threadIdx.x & 31;
+  const int e0 = L == 1 ? blockIdx.x * kResBlock + threadIdx.x
+                        : (blockIdx.x * (kResBlock / 32) + (threadIdx.x >> 5)) * kResElems<L> + min(lane / L, kResElems<L> - 1);
+  if (L == 1 ? e0 >= p.ne : __all_sync(0xffffffffu, e0 >= p.ne)) return;
+  const int e = min(e0, p.ne - 1), s = lane % L, base = L * min(lane / L, kResElems<L> - 1);
+  const bool live = e0 < p.ne && lane < L * kResElems<L>;     /* the others repeat an element */
   const int info = m.einfo[e];
   const int nen = info & 0xff, tabi = info >> 8;
   const double *tab = tabs + tabi * 80;
   double y[15];
-  gather_y(m.pos, m.patch, e, nen, tab, y);
+  if constexpr (L == 1) {
+    gather_y(m.pos, m.patch, e, nen, tab, y);
+  } else {
+    double ys[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    const int *pe = m.patch + 16 * (size_t)e;
+#pragma unroll 4
+    for (int i = 0; i < nen; i++) {
+      const double x = __ldg(m.pos + 4 * (size_t)__ldg(pe + i) + s);
+#pragma unroll
+      for (int r = 0; r < 5; r++) ys[r] += tab[r * 16 + i] * x;
+    }
+#pragma unroll
+    for (int r = 0; r < 5; r++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) y[3 * r + d] = lane3(ys[r], base, d);
+  }
   double f[15];
   int st = 0;
   const EPar<double> ep = epar<double>(p);
@@ -300,25 +341,47 @@ __global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, boo
   double N[3], M[3];
   elem_resultants<double>(g, ep, RefCol<double>{m.eref + e, ne}, N, M, st, true, tan, [&](int q, double w, double, double C[3][5]) {
     double *cq = m.cq + e;
-    for (int i = 0; i < 3; i++)
-      for (int k = 0; k < 5; k++) cq[(size_t)(15 * q + 5 * i + k) * ne] = w * C[i][k];
-  });
+    if (live)
+      for (int i = 0; i < 3; i++)
+        for (int k = 0; k < 5; k++) cq[(size_t)(15 * q + 5 * i + k) * ne] = w * C[i][k];
+  }, s, L);
+  if constexpr (L == 3) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      N[i] = lane3(N[i], base, 0) + lane3(N[i], base, 1) + lane3(N[i], base, 2);
+      M[i] = lane3(M[i], base, 0) + lane3(M[i], base, 1) + lane3(M[i], base, 2);
+    }
+  }
   elem_out(g, N, M, f);
   set_status(m.status, st);
   /* Fb_a = sum_r N[r][a] f_r, stored slot-major: fb[(3a+d)*ne + e] */
-  for (int a = 0; a < nen; a++) {
-    double fx = 0.0, fy = 0.0, fz = 0.0;
+  if constexpr (L == 1) {
+    for (int a = 0; a < nen; a++) {
+      double fx = 0.0, fy = 0.0, fz = 0.0;
 #pragma unroll
-    for (int r = 0; r < 5; r++) {
-      const double c = tab[r * 16 + a];
-      fx += c * f[3 * r]; fy += c * f[3 * r + 1]; fz += c * f[3 * r + 2];
+      for (int r = 0; r < 5; r++) {
+        const double c = tab[r * 16 + a];
+        fx += c * f[3 * r]; fy += c * f[3 * r + 1]; fz += c * f[3 * r + 2];
+      }
+      m.fb[(3 * a) * ne + e] = fx;
+      m.fb[(3 * a + 1) * ne + e] = fy;
+      m.fb[(3 * a + 2) * ne + e] = fz;
     }
-    m.fb[(3 * a) * ne + e] = fx;
-    m.fb[(3 * a + 1) * ne + e] = fy;
-    m.fb[(3 * a + 2) * ne + e] = fz;
+  } else {
+    double fs[5];
+#pragma unroll
+    for (int r = 0; r < 5; r++) fs[r] = s == 0 ? f[3 * r] : s == 1 ? f[3 * r + 1] : f[3 * r + 2];
+    for (int a = 0; a < nen; a++) {
+      double v = 0.0;
+#pragma unroll
+      for (int r = 0; r < 5; r++) v += tab[r * 16 + a] * fs[r];
+      if (live) m.fb[(3 * a + s) * ne + e] = v;
+    }
   }
-  if (p.pressure != 0.0) elem_pressure_force(m, p, e);
-  if (tan) {
+  if (live && s == 0 && p.pressure != 0.0) elem_pressure_force(m, p, e);
+  if (!tan) return;
+  double *tc = m.tcoef + e;
+  if constexpr (L == 1) {
     TanMoments<double> mo;
     mo.clear();
     for (int q = 0; q < ep.nq; q++) {
@@ -327,15 +390,33 @@ __global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, boo
         for (int k = 0; k < 5; k++) C[i][k] = m.cq[(size_t)(15 * q + 5 * i + k) * ne + e];
       mo.add(1.0, ep.hhalf * ep.theta[q], C);
     }
-    double *tc = m.tcoef + e;
     tangent_coefs<double>(g, N, M, mo, ep.tnormal, [&](int k, double v) { tc[(size_t)k * ne] = v; });
-    if (p.pressure != 0.0 && !p.pres_dead) {
-      double X[3][3];
-      for (int k = 0; k < 3; k++) load_node(m.pos, m.etri[3 * (size_t)e + k], X[k][0], X[k][1], X[k][2]);
-      const double av[3] = {X[1][0] - X[0][0], X[1][1] - X[0][1], X[1][2] - X[0][2]};
-      const double bv[3] = {X[2][0] - X[0][0], X[2][1] - X[0][1], X[2][2] - X[0][2]};
-      store_pressure_vectors<double>(av, bv, -p.pressure / 6.0, m.De + (size_t)kDeStride * e + kDePres);
+  } else {
+    __syncwarp();                                  /* the other lanes' gradients */
+    double T[4][3] = {}, U[2][2] = {};             /* TanMoments of stress s */
+    for (int q = 0; q < ep.nq; q++) {
+      const double th = ep.hhalf * ep.theta[q], th2 = th * th, th3 = th2 * th;
+      const double *C = m.cq + (size_t)(15 * q + 5 * s) * ne + e;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double v = C[(size_t)c * ne];
+        T[0][c] += v; T[1][c] += th * v; T[2][c] += th2 * v; T[3][c] += th3 * v;
+      }
+#pragma unroll
+      for (int c = 0; c < 2; c++) { const double v = C[(size_t)(3 + c) * ne]; U[0][c] += th * v; U[1][c] += th2 * v; }
     }
+    const TanShape<double> sh(g, ep.tnormal);
+    auto put = [&](int k, double v) { if (live) tc[(size_t)k * ne] = v; };
+    sh.row(s, T[0], T[1], T[2], U[0], put);
+    sh.row(3 + s, T[1], T[2], T[3], U[1], put);
+    if (live && s == 0) sh.rest(g, N, M, put);
+  }
+  if (live && s == 0 && p.pressure != 0.0 && !p.pres_dead) {
+    double X[3][3];
+    for (int k = 0; k < 3; k++) load_node(m.pos, m.etri[3 * (size_t)e + k], X[k][0], X[k][1], X[k][2]);
+    const double av[3] = {X[1][0] - X[0][0], X[1][1] - X[0][1], X[1][2] - X[0][2]};
+    const double bv[3] = {X[2][0] - X[0][0], X[2][1] - X[0][1], X[2][2] - X[0][2]};
+    store_pressure_vectors<double>(av, bv, -p.pressure / 6.0, m.De + (size_t)kDeStride * e + kDePres);
   }
 }
 
@@ -348,28 +429,40 @@ __global__ void __launch_bounds__(128) k_elem_residual(DevMesh m, KParams p, boo
    float-float, whose error sits near 1e-13.  Node positions are taken
    relative to the element's first corner in FP64 before the split, the shift
    is put back through (sum_i N_r[i]) x_c; the element forces leave as
-   doubles (hi + lo is exact in FP64) for the FP64 node sums. */
-__global__ void __launch_bounds__(128, 3) k_elem_residual_ff(DevMesh m, KParams p)
+   doubles (hi + lo is exact in FP64) for the FP64 node sums.
+
+   L = 3 shares an element among three lanes, as k_elem_residual does. */
+__device__ __forceinline__ FF lane3(FF v, int base, int s)
+{
+  return FF(__shfl_sync(0xffffffffu, v.hi, base + s), __shfl_sync(0xffffffffu, v.lo, base + s));
+}
+
+template <int L>
+__global__ void __launch_bounds__(kResBlock, 3) k_elem_residual_ff(DevMesh m, KParams p)
 {
   __shared__ FF tabs[kNumTables * 85];   /* tables, then their row sums */
   const FF *ntab = static_cast<const FF *>(m.ntabFF);
   for (int i = threadIdx.x; i < kNumTables * 85; i += blockDim.x) tabs[i] = ntab[i];
   __syncthreads();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= p.ne) return;
+  const int lane = threadIdx.x & 31;
+  const int e0 = L == 1 ? blockIdx.x * kResBlock + threadIdx.x
+                        : (blockIdx.x * (kResBlock / 32) + (threadIdx.x >> 5)) * kResElems<L> + min(lane / L, kResElems<L> - 1);
+  if (L == 1 ? e0 >= p.ne : __all_sync(0xffffffffu, e0 >= p.ne)) return;
+  const int e = min(e0, p.ne - 1), s = lane % L, base = L * min(lane / L, kResElems<L> - 1);
+  const bool live = e0 < p.ne && lane < L * kResElems<L>;     /* the others repeat an element */
   const int info = m.einfo[e];
   const int nen = info & 0xff, tabi = info >> 8;
   const FF *tab = tabs + tabi * 80, *tsum = tabs + kNumTables * 80 + tabi * 5;
-  double xc[3];
-  load_node(m.pos, m.etri[3 * (size_t)e], xc[0], xc[1], xc[2]);
+  const int *pe = m.patch + 16 * (size_t)e;
   FF y[15];
-  {
+  if constexpr (L == 1) {
+    double xc[3];
+    load_node(m.pos, m.etri[3 * (size_t)e], xc[0], xc[1], xc[2]);
     FFAcc acc[15] = {
 #define BIOFEM_Y0(r) FFAcc(tsum[r], ff_split(xc[0])), FFAcc(tsum[r], ff_split(xc[1])), FFAcc(tsum[r], ff_split(xc[2]))
         BIOFEM_Y0(0), BIOFEM_Y0(1), BIOFEM_Y0(2), BIOFEM_Y0(3), BIOFEM_Y0(4)
 #undef BIOFEM_Y0
     };
-    const int *pe = m.patch + 16 * (size_t)e;
     for (int i = 0; i < nen; i++) {
       double X, Y, Z;
       load_node(m.pos, __ldg(pe + i), X, Y, Z);
@@ -383,26 +476,65 @@ __global__ void __launch_bounds__(128, 3) k_elem_residual_ff(DevMesh m, KParams 
     }
 #pragma unroll
     for (int k = 0; k < 15; k++) y[k] = acc[k].get();
+  } else {
+    const double xc = __ldg(m.pos + 4 * (size_t)m.etri[3 * (size_t)e] + s);
+    const FF c0 = ff_split(xc);
+    FFAcc acc[5] = {FFAcc(tsum[0], c0), FFAcc(tsum[1], c0), FFAcc(tsum[2], c0), FFAcc(tsum[3], c0), FFAcc(tsum[4], c0)};
+#pragma unroll 4
+    for (int i = 0; i < nen; i++) {
+      const FF d = ff_split(__ldg(m.pos + 4 * (size_t)__ldg(pe + i) + s) - xc);
+#pragma unroll
+      for (int r = 0; r < 5; r++) acc[r].add(tab[r * 16 + i], d);
+    }
+#pragma unroll
+    for (int r = 0; r < 5; r++) {
+      const FF v = acc[r].get();
+#pragma unroll
+      for (int d = 0; d < 3; d++) y[3 * r + d] = lane3(v, base, d);
+    }
   }
   FF f[15];
   int st = 0;
   const EPar<FF> ep = epar<FF>(p);
-  elem_forces<FF>(y, ep, RefCol<FF>{m.erefF + e, (size_t)p.ne, (size_t)p.ne * (kRefPerQp * p.nq + kRefPerElem)}, f, st);
+  const RefCol<FF> ref{m.erefF + e, (size_t)p.ne, (size_t)p.ne * (kRefPerQp * p.nq + kRefPerElem)};
+  const ElemGeom<FF> g = elem_geom<FF>(y, ep);
+  FF N[3], M[3];
+  elem_resultants<FF>(g, ep, ref, N, M, st, true, false, [](int, FF, FF, FF(*)[5]) {}, s, L);
+  if constexpr (L == 3) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      N[i] = lane3(N[i], base, 0) + lane3(N[i], base, 1) + lane3(N[i], base, 2);
+      M[i] = lane3(M[i], base, 0) + lane3(M[i], base, 1) + lane3(M[i], base, 2);
+    }
+  }
+  elem_out(g, N, M, f);
   set_status(m.status, st);
   const size_t ne = p.ne;
-  for (int a = 0; a < nen; a++) {
-    const FF c0 = tab[a];
-    FFAcc fx(c0, f[0]), fy(c0, f[1]), fz(c0, f[2]);
+  if constexpr (L == 1) {
+    for (int a = 0; a < nen; a++) {
+      const FF c0 = tab[a];
+      FFAcc fx(c0, f[0]), fy(c0, f[1]), fz(c0, f[2]);
 #pragma unroll
-    for (int r = 1; r < 5; r++) {
-      const FF c = tab[r * 16 + a];
-      fx.add(c, f[3 * r]); fy.add(c, f[3 * r + 1]); fz.add(c, f[3 * r + 2]);
+      for (int r = 1; r < 5; r++) {
+        const FF c = tab[r * 16 + a];
+        fx.add(c, f[3 * r]); fy.add(c, f[3 * r + 1]); fz.add(c, f[3 * r + 2]);
+      }
+      m.fb[(3 * a) * ne + e] = ff_to_double_bits(fx.get());
+      m.fb[(3 * a + 1) * ne + e] = ff_to_double_bits(fy.get());
+      m.fb[(3 * a + 2) * ne + e] = ff_to_double_bits(fz.get());
     }
-    m.fb[(3 * a) * ne + e] = ff_to_double_bits(fx.get());
-    m.fb[(3 * a + 1) * ne + e] = ff_to_double_bits(fy.get());
-    m.fb[(3 * a + 2) * ne + e] = ff_to_double_bits(fz.get());
+  } else {
+    FF fs[5];
+#pragma unroll
+    for (int r = 0; r < 5; r++) fs[r] = s == 0 ? f[3 * r] : s == 1 ? f[3 * r + 1] : f[3 * r + 2];
+    for (int a = 0; a < nen; a++) {
+      FFAcc v(tab[a], fs[0]);
+#pragma unroll
+      for (int r = 1; r < 5; r++) v.add(tab[r * 16 + a], fs[r]);
+      if (live) m.fb[(3 * a + s) * ne + e] = ff_to_double_bits(v.get());
+    }
   }
-  if (p.pressure != 0.0) elem_pressure_force(m, p, e);
+  if (live && s == 0 && p.pressure != 0.0) elem_pressure_force(m, p, e);
 }
 
 /* heads, then tails, of the float-float form of a */
@@ -1247,15 +1379,42 @@ int launch_positions(const DevMesh &m, const KParams &p, const double *x, void *
   return (int)cudaGetLastError();
 }
 
+/* Lanes an element of k_elem_residual.  Its time is a warp's FP64 chain times
+   the warps each of the 608 FP64 units gets.  Three lanes up to two rounds of
+   ten elements a unit: 1,536 triangles 64 -> 33 us (130 -> 58 with gradients),
+   6,144 triangles 65 -> 49 (122 -> 90).  From there one lane's single round of
+   32 elements a unit is the shorter: 13,774 triangles 65 us against 90. */
+static int residual_lanes(int ne)
+{
+  constexpr int units = 4 * 152;
+  return ne <= 2 * kResElems<3> * units ? 3 : 1;
+}
+
 int launch_elem_residual(const DevMesh &m, const KParams &p, void *stream, bool tangent)
 {
-  k_elem_residual<<<blocks_for(p.ne, 128), 128, 0, (cudaStream_t)stream>>>(m, p, tangent);
+  if (residual_lanes(p.ne) == 3)
+    k_elem_residual<3><<<blocks_for(p.ne, kResElems<3> * (kResBlock / 32)), kResBlock, 0, (cudaStream_t)stream>>>(m, p, tangent);
+  else
+    k_elem_residual<1><<<blocks_for(p.ne, kResBlock), kResBlock, 0, (cudaStream_t)stream>>>(m, p, tangent);
   return (int)cudaGetLastError();
+}
+
+/* The same of k_elem_residual_ff, three CTAs an SM: a wave of 18,240 elements
+   takes 31 to 35 us with three lanes (1,536 and 13,774 triangles), a wave of
+   58,368 takes 53 to 56 with one (to 38,400 triangles). */
+static int residual_ff_lanes(int ne)
+{
+  constexpr int warps = 3 * 152 * (kResBlock / 32);
+  const int w3 = (ne - 1) / (kResElems<3> * warps) + 1, w1 = (ne - 1) / (kResElems<1> * warps) + 1;
+  return 5 * w3 < 8 * w1 ? 3 : 1;
 }
 
 int launch_elem_residual_ff(const DevMesh &m, const KParams &p, void *stream)
 {
-  k_elem_residual_ff<<<blocks_for(p.ne, 128), 128, 0, (cudaStream_t)stream>>>(m, p);
+  if (residual_ff_lanes(p.ne) == 3)
+    k_elem_residual_ff<3><<<blocks_for(p.ne, kResElems<3> * (kResBlock / 32)), kResBlock, 0, (cudaStream_t)stream>>>(m, p);
+  else
+    k_elem_residual_ff<1><<<blocks_for(p.ne, kResBlock), kResBlock, 0, (cudaStream_t)stream>>>(m, p);
   return (int)cudaGetLastError();
 }
 
