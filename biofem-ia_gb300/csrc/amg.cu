@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "amg.h"
+#include "arena.h"
 
 namespace biofem {
 namespace {
@@ -725,7 +726,7 @@ struct AmgHier {
   float *A0f = nullptr;      /* FP32 copy of an FP64 tangent */
   float *part = nullptr;
   unsigned *ticket = nullptr;
-  std::vector<void *> allocs;
+  Arena mem;
   long long bytes = 0;
   cudaStream_t st = nullptr;
   cudaGraph_t num_graph = nullptr;      /* numeric setup, captured for one tangent buffer */
@@ -740,9 +741,8 @@ int dalloc_(AmgHier *h, T **p, size_t count)
 {
   *p = nullptr;
   if (count == 0) count = 1;
-  cudaError_t e = cudaMallocAsync((void **)p, count * sizeof(T), h->st);
+  cudaError_t e = h->mem.get((void **)p, count * sizeof(T), h->st);
   if (e != cudaSuccess) return (int)e;
-  h->allocs.push_back(*p);
   h->bytes += (long long)(count * sizeof(T));
   return 0;
 }
@@ -898,7 +898,7 @@ void amg_destroy(AmgHier *h)
   cudaStreamSynchronize(h->st);
   if (h->num_exec) cudaGraphExecDestroy(h->num_exec);
   if (h->num_graph) cudaGraphDestroy(h->num_graph);
-  for (void *p : h->allocs) cudaFreeAsync(p, h->st);
+  h->mem.release(h->st);
   cudaStreamSynchronize(h->st);
   delete h;
 }

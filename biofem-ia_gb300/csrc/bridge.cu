@@ -20,6 +20,7 @@
 
 #include "amg.h"
 #include "ff.cuh"
+#include "arena.h"
 #include "biofem_host.h"
 
 namespace biofem {
@@ -159,7 +160,7 @@ struct BiofemGpuMesh_ {
   long long nnzb = 0, ncontrib = 0;
   int n_irregular = 0, maxblk = 1;
   size_t bytes = 0;
-  std::vector<void *> allocs;
+  Arena mem;
   DevMesh dm{};
   double *d_x = nullptr, *d_R = nullptr;   /* staging for host-array calls */
   void *d_K = nullptr;                      /* K values: double (FP64) or float (FP32-bulk) */
@@ -205,9 +206,8 @@ template <class T>
 static int dalloc(BiofemGpuMesh *m, T **p, size_t n)
 {
   void *q = nullptr;
-  cudaError_t e = cudaMallocAsync(&q, std::max<size_t>(n, 1) * sizeof(T), m->st);
+  cudaError_t e = m->mem.get(&q, std::max<size_t>(n, 1) * sizeof(T), m->st);
   if (e != cudaSuccess) return fail(55, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-  m->allocs.push_back(q);
   m->bytes += std::max<size_t>(n, 1) * sizeof(T);
   *p = reinterpret_cast<T *>(q);
   return 0;
@@ -228,8 +228,7 @@ static void free_mesh(BiofemGpuMesh *m)
   if (m->solver) solver_destroy(m->solver);
   if (m->amg) amg_destroy(m->amg);
   for (int i = 0; i <= kMaxTimed; i++) if (m->timer.ev[i]) cudaEventDestroy(m->timer.ev[i]);
-  for (void *p : m->allocs) cudaFreeAsync(p, m->st);
-  m->allocs.clear();
+  m->mem.release(m->st);
   if (m->st) cudaStreamSynchronize(m->st);
   if (m->side) { cudaStreamSynchronize(m->side); cudaStreamDestroy(m->side); }
   if (m->ev_fork) cudaEventDestroy(m->ev_fork);

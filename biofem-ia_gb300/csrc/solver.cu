@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "amg.h"
+#include "arena.h"
 #include "biofem_host.h"
 #include "ff.cuh"
 
@@ -484,6 +485,7 @@ struct SolverWork {
   const void *g_K = nullptr;
   const void *g_pc = nullptr;   /* preconditioner the graph was captured with (null: block-Jacobi) */
   cudaStream_t st = nullptr;   /* allocation stream */
+  Arena mem;
   long long bytes = 0;         /* device memory allocated above */
 };
 
@@ -658,7 +660,7 @@ SolverWork *solver_create(int n, int nb, int m, void *stream, int *rc)
   cudaError_t e = cudaSuccess;
   const size_t dn = sizeof(double) * (size_t)n;
   auto A = [&](void **p, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMallocAsync(p, bytes, w->st);
+    if (e == cudaSuccess) e = w->mem.get(p, bytes, w->st);
     if (e == cudaSuccess) w->bytes += (long long)bytes;
   };
   A((void **)&w->V, dn * (size_t)(m + 1));
@@ -691,9 +693,7 @@ void solver_destroy(SolverWork *w)
   if (!w) return;
   cudaStream_t st = w->st;
   cudaStreamSynchronize(st);
-  void *ptrs[] = {w->V, w->Z, w->w, w->dx, w->xt, w->Rt, w->xh, w->dinv, w->part, w->h1, w->h2, w->H,
-                  w->cs, w->sn, w->g, w->y, w->gs, w->ticket};
-  for (void *p : ptrs) if (p) cudaFreeAsync(p, st);
+  w->mem.release(st);
   cudaStreamSynchronize(st);
   if (w->ev) cudaEventDestroy(w->ev);
   if (w->evb) cudaEventDestroy(w->evb);
