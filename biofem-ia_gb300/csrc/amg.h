@@ -33,10 +33,10 @@ struct AmgLevelHost {
   std::vector<int> agg;                      /* node -> aggregate, -1 when excluded */
   std::vector<float> Q;                      /* n * bs * 6 tentative prolongator rows */
   std::vector<unsigned char> dead;           /* na * 6: coarse unknowns with no tentative column */
-  std::vector<int> prow, pcol, pblkrow;      /* P pattern (fine row -> aggregates) and block -> row */
+  std::vector<int> prow, pcol;               /* P pattern (fine row -> aggregates) */
   std::vector<int> rrow, rcol, rmap;         /* P^T pattern: aggregate -> fine rows, and the P block of each */
-  std::vector<int> trow, tcol, tblkrow;      /* T = A P pattern */
-  std::vector<int> crow, ccol, cblkrow;      /* next level's operator pattern */
+  std::vector<int> trow, tcol;               /* T = A P pattern */
+  std::vector<int> crow, ccol;               /* next level's operator pattern */
 };
 
 /* Build the symbolic hierarchy.  rowptr/colind: the nt-row block pattern of
@@ -57,9 +57,18 @@ void amg_destroy(AmgHier *h);
 /* Numeric setup from the current tangent values (FP32 blocks, or FP64 blocks
    converted into a copy when the hierarchy was created with k_is_f32 false). */
 int amg_numeric(AmgHier *h, const void *K, bool k_is_f32, cudaStream_t st);
-/* z = M^-1 v for FP64 vectors of 3*nt entries; kernels skip their work while
-   *done is nonzero (done may be null). */
-void amg_apply(AmgHier *h, const double *v, double *z, const int *done, cudaStream_t st);
+/* Where the V-cycle starts: the caller writes b = v (in FP32), r = D^-1 b and
+   d = r *theta_inv of every node (the Krylov update does so as it forms v);
+   amg_apply then leaves M^-1 v in x.  b and r hold 3 FP32 values a node, d and
+   x four, the last unused.  The kernels skip their work while *done is nonzero
+   (done may be null). */
+struct AmgStart {
+  float *b, *r, *d;
+  const float *Dinv, *theta_inv;      /* 3x3 inverse of each diagonal block, a device scalar */
+  const float *x;
+};
+AmgStart amg_start(const AmgHier *h);
+void amg_apply(AmgHier *h, const int *done, cudaStream_t st);
 int amg_levels(const AmgHier *h);
 long long amg_device_bytes(const AmgHier *h);
 

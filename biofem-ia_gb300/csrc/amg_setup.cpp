@@ -115,8 +115,7 @@ void tentative(int n, int bs, int na, const std::vector<int> &agg, const std::ve
 /* Row-wise union of column sets: out row i = sorted union over the sets
    named by src(i); marker-array merge, linear in the total input size. */
 template <class RowSources>
-void union_pattern(int nrows, int ncols, RowSources src, std::vector<int> &ptr, std::vector<int> &col,
-                   std::vector<int> &blkrow)
+void union_pattern(int nrows, int ncols, RowSources src, std::vector<int> &ptr, std::vector<int> &col)
 {
   std::vector<int> mark(ncols, -1), buf;
   ptr.assign(nrows + 1, 0);
@@ -128,9 +127,6 @@ void union_pattern(int nrows, int ncols, RowSources src, std::vector<int> &ptr, 
     col.insert(col.end(), buf.begin(), buf.end());
     ptr[i + 1] = (int)col.size();
   }
-  blkrow.resize(col.size());
-  for (int i = 0; i < nrows; i++)
-    for (int k = ptr[i]; k < ptr[i + 1]; k++) blkrow[k] = i;
 }
 
 void diag_index(int n, const std::vector<int> &ptr, const std::vector<int> &col, std::vector<int> &diag)
@@ -208,7 +204,7 @@ int amg_symbolic(int nt, const std::vector<int> &rowptr, const std::vector<int> 
       if (L.agg[i] < 0) return;
       for (int k = L.rowptr[i]; k < L.rowptr[i + 1]; k++)
         if (L.agg[L.colind[k]] >= 0) add(L.agg[L.colind[k]]);
-    }, L.prow, L.pcol, L.pblkrow);
+    }, L.prow, L.pcol);
     /* P^T by counting sort on the aggregate */
     L.rrow.assign(na + 1, 0);
     for (int c : L.pcol) L.rrow[c + 1]++;
@@ -231,14 +227,14 @@ int amg_symbolic(int nt, const std::vector<int> &rowptr, const std::vector<int> 
         const int j = L.colind[k];
         for (int q = L.prow[j]; q < L.prow[j + 1]; q++) add(L.pcol[q]);
       }
-    }, L.trow, L.tcol, L.tblkrow);
+    }, L.trow, L.tcol);
     /* next operator P^T A P */
     union_pattern(na, na, [&](int a, auto add) {
       for (int r = L.rrow[a]; r < L.rrow[a + 1]; r++) {
         const int i = L.rcol[r];
         for (int q = L.trow[i]; q < L.trow[i + 1]; q++) add(L.tcol[q]);
       }
-    }, L.crow, L.ccol, L.cblkrow);
+    }, L.crow, L.ccol);
 
     AmgLevelHost C;
     C.n = na; C.bs = k6;
