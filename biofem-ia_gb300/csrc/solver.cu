@@ -962,6 +962,15 @@ int newton_device(const DevMesh &dm, const KParams &kp, bool f32, void *dK, doub
   s.rhist[0] = rn;
   const double target = std::max(o.rtol * s.r0, o.atol);
   double eta = 0.3, rn_prev = rn;
+  /* A Newton step that took the residual down by three orders left the tangent
+     nearly as it was, and the multigrid hierarchy with it: the next step keeps
+     it (a setup costs as much as six iterations: 64 x 48 310 us of 50 each,
+     98,304 triangles 1.7 ms of 270).  Iterations with the last step's hierarchy
+     against its own, by the residual's drop: 6e6 7 / 7, 2e4 15 / 15, 9e3 41 / 41, 100
+     42 / 42, but 283 22 / 16 and 62 above 110 / 42.  A solve that takes more than
+     twice the last setup's iterations and a cycle is done again on a new one. */
+  constexpr double kKeepHierarchy = 1e-3;
+  int its_setup = 0;
   for (int it = 0; it < o.max_newton; it++) {
     if (rn <= o.rtol * s.r0 || rn <= o.atol) { s.converged = 1; break; }
     double ksp_rtol = o.gmres_rtol;
@@ -976,11 +985,12 @@ int newton_device(const DevMesh &dm, const KParams &kp, bool f32, void *dK, doub
       eta = std::min(eta, 0.9);
       ksp_rtol = std::max(std::max(eta, o.gmres_rtol), std::min(0.9, 0.5 * target / rn));
     }
+    const bool keep = amg && it > 0 && rn <= kKeepHierarchy * rn_prev;
     rn_prev = rn;
     if ((rc = jacobian(ctx, x, dR, dK, (void *)st))) { err = "jacobian"; return rc; }
     s.jacobian_evals++;
     if (amg) {
-      if ((rc = amg_numeric(amg, dK, f32, st))) { err = "multigrid setup"; return rc; }
+      if (!keep && (rc = amg_numeric(amg, dK, f32, st))) { err = "multigrid setup"; return rc; }
     } else if (f32) {
       k_bj_setup<float><<<nblk(nb, 256), 256, 0, st>>>(nb, dm.rowptr, dm.colind, (const float *)dK, w.dinv, dm.status);
     } else {
@@ -990,7 +1000,14 @@ int newton_device(const DevMesh &dm, const KParams &kp, bool f32, void *dK, doub
     k_scale_copy<<<nblk(n, 256), 256, 0, st>>>(n, dR, -1.0, w.Rt);
     int its = 0;
     double relres = 0.0;
-    if ((rc = gm.solve(w.Rt, w.dx, ksp_rtol, o.gmres_max_it, &its, &relres))) { err = "gmres"; return rc; }
+    const int most = keep ? std::min(o.gmres_max_it, 2 * its_setup + w.m) : o.gmres_max_it;
+    if ((rc = gm.solve(w.Rt, w.dx, ksp_rtol, most, &its, &relres))) { err = "gmres"; return rc; }
+    if (keep && !(relres <= ksp_rtol)) {
+      s.gmres_its_total += its;
+      if ((rc = amg_numeric(amg, dK, f32, st))) { err = "multigrid setup"; return rc; }
+      if ((rc = gm.solve(w.Rt, w.dx, ksp_rtol, o.gmres_max_it, &its, &relres))) { err = "gmres"; return rc; }
+    }
+    if (!keep) its_setup = its;
     s.gmres_its_total += its;
     s.gmres_its_last = its;
     s.gmres_relres_last = relres;
