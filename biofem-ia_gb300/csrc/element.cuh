@@ -47,6 +47,11 @@ namespace biofem {
 /* ---------------- scalar types ---------------- */
 __host__ __device__ __forceinline__ double dsqrt(double a) { return sqrt(a); }
 __host__ __device__ __forceinline__ float dsqrt(float a) { return sqrtf(a); }
+/* 1 / sqrt(a): one instruction sequence for double instead of two */
+template <class R> __host__ __device__ __forceinline__ R drsqrt(R a) { return R(1) / dsqrt(a); }
+#ifdef __CUDA_ARCH__
+template <> __device__ __forceinline__ double drsqrt(double a) { return rsqrt(a); }
+#endif
 __host__ __device__ __forceinline__ double dabs(double a) { return fabs(a); }
 __host__ __device__ __forceinline__ float dabs(float a) { return fabsf(a); }
 
@@ -111,7 +116,7 @@ __host__ __device__ __forceinline__ V3<T> cross2(const V3<T> &a, const V3<T> &b,
      S^33 etc. = S.. + alpha/2 B..(c),  Q_xy(c) of v, w, e3.
    A form costs 3 + 1 multiply-adds against the 5 to 9 of evaluating it from
    s, t, A^T v, ..., at 25 more loads a point, and FP64 is the bound: residual
-   0.39 -> 0.31 ms on the 98,304-triangle sheet, 0.63 ms with gradients. */
+   0.39 -> 0.31 ms on the 98,304-triangle sheet (0.28 now, 0.58 with gradients). */
 enum {
   kRfS33 = 0, kRfS00, kRfS11, kRfS01,                       /* mu (G^-1 + c1 s s^T) */
   kRfB33 = 4, kRfB00 = 8, kRfB11 = 12, kRfB01 = 16,         /* Ci + A Ci H */
@@ -229,7 +234,8 @@ __host__ __device__ __forceinline__ void qp_stress(const R gm[5] /* 00 11 01 02 
                                                    int iters, R sv[3], int &status, R *c33_out = nullptr,
                                                    bool final_update = true, bool grad = false, R C[3][5] = nullptr)
 {
-  const R one = R(1), two = R(2), half = R(0.5), quarter = R(0.25), four = R(4);
+  const R one = R(1), two = R(2), half = R(0.5), four = R(4);
+  const R half_K = pow2(K, 0.5f), quarter_K = pow2(K, 0.25f), half_mu = pow2(mu, 0.5f);
   const R g00 = gm[0], g11 = gm[1], g01 = gm[2], g02 = gm[3], g12 = gm[4];
   /* ElemCGDefTens: C_inv in-plane = in-plane block of gm^-1 (g33 = n.n = 1), C33 = 1 */
   const R cof00 = mad(-g12, g12, g11);
@@ -266,8 +272,7 @@ __host__ __device__ __forceinline__ void qp_stress(const R gm[5] /* 00 11 01 02 
     const bool last = it == iters - 1;
     const R J2 = r(kRfRho) * ipre * C33;
     const R Je = dsqrt(J2);
-    const R alpha = mad(K, J2 - Je, -mu);
-    const R half_a = pow2(alpha, 0.5f);
+    const R half_a = mad(half_K, J2 - Je, -half_mu);
     if (last) {
       R Bi[3];
 #pragma unroll
@@ -321,16 +326,20 @@ __host__ __device__ __forceinline__ void qp_stress(const R gm[5] /* 00 11 01 02 
       if (!final_update) break;
     }
     /* S^33 and CC3333 */
-    const R beta = pow2(K * Je, 0.5f) * (pow2(Je, 2.f) - one);
     const R B33 = mad(r(kRfB33 + 3), c22, ip[0]);
     const R S33 = mad(half_a, B33, r(kRfS33));
     const R qvv = mad(r(kRfQvv + 3), c22, ip[1]), qww = mad(r(kRfQww + 3), c22, ip[2]);
     const R qee = mad(r(kRfQee + 3), c22, ip[3]), qvw = mad(r(kRfQvw + 3), c22, ip[4]);
     const R qve = mad(r(kRfQve + 3), c22, ip[5]), qwe = mad(r(kRfQwe + 3), c22, ip[6]);
-    /* 4 CC3333 = Qvv (2 (beta - alpha) Qvv + 4 beta Qwe) + Qwe (2 beta - alpha) Qwe - alpha (4 Qvw Qve + Qww Qee) */
-    const R twob = pow2(beta, 2.f);
-    const R CC = pow2(sop(qvv, sop(twob - pow2(alpha, 2.f), qvv, pow2(twob, 2.f), qwe), qwe * (twob - alpha), qwe,
-                          -alpha, sop(pow2(qvw, 4.f), qve, qww, qee)), 0.25f);
+    /* 4 CC3333 = Qvv (2 (beta - alpha) Qvv + 4 beta Qwe) + Qwe (2 beta - alpha) Qwe - alpha (4 Qvw Qve + Qww Qee),
+       with alpha = 2 half_a, beta = 2 b and the constants holding 2 Qvw and Qww / 2:
+       CC3333 = b (Qvv + Qwe)^2 - half_a (Qvv^2 + Qwe^2 / 2 + Qvw Qve + Qww Qee) */
+    const R b = half_K * sop(Je, Je, -half, Je);
+    const R sum = qvv + qwe, sum2 = sum * sum;
+    Acc<R> quad(qvv, qvv);
+    quad.add(pow2(qwe, 0.5f), qwe); quad.add(qvw, qve); quad.add(qww, qee);
+    const R Mq = quad.get();
+    const R CC = sop(b, sum2, -half_a, Mq);
     /* ModElemC33 (active_strain.c:1654-1707) */
     if (!(dabs(CC) > R(1e-14))) { status |= 1; return; }
     const R iCC = one / CC;
@@ -354,13 +363,9 @@ __host__ __device__ __forceinline__ void qp_stress(const R gm[5] /* 00 11 01 02 
          d ln ipre + dC33/C33), B33 (wB) and the quadratic forms (p..) */
       const R e = -(damp * iCC);
       const R kj = K * (two * Je - one);
-      const R sum = qvv + qwe;
-      const R CCa = -(quarter * (two * qvv * qvv + four * qvw * qve + qwe * qwe + qww * qee));
-      const R CCb = half * sum * sum;
-      const R wJ = e * (half * kj * B33 + dC0 * (CCa * kj + CCb * ((half * K) * (four * Je - one)))) * (half * Je);
-      const R wQ = e * dC0, wa = wQ * alpha, wb = wQ * beta;
-      const R w[7] = {e * half_a, (wb - wa) * qvv + wb * qwe, -(quarter * wa * qee), -(quarter * wa * qww),
-                      -(wa * qve), -(wa * qvw), wb * qvv + (wb - half * wa) * qwe};
+      const R wJ = e * (half * kj * (B33 - dC0 * Mq) + dC0 * sum2 * (quarter_K * (four * Je - one))) * (half * Je);
+      const R wQ = e * dC0, wh = wQ * half_a, wb = two * wQ * b * sum;
+      const R w[7] = {e * half_a, wb - two * wh * qvv, -(wh * qee), -(wh * qww), -(wh * qve), -(wh * qvw), wb - wh * qwe};
       R d[4];
 #pragma unroll
       for (int m = 0; m < 4; m++) {
@@ -406,8 +411,7 @@ __host__ __device__ __forceinline__ ElemGeom<T> elem_geom(const T y[15], const E
   g.a1 = {y[0], y[1], y[2]}; g.a2 = {y[3], y[4], y[5]};
   g.Aaa = {y[6], y[7], y[8]}; g.Abb = {y[9], y[10], y[11]}; g.Aab = {y[12], y[13], y[14]};
   const V3<T> cr = cross(g.a1, g.a2);
-  const T cn = dsqrt(dot(cr, cr));
-  const T icn = one / cn;
+  const T icn = drsqrt(dot(cr, cr));
   g.n = scl(icn, cr);
   g.gc1 = scl(icn, cross(g.a2, g.n));       /* a1.(a2 x n) = a2.(n x a1) = |a1 x a2| */
   g.gc2 = scl(icn, cross(g.n, g.a1));

@@ -207,13 +207,13 @@ __global__ void k_ref_prep(DevMesh m, KParams p, const double *__restrict__ fib,
     aT(v, av); aT(w, aw); aT(e3, ae);
     /* the stress's forms in (c00, c11, c01, c22): S^ij = mu (G^ij + c1 s_i s_j)
        + alpha/2 (Ci + A Ci H)^ij with A = I - gam s t^T, H = I + gam' t s^T,
-       and Q_xy = (A^T x)^T Ci (A^T y) */
+       and Q_xy = (A^T x)^T Ci (A^T y); 2 Q_vw and Q_ww / 2, as CC3333 takes them */
     double *o = eref + (size_t)kRefPerQp * q * ne + e;
     auto form = [&](int k, double f00, double f11, double f01, double f22) {
       o[(size_t)k * ne] = f00; o[(size_t)(k + 1) * ne] = f11; o[(size_t)(k + 2) * ne] = f01; o[(size_t)(k + 3) * ne] = f22;
     };
-    auto quad = [&](int k, const double x[3], const double y[3]) {
-      form(k, x[0] * y[0], x[1] * y[1], x[0] * y[1] + x[1] * y[0], x[2] * y[2]);
+    auto quad = [&](int k, const double x[3], const double y[3], double sc = 1.0) {
+      form(k, sc * (x[0] * y[0]), sc * (x[1] * y[1]), sc * (x[0] * y[1] + x[1] * y[0]), sc * (x[2] * y[2]));
     };
     const double gg = gam * gamp, dg = gamp - gam;
     const double t00 = t[0] * t[0], t11 = t[1] * t[1], t01 = 2.0 * t[0] * t[1], t22 = t[2] * t[2];
@@ -227,8 +227,8 @@ __global__ void k_ref_prep(DevMesh m, KParams p, const double *__restrict__ fib,
     form(kRfB11, -g11 * t00, 2.0 + dg * s[1] * t[1] - g11 * t11, dg * s[1] * t[0] - g11 * t01, -g11 * t22);
     form(kRfB01, gamp * s[1] * t[0] - g01 * t00, -gam * s[0] * t[1] - g01 * t11,
          2.0 + gamp * s[1] * t[1] - gam * s[0] * t[0] - g01 * t01, -g01 * t22);
-    quad(kRfQvv, av, av); quad(kRfQww, aw, aw); quad(kRfQee, ae, ae);
-    quad(kRfQvw, av, aw); quad(kRfQve, av, ae); quad(kRfQwe, aw, ae);
+    quad(kRfQvv, av, av); quad(kRfQww, aw, aw, 0.5); quad(kRfQee, ae, ae);
+    quad(kRfQvw, av, aw, 2.0); quad(kRfQve, av, ae); quad(kRfQwe, aw, ae);
     o[(size_t)kRfRho * ne] = rho;
   }
   eref[(size_t)kRefPerQp * p.nq * ne + e] = 0.5 * (2.0 * p.hhalf) * dA0;   /* pref0 */
@@ -281,8 +281,8 @@ __device__ __forceinline__ void store_pressure_vectors(const R av[3], const R bv
 }
 
 /* L = 1: one thread per element.  For the R + K call (tan) it also evaluates the
-   stress gradients (about 300 FP64 operations a thickness point beside the
-   400 of the stress itself), keeps them in cq between the thickness loop and
+   stress gradients (about 280 FP64 operations a thickness point beside the
+   370 of the stress itself), keeps them in cq between the thickness loop and
    the moments (its own column: 15 values a point would not fit in registers
    beside the stress), and stores the kTanCoefs tangent coefficients
    k_elem_tangent reads.  One kernel serves both calls, so that R is bit for
@@ -293,8 +293,8 @@ __device__ __forceinline__ void store_pressure_vectors(const R av[3], const R bv
    y, takes thickness points s, s + 3, .., forms the tangent coefficients of
    the two resultants of stress s (N11 and M11, ..) from their moments alone, and
    scatters component s of the force; the geometry in between is formed by all
-   three.  A chain of 730 FP64 operations (1,280 with gradients) in place of
-   1,850 (3,820), at 64 cycles each. */
+   three.  A chain of some 700 FP64 operations (1,200 with gradients) in place of
+   1,760 (3,560), at 64 cycles each. */
 template <int L> constexpr int kResElems = 32 / L;      /* elements a warp */
 constexpr int kResBlock = 128;
 
@@ -340,11 +340,12 @@ __global__ void __launch_bounds__(kResBlock) k_elem_residual(DevMesh m, KParams 
   const size_t ne = p.ne;
   const ElemGeom<double> g = elem_geom<double>(y, ep);
   double N[3], M[3];
-  elem_resultants<double>(g, ep, RefCol<double>{m.eref + e, ne}, N, M, st, true, tan, [&](int q, double w, double, double C[3][5]) {
+  const double pref0 = m.eref[(size_t)kRefPerQp * ep.nq * ne + e];
+  elem_resultants<double>(g, ep, RefCol<double>{m.eref + e, ne}, N, M, st, true, tan, [&](int q, double, double, double C[3][5]) {
     double *cq = m.cq + e;
     if (live)
       for (int i = 0; i < 3; i++)
-        for (int k = 0; k < 5; k++) cq[(size_t)(15 * q + 5 * i + k) * ne] = w * C[i][k];
+        for (int k = 0; k < 5; k++) cq[(size_t)(15 * q + 5 * i + k) * ne] = C[i][k];
   }, s, L);
   if constexpr (L == 3) {
 #pragma unroll
@@ -389,22 +390,22 @@ __global__ void __launch_bounds__(kResBlock) k_elem_residual(DevMesh m, KParams 
       double C[3][5];
       for (int i = 0; i < 3; i++)
         for (int k = 0; k < 5; k++) C[i][k] = m.cq[(size_t)(15 * q + 5 * i + k) * ne + e];
-      mo.add(1.0, ep.hhalf * ep.theta[q], C);
+      mo.add(pref0 * ep.w[q], ep.hhalf * ep.theta[q], C);
     }
     tangent_coefs<double>(g, N, M, mo, ep.tnormal, [&](int k, double v) { tc[(size_t)k * ne] = v; });
   } else {
     __syncwarp();                                  /* the other lanes' gradients */
     double T[4][3] = {}, U[2][2] = {};             /* TanMoments of stress s */
     for (int q = 0; q < ep.nq; q++) {
-      const double th = ep.hhalf * ep.theta[q], th2 = th * th, th3 = th2 * th;
+      const double th = ep.hhalf * ep.theta[q], w0 = pref0 * ep.w[q], w1 = w0 * th, w2 = w1 * th, w3 = w2 * th;
       const double *C = m.cq + (size_t)(15 * q + 5 * s) * ne + e;
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const double v = C[(size_t)c * ne];
-        T[0][c] += v; T[1][c] += th * v; T[2][c] += th2 * v; T[3][c] += th3 * v;
+        T[0][c] += w0 * v; T[1][c] += w1 * v; T[2][c] += w2 * v; T[3][c] += w3 * v;
       }
 #pragma unroll
-      for (int c = 0; c < 2; c++) { const double v = C[(size_t)(3 + c) * ne]; U[0][c] += th * v; U[1][c] += th2 * v; }
+      for (int c = 0; c < 2; c++) { const double v = C[(size_t)(3 + c) * ne]; U[0][c] += w1 * v; U[1][c] += w2 * v; }
     }
     const TanShape<double> sh(g, ep.tnormal);
     auto put = [&](int k, double v) { if (live) tc[(size_t)k * ne] = v; };
@@ -553,7 +554,7 @@ __global__ void k_to_ff(const double *__restrict__ a, float *__restrict__ b, lon
    block of columns of D along the s-th of a1, a2, Aaa, Abb, Aab from the
    element's coefficients (tangent_block).  FP64-pipe bound: 245 FP64
    instructions a lane, 0.27 ms on the 98,304-triangle sheet (with the
-   residual kernel's 0.32 ms of gradients and coefficients: 0.59 ms; the
+   residual kernel's 0.30 ms of gradients and coefficients: 0.57 ms; the
    16-lane forward-mode form took 1.99 ms).  D leaves in the row assembly's fixed-point form
    (fx.cuh): per Cartesian pair (i, j) the largest exponent over the element's
    25 entries, then every entry as two 32-bit words; an element with an
@@ -1390,9 +1391,10 @@ int launch_positions(const DevMesh &m, const KParams &p, const double *x, void *
 
 /* Lanes an element of k_elem_residual.  Its time is a warp's FP64 chain times
    the warps each of the 608 FP64 units gets.  Three lanes up to two rounds of
-   ten elements a unit: 1,536 triangles 64 -> 33 us (130 -> 58 with gradients),
-   6,144 triangles 65 -> 49 (122 -> 90).  From there one lane's single round of
-   32 elements a unit is the shorter: 13,774 triangles 65 us against 90. */
+   ten elements a unit: 1,536 triangles 62 -> 33 us (123 -> 55 with gradients),
+   6,144 triangles 62 -> 47 (115 -> 86), 12,160 triangles 63 -> 49 (115 -> 87).
+   From there one lane's single round of 32 elements a unit is the shorter:
+   13,774 triangles 64 us against 85 (115 against 131). */
 static int residual_lanes(int ne)
 {
   constexpr int units = 4 * 152;
@@ -1410,7 +1412,7 @@ int launch_elem_residual(const DevMesh &m, const KParams &p, void *stream, bool 
 
 /* The same of k_elem_residual_ff, three CTAs an SM: a wave of 18,240 elements
    takes 31 to 35 us with three lanes (1,536 and 13,774 triangles), a wave of
-   58,368 takes 53 to 56 with one (to 38,400 triangles). */
+   58,368 takes 52 to 58 with one (to 38,400 triangles). */
 static int residual_ff_lanes(int ne)
 {
   constexpr int warps = 3 * 152 * (kResBlock / 32);
