@@ -38,12 +38,12 @@ for _p in (ROOT, ROOT / "biofem-ia_gb300"):
 METRIC = "K+R assembly elems/s & %HBM; served load-steps/s, p50/p99; FP32 vs FP64"
 # dram__bytes_read.sum + dram__bytes_write.sum per launch on the 256x192
 # workload, from one ncu capture of each kernel (profiles/, bytes)
-DRAM_BYTES_C2 = {"elem_residual": 60.582e6 + 193.670e6, "elem_tangent": 241.039e6 + 160.028e6,
-                 "row_assemble": 289.613e6 + 106.150e6, "elem_residual_ff": 59.955e6 + 2.915e6,
-                 "elem_tangent_fp32": 36.505e6 + 33.795e6, "row_assemble_fp32": 195.243e6 + 48.489e6}
+DRAM_BYTES_C2 = {"elem_residual": 123.134e6 + 147.731e6, "elem_tangent": 116.889e6 + 131.661e6,
+                 "row_assemble": 288.873e6 + 107.673e6, "elem_residual_ff": 117.351e6 + 9.790e6,
+                 "elem_tangent_fp32": 69.859e6 + 50.297e6, "row_assemble_fp32": 189.690e6 + 46.157e6}
 # sm__pipe_fp64_cycles_active (fraction of peak sustained active) per kernel
 # in the same captures
-FP64_PIPE_ACTIVE_C2 = {"elem_residual": 0.884, "elem_tangent": 0.893, "row_assemble": 0.937}
+FP64_PIPE_ACTIVE_C2 = {"elem_residual": 0.893, "elem_tangent": 0.890, "row_assemble": 0.326}
 # FP64 FMA throughput of this GB300, measured by the DFMA loop of the FP64 pipe
 # probe (biofem-ia_gb300/csrc/probe_fp64.cu): TFLOP/s
 FP64_DFMA_TFLOPS = 1.057
@@ -730,8 +730,8 @@ def run_ours(args):
                      "note": "of measured HBM copy bandwidth; achieved = canonical algorithmic bytes of one R+K "
                              "evaluation (patch ids, x and X, fibre and activation, R, K values once) / the dominant "
                              "kernel's live launch time (CUDA events on the launch stream); traffic = dram read + "
-                             "write of one launch of that kernel on C2 from an ncu capture; the step is FP64-pipe "
-                             "bound, see compute_roofline"},
+                             "write of one launch of that kernel on C2 from an ncu capture; the element kernels are "
+                             "FP64-pipe bound, the row assembly integer-multiply bound, see compute_roofline"},
         "compute_roofline": {"kernel": "whole R+K step", "bound": "fp64", "step_ms": ms,
                              "canonical_flops_per_step": f_alg,
                              "achieved_tflops_canonical": f_alg / (ms * 1e-3) / 1e12,
@@ -740,9 +740,9 @@ def run_ours(args):
                              "peak_source": "measured DFMA loop on this GB300 (FP64 pipe probe)",
                              "fp64_pipe_active_frac": FP64_PIPE_ACTIVE_C2,
                              "note": "canonical F_alg (the B^T D B contraction at every thickness point) over the "
-                                     "whole step time; the contraction itself runs in k_row_assemble on the 15 "
-                                     "generalised coordinates (about 18.4 kflop per element, against 25.9 kflop "
-                                     "canonical at q = 3); fp64_pipe_active_frac is sm__pipe_fp64_cycles_active per "
+                                     "whole step time; the contraction itself runs in k_row_assemble_fx on the 15 "
+                                     "generalised coordinates, in exact integer arithmetic on the integer pipe, so "
+                                     "the fraction of the FP64 peak can exceed 1; fp64_pipe_active_frac is sm__pipe_fp64_cycles_active per "
                                      "kernel on C2 (ncu)"},
         "kernels_ms": dict(zip(KERNELS_FP64, kms)),
         "residual_only": {"ms_per_step": sum(r_ms) / len(r_ms), "elems_per_s": ne / (sum(r_ms) / len(r_ms) * 1e-3)},

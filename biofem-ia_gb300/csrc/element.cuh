@@ -709,17 +709,19 @@ __host__ __device__ __forceinline__ void tangent_block(int s, Load ld, R D[15][3
   }
 }
 
-/* ---------------- tangent contraction (row assembly) ---------------- */
+/* ---------------- tangent contraction ---------------- */
 /* The element stiffness is K_e = N^T D N with D = df/dy (15 x 15) and N the
-   5 x nen basis table acting on each Cartesian component.  The row assembly
-   forms it one block row a at a time:
+   5 x nen basis table acting on each Cartesian component; one block row a at a
+   time:
      w = (N[:,a] (x) I3)^T D          (3 x 15, w[15 i + k] = sum_r N[r][a] D[3r+i][k]),
      K_ab[i][j] = sum_s N[s][b] w[15 i + 3 s + j],
    plus, when a and b are corner slots of the triangle, the follower-pressure
    block: the cross-product matrix of sc v_b, v_b the corner's vector.
+   This is the plain form, which the host tests contract with; the row
+   assemblies of kernels.cu take the same sums in their own number formats.
    Both sums run over the five basis rows, so the operands are kept with that
-   index innermost, padded to 8, for vector loads: the table as
-   tabT[8 b + s] = N[s][b] and w as wT[8 (3 i + j) + s] = w[15 i + 3 s + j]. */
+   index innermost, padded to 8: the table as tabT[8 b + s] = N[s][b] and w as
+   wT[8 (3 i + j) + s] = w[15 i + 3 s + j]. */
 constexpr int kRowPad = 8;
 
 /* five consecutive values from a 16-byte aligned address */

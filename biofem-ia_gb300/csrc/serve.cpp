@@ -128,9 +128,9 @@ int BiofemServeEstimateBytes(int32_t n_v, int32_t n_elmt, int32_t n_ghosts, int3
   if (!bytes) return 85;
   const int64_t nt = (int64_t)n_v + n_ghosts;
   const int m = gmres_restart > 0 ? gmres_restart : 30;
-  /* per element: tangent block df/dy (240 values), forces, thickness-point
-     metrics, primal geometry, resultants and C33 values (FP64; 3 points,
-     3 sub-iterations), reference constants, row-assembly lists and records
+  /* per element: tangent block df/dy (244 values), forces, stress gradients
+     and tangent coefficients (FP64; 3 points), reference constants (an upper
+     bound with room for more points), row-assembly lists and records
      (80 bytes for each of the element's ~12 row contributions); per node:
      tangent row (~37 blocks), pattern, flexible-GMRES bases V and Z,
      multigrid hierarchy (FP32 copy of the tangent for FP64 handles, P, A P,
