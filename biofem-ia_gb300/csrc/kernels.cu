@@ -5,7 +5,7 @@
  *                    x_g = x_nv2 + x_nv1 - x_nv3 (GlobalGhost, bending.c:1763-1814)
  *   k_ref_prep       one-time reference geometry per element (geom0 + the
  *                    reference half of ElemUpdateG and ElemActDefGrad)
- *   k_elem_residual  one thread per element: geometry, closed-form stress,
+ *   k_elem_residual  one thread, or three lanes, per element: geometry, stress,
  *                    element forces Fb (ElemUpdFint) and the follower-pressure
  *                    corner force (SurfaceNormalPressure, external.c:589-624)
  *                    (and, for the FP64 tangent, the stress gradients and the
