@@ -104,7 +104,7 @@ struct DevMesh {
   int *dptr, *didx;          /* per node, the real triangles with that corner, in triangle order */
   double *xn, *xnm1, *xd, *xdd;   /* 3*nt dynamic state (previous positions, velocity, acceleration) */
   double *dyn_diag;          /* nt: d Fdyn / d x on the diagonal of each free row */
-  unsigned short *dexp;      /* FP64 handles: 16*ne exponent fields of D, one per Cartesian pair (fx.cuh) */
+  unsigned *dexp;            /* FP64 handles: kFxExps*ne words of exponent fields of D, one per Cartesian pair (fx.cuh) */
   double *cq;                /* FP64 handles: 15 nq x ne stress gradients d S / d metric (k_elem_residual's own scratch) */
   double *tcoef;             /* FP64 handles: kTanCoefs x ne tangent coefficients, k_elem_residual -> k_elem_tangent */
   unsigned long long *fmax;  /* max |Fext| as ordered bits */

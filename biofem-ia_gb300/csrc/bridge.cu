@@ -589,7 +589,7 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
       }
     int *d_ntabFx = nullptr;
     unsigned char *d_rgrow = nullptr;
-    if ((rc = dupload(m, &d_ntabFx, tabsFx)) || (rc = dalloc(m, &d_rgrow, (size_t)nt)) || (rc = dalloc(m, &dm.dexp, 16 * (size_t)ne)) ||
+    if ((rc = dupload(m, &d_ntabFx, tabsFx)) || (rc = dalloc(m, &d_rgrow, (size_t)nt)) || (rc = dalloc(m, &dm.dexp, kFxExps * (size_t)ne)) ||
         (rc = dalloc(m, &dm.De, (size_t)kDeStride * ne)) || (rc = dalloc(m, &dK, 9 * (size_t)m->nnzb)) ||
         (rc = dalloc(m, &dm.cq, 15 * (size_t)kp.nq * ne)) || (rc = dalloc(m, &dm.tcoef, (size_t)kTanCoefs * ne))) {
       free_mesh(m);

@@ -558,7 +558,9 @@ __global__ void k_to_ff(const double *__restrict__ a, float *__restrict__ b, lon
    16-lane forward-mode form took 1.99 ms).  D leaves in the row assembly's fixed-point form
    (fx.cuh): per Cartesian pair (i, j) the largest exponent over the element's
    25 entries, then every entry as two 32-bit words; an element with an
-   infinity or NaN keeps its doubles and is marked kFxRaw. */
+   infinity or NaN, or with a pair near underflow, keeps its doubles and is
+   marked kFxRaw.  The pressure vectors' exponents go
+   beside D's (fx_pack), so that a load larger than D does not take D's digits. */
 constexpr int kTanElems = 6;         /* elements per warp */
 
 /* place of entry (k = 5 r + s, q = 3 i + j) of D in an FP64 element block, see the
@@ -579,34 +581,43 @@ __global__ void __launch_bounds__(128) k_elem_tangent(DevMesh m, KParams p)
   tangent_block<double>(s, [&](int k) { return __ldg(tc + (size_t)k * ne); }, D);
   const bool pres_live = p.pressure != 0.0 && !p.pres_dead;
   const double *pv = m.De + (size_t)kDeStride * ee + kDePres + 3 * min(s, 2);
-  /* exponent of each (i, j) over this lane's five rows, two to a register, then over the element's five lanes */
-  unsigned eb[5];
+  /* exponent of each (i, j) over this lane's five rows, then of the pressure vectors' components (one corner
+     read here), two to a register, then over the element's five lanes */
+  unsigned eb[6] = {0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll
-  for (int q = 0; q < 9; q++) {
+  for (int q = 0; q < 12; q++) {
     int h = 0;
+    if (q < 9) {
 #pragma unroll
-    for (int r = 0; r < 5; r++) h = max(h, __double2hiint(D[3 * r + q / 3][q % 3]) & 0x7fffffff);
-    /* the pressure block's entry (i, j) is component 3 - i - j of the three corner vectors, one of them read here */
-    const int i = q / 3, j = q % 3;
-    if (i != j && pres_live && s < 3) h = max(h, __double2hiint(pv[3 - i - j]) & 0x7fffffff);
+      for (int r = 0; r < 5; r++) h = max(h, __double2hiint(D[3 * r + q / 3][q % 3]) & 0x7fffffff);
+    } else if (pres_live && s < 3) {
+      h = __double2hiint(pv[q - 9]) & 0x7fffffff;
+    }
     h >>= 20;
-    eb[q / 2] = q % 2 ? eb[q / 2] | ((unsigned)h << 16) : (unsigned)h;
+    eb[q / 2] |= (unsigned)h << (q % 2 * 16);
   }
 #pragma unroll
   for (int k = 1; k < 5; k++) {
     const int src = lane < 5 * kTanElems ? 5 * g + (s + k) % 5 : lane;
 #pragma unroll
-    for (int q = 0; q < 5; q++) eb[q] = __vmaxu2(eb[q], __shfl_sync(0xffffffffu, eb[q], src));
+    for (int q = 0; q < 6; q++) eb[q] = __vmaxu2(eb[q], __shfl_sync(0xffffffffu, eb[q], src));
   }
+  auto field = [&](int q) { return (int)(q % 2 ? eb[q / 2] >> 16 : eb[q / 2] & 0xffffu); };
+  /* the pressure block's entry (i, j) is component 3 - i - j of the corner vectors */
+  auto load = [&](int q) { return q % 4 ? field(12 - q / 3 - q % 3) : 0; };
   bool raw = false;
+  int most = 0;
 #pragma unroll
-  for (int q = 0; q < 5; q++) raw |= (eb[q] & 0xffffu) == (unsigned)kFxRaw || (eb[q] >> 16) == (unsigned)kFxRaw;
+  for (int q = 0; q < 9; q++) {
+    raw |= field(q) == kFxRaw || load(q) == kFxRaw ||
+           (field(q) && (field(q) < kFxMinExp || load(q) > field(q) + kFxMaxExcess));
+    most = max(most, field(q));
+  }
   if (!live) return;
   if (s == 0) {
-    const unsigned bad = kFxRaw | (kFxRaw << 16);
-    uint4 *dst = reinterpret_cast<uint4 *>(m.dexp + 16 * (size_t)e);
-    dst[0] = raw ? make_uint4(bad, bad, bad, bad) : make_uint4(eb[0], eb[1], eb[2], eb[3]);
-    dst[1] = make_uint4(raw ? bad : eb[4], 0u, 0u, 0u);
+    unsigned *dst = m.dexp + kFxExps * (size_t)e;
+#pragma unroll
+    for (int q = 0; q < 9; q++) dst[q] = raw ? fx_pack(kFxRaw, 0, kFxRaw) : fx_pack(field(q), load(q), most);
   }
   double *De = m.De + (size_t)kDeStride * e;
 #pragma unroll
@@ -614,7 +625,7 @@ __global__ void __launch_bounds__(128) k_elem_tangent(DevMesh m, KParams p)
 #pragma unroll
     for (int q = 0; q < 9; q++) {
       const double d = D[3 * r + q / 3][q % 3];
-      const Fx v = fx_split(fx_from_double(d, (int)(q % 2 ? eb[q / 2] >> 16 : eb[q / 2] & 0xffffu)));
+      const Fx v = fx_split(fx_from_double(d, field(q)));
       const int2 w = raw ? make_int2(__double2loint(d), __double2hiint(d)) : make_int2(v.lo, v.hi);
       *reinterpret_cast<int2 *>(De + fx_place(5 * r + s, q)) = w;
     }
@@ -844,15 +855,20 @@ __device__ __forceinline__ int row_find(const int *cols, int nb, int node)
 __host__ __device__ __forceinline__ size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 /* FP64 row assembly in fixed point (fx.cuh); the follower-pressure vectors
-   are converted to the row's units and added with it.  A row with an element
-   whose D is not finite takes row_assemble_raw, plain FP64.
+   are converted to the row's units and added with it.
 
    Why integers: the FP64 form of this sum ran at 93 % of the FP64 pipe
-   (1.94 ms on the 98,304-triangle sheet, q = 3); K's error against a 64-bit
-   reference is measured no larger (see fx.cuh for the bound).  Now 0.49 ms,
+   (1.94 ms on the 98,304-triangle sheet, q = 3).  Now 0.49 ms,
    bound by the integer multiplies (IMAD.WIDE, four cycles a warp).  Fetching
    the next contributions' D early, as the FP32 form does, needs 126 registers
-   and halves the warps: 0.58 ms. */
+   and halves the warps: 0.58 ms.
+
+   A sum of integers has one unit, 2^-57.6 of the row's largest element of the
+   Cartesian pair, so a far smaller element would keep fewer bits than a
+   double.  A row takes integers only while none lies too far below (fx_pack);
+   the others (elements of very different size or stiffness side by side, a load
+   far above D), and rows with infinities, NaN or magnitudes near the ends of
+   the exponent range, are summed in double (row_assemble_wide). */
 struct FxRowBuf {
   long long *acc;     /* kRowWords maxblk */
   int *rec;           /* kRowCopies records */
@@ -899,42 +915,82 @@ __device__ __forceinline__ long long fx_entry_reg(const FxRegular &reg, const Fx
   return sum.value();
 }
 
-/* The row's sum in FP64, one contribution after another in element order:
-   for rows with an infinite or NaN element, or of magnitudes near the smallest
-   double (neither in a converging solve).  Lane q < 9 forms entry q. */
-__device__ __noinline__ void row_assemble_raw(const DevMesh &m, int c0, int c1, bool pres_live, double *acc,
-                                              int nb, int lane)
+/* The row's sum in double over the same lanes and copies, in units of
+   1 / reg.wide: an element's sums stay integers in its own units and are added
+   as doubles (fx_wide), so that elements of any size keep their digits; one
+   that holds doubles, or is near overflow, takes FP64 throughout. */
+__device__ __noinline__ void row_assemble_wide(const DevMesh &m, const FxRegular &reg, int c0, int c1, bool pres_live,
+                                               double *racc, int nb, int lane)
 {
-  for (int t = lane; t < 9 * nb; t += 32) acc[t] = 0.0;
-  __syncwarp();
-  if (lane < 9)
-    for (int c = c0; c < c1; c++) {
-      const int *rc = m.rrec + (size_t)kRowRec * c;
-      const int e = rc[0] & ((1 << 27) - 1), a = rc[0] >> 27, info = rc[1], cs = rc[2], nen = info & 0xff;
-      const double *tab = m.ntab + (info >> 8) * 80;
-      const double *De = m.De + (size_t)kDeStride * e;
-      const int eb = m.dexp[16 * (size_t)e + lane];
-      double w[5];
-      for (int s = 0; s < 5; s++) {
-        w[s] = 0.0;
-        for (int r = 0; r < 5; r++) {
-          const double d = De[fx_place(5 * r + s, lane)];
-          w[s] = fma(tab[16 * r + a], eb == kFxRaw ? d : fx_to_double(Fx{__double2loint(d), __double2hiint(d)}, eb), w[s]);
+  double *acc = racc + lane;
+  for (int t = 0; t < nb; t++) acc[kRowWords * t] = 0.0;
+  const int pc = lane / 9, q = lane - 9 * pc;
+  for (int cb = c0; cb < c1; cb += kRowCopies) {
+    const bool on = pc < min(kRowCopies, c1 - cb);
+    const int *rc = m.rrec + (size_t)kRowRec * (on ? cb + pc : cb);
+    const int e = rc[0] & ((1 << 27) - 1), a = rc[0] >> 27, info = rc[1];
+    const double *De = m.De + (size_t)kDeStride * e;
+    if (on) {
+      const int nen = info & 0xff, eb = fx_d_exp(m.dexp[kFxExps * (size_t)e + q]);
+      const bool f64 = eb > kFxMaxWide;
+      const int2 *tab = reinterpret_cast<const int2 *>(m.ntabFx) + (info >> 8) * 16 * kFxTab;
+      const double *tabd = m.ntab + (info >> 8) * 80;
+      Fx w[5];
+      double wd[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+      if (!f64) {
+        FxSum<62> sum[5];
+#pragma unroll
+        for (int k = 0; k < 25; k++) {
+          const int2 n = __ldg(tab + a * kFxTab + k / 5), d = __ldg(reinterpret_cast<const int2 *>(De + fx_place(k, q)));
+          sum[k % 5].add(Fx{n.x, n.y}, Fx{d.x, d.y});
         }
+#pragma unroll
+        for (int s = 0; s < 5; s++) w[s] = fx_split(sum[s].value());
+      } else {
+        for (int r = 0; r < 5; r++)
+#pragma unroll
+          for (int s = 0; s < 5; s++) {
+            const double d = De[fx_place(5 * r + s, q)];
+            wd[s] = fma(__ldg(tabd + 16 * r + a), eb == kFxRaw ? d : fx_to_double(Fx{__double2loint(d), __double2hiint(d)}, eb), wd[s]);
+          }
+#pragma unroll
+        for (int s = 0; s < 5; s++) wd[s] *= reg.wide;
       }
-      const int corner[3] = {cs & 31, (cs >> 5) & 31, (cs >> 10) & 31};
-      const bool acorner = pres_live && (a == corner[0] || a == corner[1] || a == corner[2]);
       for (int b = 0; b < nen; b++) {
         const unsigned sl = (unsigned)rc[4 + b];
-        const int np = (sl & kRowSlotGhost) && !(sl & kRowSlotDup) ? 3 : 1;
         double v = 0.0;
-        for (int s = 0; s < 5; s++) v = fma(tab[16 * s + b], w[s], v);
-        if (acorner)
-          for (int k = 0; k < 3; k++)
-            if (b == corner[k]) v += skew_entry(lane / 3, lane % 3, De + kDePres + 3 * k, 1.0);
-        for (int k = 0; k < np; k++) acc[9 * ((sl >> (10 * k)) & 1023u) + lane] += k == 2 ? -v : v;
+        if (!f64) {
+          FxSum<63> sum;
+#pragma unroll
+          for (int s = 0; s < 5; s++) {
+            const int2 n = __ldg(tab + b * kFxTab + s);
+            sum.add(Fx{n.x, n.y}, w[s]);
+          }
+          v = fx_wide(sum.value(), eb);
+        } else {
+#pragma unroll
+          for (int s = 0; s < 5; s++) v = fma(__ldg(tabd + 16 * s + b), wd[s], v);
+        }
+        acc[kRowWords * (int)(sl & 1023u)] += v;
+        if ((sl & kRowSlotGhost) && !(sl & kRowSlotDup)) {   /* a repeated real node has one target */
+          acc[kRowWords * (int)((sl >> 10) & 1023u)] += v;
+          acc[kRowWords * (int)((sl >> 20) & 1023u)] -= v;
+        }
       }
     }
+    if (!pres_live) continue;
+    __syncwarp();                                    /* the contributions' own adds are done */
+    const int cs = rc[2], s0 = cs & 31, s1 = (cs >> 5) & 31, s2 = (cs >> 10) & 31;
+    if (on && (a == s0 || a == s1 || a == s2)) {     /* lanes as in the integer form below */
+      const int k = q / 3, d = q - 3 * k;
+      const unsigned sl = (unsigned)rc[4 + (k == 0 ? s0 : k == 1 ? s1 : s2)];
+      const double v = De[kDePres + q] * reg.wide;
+      double *dst = acc - q + kRowWords * (int)(sl & 1023u);
+      dst[d == 0 ? 5 : d == 1 ? 6 : 1] -= v;
+      dst[d == 0 ? 7 : d == 1 ? 2 : 3] += v;
+    }
+    __syncwarp();
+  }
 }
 
 __global__ void __launch_bounds__(256, 3) k_row_assemble_fx(DevMesh m, KParams p, FxRegular reg, double *__restrict__ K,
@@ -960,20 +1016,25 @@ __global__ void __launch_bounds__(256, 3) k_row_assemble_fx(DevMesh m, KParams p
   const int pc = lane / 9, q = lane - 9 * pc;       /* contribution and entry; lanes 27..31 idle */
   int4 nrec = make_int4(0, 0, 0, 0);
   if (lane < (kRowRec / 4) * min(kRowCopies, c1 - c0)) nrec = __ldg(rrec4 + (size_t)(kRowRec / 4) * c0 + lane);
-  /* the row's exponent of entry q, over all contributions */
-  int eb = 0;
+  /* the row's exponent of entry q over all contributions, and the largest that each of them allows */
+  int eb = 0, most = kFxRaw;
   for (int c = c0 + pc; c < c1; c += kRowCopies)
-    if (pc < kRowCopies) eb = max(eb, (int)m.dexp[16 * (size_t)(__ldg(m.rrec + (size_t)kRowRec * c) & ((1 << 27) - 1)) + q]);
+    if (pc < kRowCopies) {
+      const unsigned x = m.dexp[kFxExps * (size_t)(__ldg(m.rrec + (size_t)kRowRec * c) & ((1 << 27) - 1)) + q];
+      eb = max(eb, fx_row_exp(x));
+      most = min(most, fx_most_exp(x));
+    }
   {
     const int l1 = lane >= 27 ? lane : (lane + 9) % 27, l2 = lane >= 27 ? lane : (lane + 18) % 27;
     const int x1 = __shfl_sync(0xffffffffu, eb, l1), x2 = __shfl_sync(0xffffffffu, eb, l2);
     eb = max(eb, max(x1, x2));
   }
-  const bool raw = __any_sync(0xffffffffu, (eb > 0 && eb < kFxMinExp) || eb > kFxMaxExp);
-  if (raw) {
-    row_assemble_raw(m, c0, c1, pres_live, reinterpret_cast<double *>(B.acc), nb, lane);
+  const int grow = m.rgrow[i];
+  const bool wide = __any_sync(0xffffffffu, (eb > 0 && eb < kFxMinExp) || eb > kFxMaxExp || eb + grow > most);
+  if (wide) {
+    row_assemble_wide(m, reg, c0, c1, pres_live, reinterpret_cast<double *>(B.acc), nb, lane);
   } else {
-    eb += m.rgrow[i];
+    eb += grow;
     if (lane < 9) { B.sc[lane] = ldexp(reg.unit, eb - 1022); B.eb[lane] = eb; }
     long long *acc = B.acc + lane;
     for (int t = 0; t < nb; t++) acc[kRowWords * t] = 0;
@@ -990,7 +1051,7 @@ __global__ void __launch_bounds__(256, 3) k_row_assemble_fx(DevMesh m, KParams p
       Fx w[5];
       if (on) {
         const int4 *D = reinterpret_cast<const int4 *>(m.De + (size_t)kDeStride * e) + q;
-        const int sh = eb - (int)m.dexp[16 * (size_t)e + q];
+        const int sh = eb - fx_d_exp(m.dexp[kFxExps * (size_t)e + q]);
         if ((info >> 8) == 0) {
           const int *nr = reg.n[a];
           const int n[5] = {nr[0], nr[1], nr[2], nr[3], nr[4]};
@@ -1066,8 +1127,8 @@ __global__ void __launch_bounds__(256, 3) k_row_assemble_fx(DevMesh m, KParams p
           const double v = m.De[(size_t)kDeStride * e + kDePres + q];
           const int qm = d == 0 ? 5 : d == 1 ? 6 : 1, qp = d == 0 ? 7 : d == 1 ? 2 : 3;
           long long *dst = acc - q + kRowWords * (int)(sl & 1023u);
-          dst[qm] -= fx_shift(fx_from_double(v * reg.den2, B.eb[qm] + kFxDenBits), 60 - kFxDenBits - kFxUnit);
-          dst[qp] += fx_shift(fx_from_double(v * reg.den2, B.eb[qp] + kFxDenBits), 60 - kFxDenBits - kFxUnit);
+          dst[qm] -= fx_load(v * reg.den2, B.eb[qm]);
+          dst[qp] += fx_load(v * reg.den2, B.eb[qp]);
         }
       }
       __syncwarp();   /* the records are rewritten by the next three */
@@ -1082,7 +1143,13 @@ __global__ void __launch_bounds__(256, 3) k_row_assemble_fx(DevMesh m, KParams p
   int blk = lane / 9, qq = lane - 9 * blk;
   for (int t = lane; t < 9 * nb; t += 32) {
     const long long *c = B.acc + kRowWords * blk + qq;
-    double v = raw ? reinterpret_cast<const double *>(B.acc)[t] : (double)(c[0] + c[9] + c[18]) * B.sc[qq];
+    double v;
+    if (wide) {
+      const double *f = reinterpret_cast<const double *>(c);
+      v = ((f[0] + f[9]) + f[18]) * reg.unwide;
+    } else {
+      v = (double)(c[0] + c[9] + c[18]) * B.sc[qq];
+    }
     if (blk == pd && qq % 4 == 0) v += dd;
     if (fmax > 1.0) v *= sc;
     Kr[colmajor ? t - qq + 3 * (qq % 3) + qq / 3 : t] = v;
@@ -1556,6 +1623,8 @@ bool regular_tables(const double *tab0, int den, RowTables &t)
     }
   t.x.den2 = (double)den * den;
   t.x.unit = ldexp(1.0 / t.x.den2, -kFxUnit);
+  t.x.wide = ldexp(t.x.den2, -kFxDenBits);
+  t.x.unwide = ldexp(1.0 / t.x.den2, kFxDenBits);
   return ok;
 }
 
