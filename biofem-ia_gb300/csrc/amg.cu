@@ -24,10 +24,14 @@ namespace {
 
 constexpr int kPowerIts = 12;
 /* The power iterations whose norm is taken (the next one's iterate is divided
-   by it): the last two give the estimate, the others keep the values in range
-   for eigenvalues up to 1e9.  A norm is a reduction over the whole launch, half
-   of a small level's time. */
+   by it): the last two give the estimate.  A norm is a reduction over the whole
+   launch, half of a small level's time.  The iterate before a norm is divided by
+   the power of two of its largest entry (an atomic a warp, 1 us a launch), so
+   that the sum of squares meets one factor of the eigenvalue, not four; the
+   iterates between hold three.  That serves to 1e12, more than a nearly singular
+   diagonal block gives (k_dinv takes 1e-12 of a block for zero). */
 constexpr bool power_norm(int it) { return it == 3 || it == 7 || it >= kPowerIts - 2; }
+constexpr bool power_largest(int it) { return !power_norm(it) && power_norm(it + 1); }
 constexpr int kPowerBlocks = 912;    /* 6 x 152 SMs; the norm's partial sums */
 
 inline int nblk(long long n, int bs) { return (int)((n + bs - 1) / bs); }
@@ -186,9 +190,11 @@ __global__ void k_to_f32(long long n, const double *__restrict__ a, float *__res
 /* inverse of each diagonal block by Gauss-Jordan with partial pivoting; a
    vanishing pivot leaves that unknown as identity */
 template <int BS>
-__global__ void k_dinv(int n, const int *__restrict__ diag, const float *__restrict__ A, float *__restrict__ Dinv)
+__global__ void k_dinv(int n, const int *__restrict__ diag, const float *__restrict__ A, float *__restrict__ Dinv,
+                       unsigned *__restrict__ largest)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kPowerIts) largest[i] = 0u;      /* the power iterations', which follow */
   if (i >= n) return;
   float a[BS][BS], v[BS][BS];
   const int k = diag[i];
@@ -238,9 +244,17 @@ __global__ void k_dinv(int n, const int *__restrict__ diag, const float *__restr
     for (int c = 0; c < BS; c++) o[r * BS + c] = v[r][c];
 }
 
-/* one power-iteration step on D^-1 A: y = D^-1 A x / s_prev (x = a fixed
-   pseudo-random vector on the first step), and ||y|| into norm_out via a
-   fixed-order last-block reduction */
+/* 1 / 2^floor(log2 v) of a positive float's bits; 1 for zero, infinity and NaN */
+__device__ __forceinline__ float inverse_power_of_two(unsigned v)
+{
+  const unsigned f = v >> 23;
+  return f == 0u || f == 255u ? 1.f : __uint_as_float((254u - min(f, 253u)) << 23);
+}
+
+/* one power-iteration step on D^-1 A: y = D^-1 A x over the last norm (s_prev), or
+   the power of two of the last step's largest entry (big_prev); x = a fixed
+   pseudo-random vector on the first step.  Then ||y|| into norm_out via a
+   fixed-order last-block reduction, or y's largest entry into big_out. */
 __device__ __forceinline__ float start_vec(unsigned i)
 {
   unsigned h = i * 2654435761u;
@@ -252,14 +266,16 @@ template <int BS, int NW>
 __global__ void __launch_bounds__(256) k_power(int n, const int *__restrict__ rowptr, const int *__restrict__ colind,
                                                const float *__restrict__ A, const float *__restrict__ Dinv,
                                                const float *__restrict__ x, const float *__restrict__ s_prev,
-                                               float *__restrict__ y, float *__restrict__ part,
-                                               unsigned *__restrict__ ticket, float *__restrict__ norm_out)
+                                               const unsigned *__restrict__ big_prev, float *__restrict__ y,
+                                               float *__restrict__ part, unsigned *__restrict__ ticket,
+                                               float *__restrict__ norm_out, unsigned *__restrict__ big_out)
 {
   __shared__ float red[8];
   __shared__ int last;
   const int lane = threadIdx.x & 31;
-  const float s = s_prev ? 1.f / fmaxf(*s_prev, 1e-30f) : 1.f;
+  const float s = s_prev ? 1.f / fmaxf(*s_prev, 1e-30f) : big_prev ? inverse_power_of_two(*big_prev) : 1.f;
   float local = 0.f;
+  unsigned big = 0u;
   for (int r0 = 0; r0 < n; r0 += kRowCta / NW * gridDim.x) {     /* one turn where NW > 1 (host) */
     RowPlace<NW> at(n - r0);
     const int row = r0 + at.row;
@@ -280,9 +296,16 @@ __global__ void __launch_bounds__(256) k_power(int n, const int *__restrict__ ro
       v *= s;
       y[(size_t)row * kStride<BS> + lane] = v;
       local = fmaf(v, v, local);
+      big = max(big, __float_as_uint(fabsf(v)));
     }
   }
-  if (!norm_out) return;
+  if (!norm_out) {
+    if (big_out) {
+      big = __reduce_max_sync(0xffffffffu, big);
+      if (lane == 0 && big) atomicMax(big_out, big);
+    }
+    return;
+  }
   for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
   if (lane == 0) red[threadIdx.x >> 5] = local;
   __syncthreads();
@@ -995,6 +1018,7 @@ struct AmgLevelDev {
   float *b = nullptr, *x = nullptr, *r = nullptr, *d = nullptr, *y = nullptr;
   LevelPar *par = nullptr;
   float *norms = nullptr;     /* kPowerIts power-iteration norms */
+  unsigned *largest = nullptr;   /* and largest entries */
 };
 
 struct AmgHier {
@@ -1039,17 +1063,20 @@ template <int BS>
 void numeric_level(AmgHier *h, int l, cudaStream_t st)
 {
   AmgLevelDev &L = h->L[l];
-  k_dinv<BS><<<nblk(L.n, 128), 128, 0, st>>>(L.n, L.diag, L.A, L.Dinv);
+  k_dinv<BS><<<nblk(L.n, 128), 128, 0, st>>>(L.n, L.diag, L.A, L.Dinv, L.largest);
   by_warps<BS>(L.n, [&](auto nw) {
     constexpr int NW = decltype(nw)::value;
     const int ctas = nblk((long long)NW * L.n, kRowCta), grid = NW > 1 ? ctas : std::min(kPowerBlocks, ctas);
     const float *s_prev = nullptr;
+    const unsigned *big_prev = nullptr;
     for (int it = 0; it < kPowerIts; it++) {
       float *norm = power_norm(it) ? L.norms + it : nullptr;
+      unsigned *big = power_largest(it) ? L.largest + it : nullptr;
       k_power<BS, NW><<<grid, 32 * kRowCta, 0, st>>>(L.n, L.rowptr, L.colind, L.A, L.Dinv,
-                                                     it == 0 ? nullptr : (it & 1 ? L.x : L.d), s_prev, it & 1 ? L.d : L.x,
-                                                     h->part, h->ticket, norm);
+                                                     it == 0 ? nullptr : (it & 1 ? L.x : L.d), s_prev, big_prev,
+                                                     it & 1 ? L.d : L.x, h->part, h->ticket, norm, big);
       s_prev = norm;
+      big_prev = big;
     }
   });
   k_level_params<<<1, 32, 0, st>>>(L.norms + kPowerIts - 1, L.par);
@@ -1166,6 +1193,7 @@ AmgHier *amg_create(int nt, const std::vector<int> &rowptr, const std::vector<in
     if (!e) e = dalloc_(h, &L.y, nv);
     if (!e) e = dalloc_(h, &L.par, 1);
     if (!e) e = dalloc_(h, &L.norms, kPowerIts);
+    if (!e) e = dalloc_(h, &L.largest, kPowerIts);
     if (l < nl - 1) {
       L.nnzP = (long long)S.pcol.size();
       L.nnzT = (long long)S.tcol.size();
