@@ -838,14 +838,19 @@ class Gmres {
     return (int)(e == cudaSuccess ? host_wait(st_, w_.evb) : e);
   }
 
-  /* solve K dx = b (dx zeroed on entry); iterations in *its */
+  /* solve K dx = b from dx = 0; iterations in *its */
   int solve(const double *b, double *dx, double rtol, int maxit, int *its, double *relres)
   {
-    const int n = w_.n;
     *its = 0;
     *relres = 0.0;
-    cudaMemsetAsync(dx, 0, n * sizeof(double), st_);
+    cudaMemsetAsync(dx, 0, w_.n * sizeof(double), st_);
     k_solve_begin<<<1, 32, 0, st_>>>(rtol, w_.gs);
+    return resume(b, dx, rtol, maxit, its, relres);
+  }
+
+  /* the same solve, from the dx, *its and state that it was left with */
+  int resume(const double *b, double *dx, double rtol, int maxit, int *its, double *relres)
+  {
     int rc = 0;
     while (*its < maxit) {
       if ((rc = run_cycle(b, dx))) return rc;
@@ -967,10 +972,16 @@ int newton_device(const DevMesh &dm, const KParams &kp, bool f32, void *dK, doub
      it (a setup costs as much as six iterations: 64 x 48 310 us of 50 each,
      98,304 triangles 1.7 ms of 270).  Iterations with the last step's hierarchy
      against its own, by the residual's drop: 6e6 7 / 7, 2e4 15 / 15, 9e3 41 / 41, 100
-     42 / 42, but 283 22 / 16 and 62 above 110 / 42.  A solve that takes more than
-     twice the last setup's iterations and a cycle is done again on a new one. */
+     42 / 42, but 283 22 / 16 and 62 above 110 / 42.  A solve that needs more than
+     twice the iterations that the last setup's rate promises for its tolerance,
+     and a cycle, goes on from where it is with a new one.
+     An FP64 handle keeps its FP32 copy of the tangent with the hierarchy; on an
+     FP32 handle the finest level's operator is the tangent itself, the new one,
+     with the old P and P^T A P: a fixed preconditioner all the same, and under
+     this rule as good (load steps of 32 x 24 to 256 x 192 cells, fixed and
+     adaptive tolerances, both precisions: the iterations of a setup every step). */
   constexpr double kKeepHierarchy = 1e-3;
-  int its_setup = 0;
+  double rate = 0.0;       /* log of the residual's factor an iteration, since the last setup */
   for (int it = 0; it < o.max_newton; it++) {
     if (rn <= o.rtol * s.r0 || rn <= o.atol) { s.converged = 1; break; }
     double ksp_rtol = o.gmres_rtol;
@@ -1000,14 +1011,28 @@ int newton_device(const DevMesh &dm, const KParams &kp, bool f32, void *dK, doub
     k_scale_copy<<<nblk(n, 256), 256, 0, st>>>(n, dR, -1.0, w.Rt);
     int its = 0;
     double relres = 0.0;
-    const int most = keep ? std::min(o.gmres_max_it, 2 * its_setup + w.m) : o.gmres_max_it;
+    int most = o.gmres_max_it;
+    if (keep && rate < 0.0) most = (int)std::min((double)most, 2.0 * std::ceil(std::log(ksp_rtol) / rate) + w.m);
     if ((rc = gm.solve(w.Rt, w.dx, ksp_rtol, most, &its, &relres))) { err = "gmres"; return rc; }
-    if (keep && !(relres <= ksp_rtol)) {
-      s.gmres_its_total += its;
+    int its0 = 0;
+    double relres0 = 1.0;
+    bool set_up = !keep;
+    if (keep && !(relres <= ksp_rtol) && its < o.gmres_max_it) {
+      its0 = its;
+      relres0 = relres;
+      set_up = true;
       if ((rc = amg_numeric(amg, dK, f32, st))) { err = "multigrid setup"; return rc; }
-      if ((rc = gm.solve(w.Rt, w.dx, ksp_rtol, o.gmres_max_it, &its, &relres))) { err = "gmres"; return rc; }
+      if (!std::isfinite(relres)) {          /* nothing to go on from */
+        s.gmres_its_total += its;
+        its0 = 0;
+        relres0 = 1.0;
+        rc = gm.solve(w.Rt, w.dx, ksp_rtol, o.gmres_max_it, &its, &relres);
+      } else {
+        rc = gm.resume(w.Rt, w.dx, ksp_rtol, o.gmres_max_it, &its, &relres);
+      }
+      if (rc) { err = "gmres"; return rc; }
     }
-    if (!keep) its_setup = its;
+    if (set_up && its > its0) rate = std::log(std::max(relres / relres0, 1e-300)) / (its - its0);
     s.gmres_its_total += its;
     s.gmres_its_last = its;
     s.gmres_relres_last = relres;
