@@ -1031,7 +1031,6 @@ struct AmgHier {
   float *part = nullptr;
   unsigned *ticket = nullptr;
   Arena mem;
-  long long bytes = 0;
   cudaStream_t st = nullptr;
   cudaGraph_t num_graph = nullptr;      /* numeric setup, captured for one tangent buffer */
   cudaGraphExec_t num_exec = nullptr;
@@ -1047,7 +1046,6 @@ int dalloc_(AmgHier *h, T **p, size_t count)
   if (count == 0) count = 1;
   cudaError_t e = h->mem.get((void **)p, count * sizeof(T), h->st);
   if (e != cudaSuccess) return (int)e;
-  h->bytes += (long long)(count * sizeof(T));
   return 0;
 }
 
@@ -1260,7 +1258,7 @@ void amg_destroy(AmgHier *h)
 }
 
 int amg_levels(const AmgHier *h) { return h ? h->nl : 0; }
-long long amg_device_bytes(const AmgHier *h) { return h ? h->bytes : 0; }
+long long amg_device_bytes(const AmgHier *h) { return h ? (long long)h->mem.held() : 0; }
 
 static void enqueue_numeric(AmgHier *h, const void *K, bool k_is_f32, cudaStream_t st)
 {

@@ -44,6 +44,9 @@ class Arena {
     return cudaSuccess;
   }
 
+  /* device memory taken from the pool, the unused ends of slabs included */
+  size_t held() const { return held_; }
+
   void release(cudaStream_t st)
   {
     for (void *p : slabs_) cudaFreeAsync(p, st);

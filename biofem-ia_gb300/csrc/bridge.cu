@@ -159,7 +159,6 @@ struct BiofemGpuMesh_ {
   std::vector<int> rowptr, colind;
   long long nnzb = 0, ncontrib = 0;
   int n_irregular = 0, maxblk = 1;
-  size_t bytes = 0;
   Arena mem;
   DevMesh dm{};
   double *d_x = nullptr, *d_R = nullptr;   /* staging for host-array calls */
@@ -208,7 +207,6 @@ static int dalloc(BiofemGpuMesh *m, T **p, size_t n)
   void *q = nullptr;
   cudaError_t e = m->mem.get(&q, std::max<size_t>(n, 1) * sizeof(T), m->st);
   if (e != cudaSuccess) return fail(55, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-  m->bytes += std::max<size_t>(n, 1) * sizeof(T);
   *p = reinterpret_cast<T *>(q);
   return 0;
 }
@@ -654,7 +652,7 @@ int GetGpuMeshInfo(const BiofemGpuMesh *m, BiofemMeshInfo *info)
   info->n_dof = 3 * (m->topo.n_v + m->topo.n_ghosts);
   info->n_irregular = m->n_irregular;
   info->nnzb = m->nnzb; info->n_contrib = m->ncontrib;
-  info->device_bytes = (int64_t)m->bytes + solver_device_bytes(m->solver) + amg_device_bytes(m->amg);
+  info->device_bytes = (int64_t)m->mem.held() + solver_device_bytes(m->solver) + amg_device_bytes(m->amg);
   info->precision = m->prm.precision;
   return 0;
 }

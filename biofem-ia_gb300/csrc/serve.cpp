@@ -15,6 +15,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -69,8 +70,25 @@ struct BiofemServe_ {
   std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
 };
 
-extern "C" int BiofemServeEstimateBytes(int32_t n_v, int32_t n_elmt, int32_t n_ghosts, int32_t precision,
-                                        int32_t gmres_restart, int64_t *bytes);
+/* What a request's handle, solver and hierarchy take from the pool, slabs
+   included (measured 0.45 to 0.89 of this, 24 to 98,304 triangles, 2 to 6
+   points).  Per element: tangent block df/dy (244 values), forces, stress
+   gradients and tangent coefficients (FP64), reference constants (45 values a
+   thickness point; FP32-bulk handles keep them twice, 720 bytes a point above
+   three; FP64's 6800 hold six), row-assembly lists and records (80 bytes for
+   each of the element's ~12 row contributions); per node: tangent row (~37
+   blocks), pattern, flexible-GMRES bases V and Z, multigrid hierarchy (FP32 copy
+   of the tangent for FP64 handles, P, A P, the coarse operators). */
+static int64_t estimate_bytes(int32_t n_v, int32_t n_elmt, int32_t n_ghosts, int32_t precision, int32_t n_qp,
+                              int32_t gmres_restart)
+{
+  const int64_t nt = (int64_t)n_v + n_ghosts;
+  const int m = gmres_restart > 0 ? gmres_restart : 30;
+  const int more = std::min(std::max(n_qp, 3), biofem::kMaxQp) - 3;
+  const int64_t per_elem = (precision == BIOFEM_FP64 ? 6800 : 3500 + 720 * more) + 12 * 80;
+  const int64_t per_node = (precision == BIOFEM_FP64 ? 3500 + 1400 : 2100) + (int64_t)(2 * m + 8) * 24 + 3450;
+  return (per_elem * n_elmt + per_node * nt) * 5 / 4 + (8 << 20);
+}
 
 static void worker_main(BiofemServe_ *E)
 {
@@ -126,18 +144,7 @@ int BiofemServeEstimateBytes(int32_t n_v, int32_t n_elmt, int32_t n_ghosts, int3
                              int32_t gmres_restart, int64_t *bytes)
 {
   if (!bytes) return 85;
-  const int64_t nt = (int64_t)n_v + n_ghosts;
-  const int m = gmres_restart > 0 ? gmres_restart : 30;
-  /* per element: tangent block df/dy (244 values), forces, stress gradients
-     and tangent coefficients (FP64; 3 points), reference constants (an upper
-     bound with room for more points), row-assembly lists and records
-     (80 bytes for each of the element's ~12 row contributions); per node:
-     tangent row (~37 blocks), pattern, flexible-GMRES bases V and Z,
-     multigrid hierarchy (FP32 copy of the tangent for FP64 handles, P, A P,
-     the coarse operators) */
-  const int64_t per_elem = (precision == BIOFEM_FP64 ? 6800 : 3500) + 12 * 80;
-  const int64_t per_node = (precision == BIOFEM_FP64 ? 3500 + 1400 : 2100) + (int64_t)(2 * m + 8) * 24 + 3450;
-  *bytes = (per_elem * n_elmt + per_node * nt) * 5 / 4 + (8 << 20);
+  *bytes = estimate_bytes(n_v, n_elmt, n_ghosts, precision, biofem::kMaxQp, gmres_restart);
   return 0;
 }
 
@@ -175,7 +182,7 @@ int ServeSubmit(BiofemServe *E, const BiofemMeshDesc *d, const BiofemParams *prm
   r->desc.bnodes = r->bn.data(); r->desc.n_fib = r->fib.data(); r->desc.gamma_scale = r->gs.data();
   r->prm = *prm;
   if (opt) r->opt = *opt; else BiofemNewtonDefaults(&r->opt);
-  BiofemServeEstimateBytes(d->n_v, d->n_elmt, ng, prm->precision, r->opt.gmres_restart, &r->est);
+  r->est = estimate_bytes(d->n_v, d->n_elmt, ng, prm->precision, prm->n_qp, r->opt.gmres_restart);
   std::lock_guard<std::mutex> lk(E->mu);
   if (r->est > E->budget) { delete r; return 55; }   /* PETSC_ERR_MEM: can never be admitted */
   r->ticket = E->next_ticket++;

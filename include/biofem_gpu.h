@@ -96,8 +96,8 @@ typedef struct {
   int32_t n_irregular;         /* elements on the one-step-subdivision branch */
   int64_t nnzb;                /* 3x3 blocks in the tangent pattern */
   int64_t n_contrib;           /* element-block contributions (assembly map size) */
-  int64_t device_bytes;        /* device memory held by the handle: mesh arrays, and once a Newton solve has
-                                  run, its GMRES work and multigrid hierarchy */
+  int64_t device_bytes;        /* device memory taken by the handle, unused ends of its slabs included: mesh arrays,
+                                  and once a Newton solve has run, its GMRES work and multigrid hierarchy */
   int32_t precision;           /* BIOFEM_FP64 or BIOFEM_FP32_BULK */
 } BiofemMeshInfo;
 
@@ -304,7 +304,8 @@ int ServeSubmit(BiofemServe *s, const BiofemMeshDesc *mesh, const BiofemParams *
 int ServeWait(BiofemServe *s, int64_t ticket, double *x_out, BiofemNewtonStats *stats, double times[3]);
 int ServeStatsGet(BiofemServe *s, int64_t out[6]);
 int ServeDestroy(BiofemServe *s);
-/* Device-memory estimate the serving loop admits a request by. */
+/* Device-memory estimate of a request with the most thickness points; the serving
+   loop admits by the same with the request's own. */
 int BiofemServeEstimateBytes(int32_t n_v, int32_t n_elmt, int32_t n_ghosts, int32_t precision,
                              int32_t gmres_restart, int64_t *bytes);
 
