@@ -71,8 +71,13 @@ __host__ __device__ __forceinline__ double fx_to_double(Fx d, int eb)
   return ldexp((double)(((long long)d.hi << 32) + d.lo), eb - 1022 - 60);
 }
 
-/* N den 2^48 */
-__host__ __device__ __forceinline__ Fx fx_table(double n, int den) { return fx_split(llrint(n * den * 281474976710656.0)); }
+/* N den 2^48 to the nearest integer: the product and its rounding error apart,
+   which is up to 2^8 of these units */
+__host__ __device__ __forceinline__ Fx fx_table(double n, int den)
+{
+  const double p = n * den, e = fma(n, (double)den, -p), scale = 281474976710656.0;
+  return fx_split(llrint(p * scale) + llrint(e * scale));
+}
 
 /* a sum of products a b / 2^S, rounded to nearest */
 template <int S> struct FxSum {
@@ -96,6 +101,15 @@ template <int S> struct FxIntSum {
   }
   __host__ __device__ __forceinline__ long long value() const { return hi * (1ll << (32 - S)) + (lo >> S); }
 };
+
+/* one entry of an element's block through a table column n: sum n w, in units of K den^2 */
+__host__ __device__ __forceinline__ long long fx_entry(const Fx n[5], const Fx w[5])
+{
+  FxSum<63> sum;
+#pragma unroll
+  for (int s = 0; s < 5; s++) sum.add(n[s], w[s]);
+  return sum.value();
+}
 
 constexpr int kFxDenBits = 27;       /* den^2 < 2^27 */
 constexpr int kFxUnit = 31;          /* K den^2 in units of 2^(E - 31) */

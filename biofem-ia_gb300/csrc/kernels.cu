@@ -895,16 +895,7 @@ __device__ __forceinline__ FxRowBuf fx_row_buf(unsigned char *q, int maxblk)
   return b;
 }
 
-/* one entry of the block of column n */
-__device__ __forceinline__ long long fx_entry(const Fx n[5], const Fx w[5])
-{
-  FxSum<63> sum;
-#pragma unroll
-  for (int s = 0; s < 5; s++) sum.add(n[s], w[s]);
-  return sum.value();
-}
-
-/* the same of the regular table's column B, whose values are small integers over a common denominator */
+/* fx_entry of the regular table's column B, whose values are small integers over a common denominator */
 template <int B>
 __device__ __forceinline__ long long fx_entry_reg(const FxRegular &reg, const Fx w[5])
 {
@@ -960,13 +951,13 @@ __device__ __noinline__ void row_assemble_wide(const DevMesh &m, const FxRegular
         const unsigned sl = (unsigned)rc[4 + b];
         double v = 0.0;
         if (!f64) {
-          FxSum<63> sum;
+          Fx n[5];
 #pragma unroll
           for (int s = 0; s < 5; s++) {
-            const int2 n = __ldg(tab + b * kFxTab + s);
-            sum.add(Fx{n.x, n.y}, w[s]);
+            const int2 x = __ldg(tab + b * kFxTab + s);
+            n[s] = Fx{x.x, x.y};
           }
-          v = fx_wide(sum.value(), eb);
+          v = fx_wide(fx_entry(n, w), eb);
         } else {
 #pragma unroll
           for (int s = 0; s < 5; s++) v = fma(__ldg(tabd + 16 * s + b), wd[s], v);
