@@ -24,7 +24,8 @@ constexpr int kCapTable = 11;     /* flat apex-cap triangle: a1 = x2 - x1, a2 = 
 constexpr int kNumTables = 12;    /* 0 = regular 12-node patch, v = 3..10 irregular, kCapTable */
 constexpr int kDeStride = 244;    /* per-element tangent block: D = df/dy (25 x 9, with padding), then */
 constexpr int kDePres = 234;      /* the three follower-pressure corner vectors (9); 16-byte aligned */
-constexpr int kMaxRowBlocks = 1023;   /* tangent blocks per row the row assembly handles (10-bit slot targets) */
+constexpr int kMaxRowBlocks = 1023;   /* tangent blocks per row that a record can name (10-bit slot targets); a row of
+                                         more than some 900 does not fit in shared memory and is refused there */
 constexpr int kRowRec = 20;           /* ints per row-assembly record (80 bytes, 16-byte aligned) */
 constexpr unsigned kRowSlotGhost = 1u << 31;   /* record slot target of a ghost slot: three packed parents */
 constexpr unsigned kRowSlotDup = 1u << 30;     /* with kRowSlotGhost: a slot repeating an earlier slot's real node

@@ -552,13 +552,16 @@ int PrepareGpuMeshOnStream(const BiofemMeshDesc *mesh, const BiofemParams *param
   }
   dm.nnzb = m->nnzb;
   dm.maxblk = m->maxblk;
-  if (m->maxblk > row_assemble_max_blocks(params->precision != BIOFEM_FP64)) {
-    free_mesh(m);
-    return fail(63, "a tangent row has more blocks than the FP32 row assembly holds in registers");
-  }
   {
-    cudaError_t ce = (cudaError_t)row_assemble_configure(m->maxblk, params->precision != BIOFEM_FP64);
-    if (ce != cudaSuccess) { free_mesh(m); return fail(76, std::string("row assembly configuration: ") + cudaGetErrorString(ce)); }
+    const bool f32 = params->precision != BIOFEM_FP64;
+    const std::string longest = "a tangent row of " + std::to_string(m->maxblk) + " blocks: ";
+    if (m->maxblk > row_assemble_max_blocks(f32)) {
+      const std::string most = std::to_string(row_assemble_max_blocks(f32));
+      free_mesh(m);
+      return fail(63, longest + "this precision's row assembly takes " + most);
+    }
+    cudaError_t ce = (cudaError_t)row_assemble_configure(m->maxblk, f32);
+    if (ce != cudaSuccess) { free_mesh(m); return fail(76, longest + "row assembly configuration: " + cudaGetErrorString(ce)); }
   }
   double *d_fib = nullptr, *d_gsc = nullptr, *d_eref = nullptr;
   const size_t nref = (size_t)(kRefPerQp * kp.nq + kRefPerElem) * ne;

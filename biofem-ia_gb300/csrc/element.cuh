@@ -112,7 +112,7 @@ __host__ __device__ __forceinline__ V3<T> cross2(const V3<T> &a, const V3<T> &b,
 /* Reference constants of one (element, thickness point), kRefPerQp values.
    Everything the stress contracts the in-plane inverse metric with is linear
    in c = (c00, c11, c01, c22), so the constants are the forms' coefficients,
-   four each, computed once per mesh (ref_point_consts in kernels.cu):
+   four each, computed once per mesh (k_ref_prep in kernels.cu):
      S^33 etc. = S.. + alpha/2 B..(c),  Q_xy(c) of v, w, e3.
    A form costs 3 + 1 multiply-adds against the 5 to 9 of evaluating it from
    s, t, A^T v, ..., at 25 more loads a point, and FP64 is the bound: residual
@@ -717,8 +717,9 @@ __host__ __device__ __forceinline__ void tangent_block(int s, Load ld, R D[15][3
      K_ab[i][j] = sum_s N[s][b] w[15 i + 3 s + j],
    plus, when a and b are corner slots of the triangle, the follower-pressure
    block: the cross-product matrix of sc v_b, v_b the corner's vector.
-   This is the plain form, which the host tests contract with; the row
-   assemblies of kernels.cu take the same sums in their own number formats.
+   This is the plain form, for the host tests alone; the row assemblies of
+   kernels.cu take the same sums in their own number formats and layouts (the
+   FP64 one's are tested on the host through fx.cuh).
    Both sums run over the five basis rows, so the operands are kept with that
    index innermost, padded to 8: the table as tabT[8 b + s] = N[s][b] and w as
    wT[8 (3 i + j) + s] = w[15 i + 3 s + j]. */

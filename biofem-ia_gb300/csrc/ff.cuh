@@ -100,7 +100,6 @@ __host__ __device__ __forceinline__ FF dsqrt(FF a)
   return ff_fast_two_sum(s, r / (2.f * s));
 }
 
-__host__ __device__ __forceinline__ FF val(FF a) { return a; }
 
 /* Bit-level conversions between double and float-float that run on the
    integer and FP32 pipes only (no double-precision instruction): on this GPU

@@ -852,8 +852,6 @@ __device__ __forceinline__ int row_find(const int *cols, int nb, int node)
   return lo;
 }
 
-__host__ __device__ __forceinline__ size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
-
 /* FP64 row assembly in fixed point (fx.cuh); the follower-pressure vectors
    are converted to the row's units and added with it.
 
@@ -1153,7 +1151,7 @@ __global__ void __launch_bounds__(256, 3) k_row_assemble_fx(DevMesh m, KParams p
    Kahan compensation beside it.  Latency and the L1 data path bound it:
    0.38 -> 0.26 ms on the 98,304-triangle sheet (0.31 without the early loads
    of D). */
-constexpr int kRowRegMax = 64;
+constexpr int kRowF32Max = 64;       /* longest row that an FP32-bulk handle accepts */
 
 __host__ __device__ __forceinline__ size_t row_f32_bytes(int maxblk)
 {
@@ -1619,7 +1617,7 @@ bool regular_tables(const double *tab0, int den, RowTables &t)
   return ok;
 }
 
-int row_assemble_max_blocks(bool f32) { return f32 ? kRowRegMax : kMaxRowBlocks; }
+int row_assemble_max_blocks(bool f32) { return f32 ? kRowF32Max : kMaxRowBlocks; }
 
 int launch_row_assemble(const DevMesh &m, const KParams &p, const RowTables &t, void *K, bool f32, bool colmajor, void *stream)
 {
