@@ -26,7 +26,7 @@ constexpr int kPowerIts = 12;
 /* The power iterations whose norm is taken (the next one's iterate is divided
    by it): the last two give the estimate.  A norm is a reduction over the whole
    launch, half of a small level's time.  The iterate before a norm is divided by
-   the power of two of its largest entry (an atomic a warp, 1 us a launch), so
+   the power of two of its largest entry (an atomic a CTA), so
    that the sum of squares meets one factor of the eigenvalue, not four; the
    iterates between hold three.  That serves to 1e12, more than a nearly singular
    diagonal block gives (k_dinv takes 1e-12 of a block for zero). */
@@ -301,8 +301,14 @@ __global__ void __launch_bounds__(256) k_power(int n, const int *__restrict__ ro
   }
   if (!norm_out) {
     if (big_out) {
+      __shared__ unsigned most[8];
       big = __reduce_max_sync(0xffffffffu, big);
-      if (lane == 0 && big) atomicMax(big_out, big);
+      if (lane == 0) most[threadIdx.x >> 5] = big;
+      __syncthreads();
+      if (threadIdx.x < 8) {
+        big = __reduce_max_sync(0xffu, most[threadIdx.x]);
+        if (threadIdx.x == 0) atomicMax(big_out, big);
+      }
     }
     return;
   }
