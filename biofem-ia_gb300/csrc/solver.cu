@@ -1024,7 +1024,7 @@ int newton_device(const DevMesh &dm, const KParams &kp, bool f32, void *dK, doub
         s.gmres_its_total += its;
         its0 = 0;
         relres0 = 1.0;
-        rc = gm.solve(w.Rt, w.dx, ksp_rtol, o.gmres_max_it, &its, &relres);
+        rc = gm.solve(w.Rt, w.dx, ksp_rtol, o.gmres_max_it - its, &its, &relres);
       } else {
         rc = gm.resume(w.Rt, w.dx, ksp_rtol, o.gmres_max_it, &its, &relres);
       }
