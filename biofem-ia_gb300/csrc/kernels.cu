@@ -559,8 +559,8 @@ __global__ void k_to_ff(const double *__restrict__ a, float *__restrict__ b, lon
    (fx.cuh): per Cartesian pair (i, j) the largest exponent over the element's
    25 entries, then every entry as two 32-bit words; an element with an
    infinity or NaN, or with a pair near underflow, keeps its doubles and is
-   marked kFxRaw.  The pressure vectors' exponents go
-   beside D's (fx_pack), so that a load larger than D does not take D's digits. */
+   marked kFxRaw.  The pressure vectors' exponents go beside D's (fx_pack), so
+   that a load larger than D does not take D's digits. */
 constexpr int kTanElems = 6;         /* elements per warp */
 
 /* place of entry (k = 5 r + s, q = 3 i + j) of D in an FP64 element block, see the
